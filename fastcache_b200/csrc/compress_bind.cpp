@@ -108,8 +108,9 @@ void select_compact(Tensor pool, const Tensor& scores, const Tensor& block_table
   TORCH_CHECK(scores.size(0) == kv_lens.numel() && scores.size(1) == pool.size(0) && scores.size(2) == pool.size(3),
               "scores do not match the pool / batch");
   c10::cuda::CUDAGuard guard(pool.device());
+  Tensor kept = torch::empty(scores.sizes(), scores.options().dtype(torch::kInt32));   // row numbers of what stays
   fc::launch_select_compact(pool.data_ptr(), scores.data_ptr<float>(), block_tables.data_ptr<int>(),
-                            kv_lens.data_ptr<int>(), n_kepts.data_ptr<int>(), int(kv_lens.numel()),
+                            kv_lens.data_ptr<int>(), n_kepts.data_ptr<int>(), kept.data_ptr<int>(), int(kv_lens.numel()),
                             int(pool.size(0)), int(pool.size(2)), int(pool.size(4)), int(pool.size(3)),
                             int(pool.size(5)), int(block_tables.size(1)), int(scores.size(3)),
                             reinterpret_cast<uint32_t*>(status.data_ptr<int>()), at::cuda::getCurrentCUDAStream());

@@ -4,13 +4,15 @@
 // Pool layout [L, 2, num_blocks, Hkv, block_size, D] bf16 (rows of one head contiguous in a block).  Scores are fp32
 // [n_seq, L, Hkv, s_stride], higher = keep (+inf = always keep).
 //
-// select_compact: one CTA per (kv head, layer, request).  The scores of the
-// request are turned into order-preserving 32-bit keys in shared memory, the
-// k-th largest key is found with a 4-pass radix select, and the kept rows
-// (ties resolved toward later rows) are moved to the front of the request's rows
-// in ascending order.  A destination index never exceeds its source index, and
-// each 128-row chunk is read completely into registers before it is written, so
-// the compaction is safe in place.
+// select_compact, two kernels.  `select_rows_kernel`: one CTA per (kv head, layer, request) turns the scores of the
+// request into order-preserving 32-bit keys in shared memory, finds the k-th largest key with a 4-pass radix select and
+// writes the kept rows (ties resolved toward later rows) in ascending order to `kept`.  `move_rows_kernel`: K and V
+// and their 64-wide column ranges are separate CTAs (they share no byte), each moves its part of the kept rows to the
+// front of the request's rows, 256 rows at a time.  A destination index never exceeds its source index, and a chunk
+// is read completely into registers before it is written, so the compaction is safe in place.
+// Bound by the copy of the kept rows.  Selection and moves in one kernel left 256 CTAs of 256 threads for 8 requests x 4
+// layers x 8 heads, which walked all rows, kept or not, with one 64 KB chunk in flight: 235 us for 26120 rows of which
+// half stay (428 MB to move); now 19 us for the selection and 76 us for the moves.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -32,15 +34,29 @@ __device__ __forceinline__ uint32_t float_key(float f) {
 
 // scores[seq, layer, h, tok] = sign * ||K[tok, h, :]||      (mode 0: per head)
 //                            = mean_h ||K[tok, h, :]||       (mode 1: shared by heads, largest kept)
+// One CTA: 32 consecutive rows of every head; the norms pass through shared memory so that the scores are written 32
+// consecutive floats at a time.  Hkv <= 32 (checked on the host).  Sixteen lanes read one 16-byte piece each of a row.
+// Bound by the read of K: WIDE (head_dim 128, heads a multiple of eight) has sixteen rows in flight per group of lanes
+// and forms their sixteen sums with 15 shuffles instead of 64 (lanes exchange halves of what they hold, so lane i
+// ends with the sum of row i; the additions pair up as in the butterfly).  26120 rows
+// in 4 layers x 8 heads (214 MB): 82 us with one row in flight per group and unrolled step, 49 us so.
 constexpr int KN_ROWS = 32;
 
+__device__ __forceinline__ float square_sum(const uint4& v, float ss) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {        // a bf16 is the upper half of the fp32 with the same value
+    const float a = __uint_as_float(w[e] << 16), b = __uint_as_float(w[e] & 0xffff0000u);
+    ss += a * a + b * b;
+  }
+  return ss;
+}
+
+template <bool WIDE>
 __global__ void __launch_bounds__(256)
 knorm_score_kernel(const bf16* __restrict__ pool, const int* __restrict__ block_tables,
                    const int* __restrict__ kv_lens, float* __restrict__ scores, int L, int num_blocks,
                    int block_size, int Hkv, int D, int max_blocks, int s_stride, int mode, uint32_t* status) {
-  // One CTA: 32 consecutive rows of every head.  Sixteen lanes read one 16-byte piece each of a row (rows of one
-  // head are adjacent in a block, so consecutive lane groups read consecutive memory); the norms pass through
-  // shared memory so that the scores are written 32 consecutive floats at a time.  Hkv <= 32 (checked on the host).
   __shared__ float sn[KN_ROWS][33];
   const int seq = blockIdx.z, layer = blockIdx.y;
   const int len = kv_lens[seq];
@@ -50,32 +66,61 @@ knorm_score_kernel(const bf16* __restrict__ pool, const int* __restrict__ block_
   const long long kbase = ((long long)layer * 2 + 0) * num_blocks;
   const int* bt = block_tables + (long long)seq * max_blocks;
   const int rows = KN_ROWS * Hkv;
-#pragma unroll 4
-  for (int r = grp; r < rows; r += 16) {
-    const int h = r / KN_ROWS, tl = r % KN_ROWS;
-    const int tok = tok0 + tl;
-    float ss = 0.f;
-    if (tok < len) {
-      const int blk = bt[tok / block_size];
-      if (blk < 0 || blk >= num_blocks) {
-        report(status, ST_BAD_INDEX);
-      } else {
-        const uint4* row = reinterpret_cast<const uint4*>(
-            pool + (((kbase + blk) * Hkv + h) * block_size + tok % block_size) * D);
-        for (int i = sub; i < D / 8; i += 16) {
-          const uint4 v = row[i];
-          const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+  if constexpr (WIDE) {
+    // rows grp and grp + 16 of every head: two look-ups in the block table, then one stride from head to head
+    const uint4* row[2];
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {        // a bf16 is the upper half of the fp32 with the same value
-            const float a = __uint_as_float(w[e] << 16), b = __uint_as_float(w[e] & 0xffff0000u);
-            ss += a * a + b * b;
-          }
-        }
+    for (int i = 0; i < 2; ++i) {
+      const int tok = tok0 + grp + 16 * i;
+      row[i] = nullptr;
+      if (tok < len) {
+        const int blk = bt[tok / block_size];
+        if (blk < 0 || blk >= num_blocks) report(status, ST_BAD_INDEX);
+        else row[i] = reinterpret_cast<const uint4*>(pool + ((kbase + blk) * Hkv * block_size + tok % block_size) * 128) + sub;
       }
     }
+    const long long head = (long long)block_size * 16;                 // 16-byte pieces from head to head
+    for (int h0 = 0; h0 < Hkv; h0 += 8) {
+      uint4 v[16];
 #pragma unroll
-    for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    if (sub == 0) sn[tl][h] = sqrtf(ss);
+      for (int i = 0; i < 16; ++i) {
+        v[i] = make_uint4(0, 0, 0, 0);
+        if (row[i & 1] != nullptr) v[i] = row[i & 1][(h0 + (i >> 1)) * head];
+      }
+      float x[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) x[i] = square_sum(v[i], 0.f);
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) {
+        const bool up = (sub & o) != 0;                                // this lane goes on with the upper half
+#pragma unroll
+        for (int i = 0; i < o; ++i) {
+          const float give = up ? x[i] : x[i + o], keep = up ? x[i + o] : x[i];
+          x[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+      }
+      sn[grp + 16 * (sub & 1)][h0 + (sub >> 1)] = sqrtf(x[0]);
+    }
+  } else {
+#pragma unroll 4
+    for (int r = grp; r < rows; r += 16) {
+      const int h = r / KN_ROWS, tl = r % KN_ROWS;
+      const int tok = tok0 + tl;
+      float ss = 0.f;
+      if (tok < len) {
+        const int blk = bt[tok / block_size];
+        if (blk < 0 || blk >= num_blocks) {
+          report(status, ST_BAD_INDEX);
+        } else {
+          const uint4* row = reinterpret_cast<const uint4*>(
+              pool + (((kbase + blk) * Hkv + h) * block_size + tok % block_size) * D);
+          for (int i = sub; i < D / 8; i += 16) ss = square_sum(row[i], ss);
+        }
+      }
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      if (sub == 0) sn[tl][h] = sqrtf(ss);
+    }
   }
   __syncthreads();
   float* out = scores + (((long long)seq * L + layer) * Hkv) * s_stride;
@@ -95,15 +140,14 @@ knorm_score_kernel(const bf16* __restrict__ pool, const int* __restrict__ block_
   }
 }
 
-constexpr int SC_THREADS = 256;
-constexpr int SC_CHUNK = 128;
+// 1024 threads: the four passes are chains of shared-memory latencies, so a request of a few thousand rows wants few
+// rows per thread
+constexpr int SC_THREADS = 1024;
 
-template <int D>
+// kept [n_seq, L, Hkv, s_stride]: the first n_kept entries of a row are the kept rows, ascending
 __global__ void __launch_bounds__(SC_THREADS)
-select_compact_kernel(bf16* __restrict__ pool, const float* __restrict__ scores,
-                      const int* __restrict__ block_tables, const int* __restrict__ kv_lens,
-                      const int* __restrict__ n_kepts, int L, int num_blocks, int block_size, int Hkv,
-                      int max_blocks, int s_stride, uint32_t* status) {
+select_rows_kernel(const float* __restrict__ scores, const int* __restrict__ kv_lens, const int* __restrict__ n_kepts,
+                   int* __restrict__ kept, int L, int Hkv, int s_stride) {
   extern __shared__ uint32_t sm[];
   const int h = blockIdx.x, layer = blockIdx.y, seq = blockIdx.z;
   const int S = kv_lens[seq];
@@ -124,7 +168,7 @@ select_compact_kernel(bf16* __restrict__ pool, const float* __restrict__ scores,
   uint32_t prefix = 0, mask = 0;
   int remaining = k;                         // rank still to find inside the current prefix class
   for (int shift = 24; shift >= 0; shift -= 8) {
-    hist[tid] = 0;
+    if (tid < 256) hist[tid] = 0;
     __syncthreads();
     // scores of one request share their leading bits, so most keys of a warp fall into the same bin: the lanes
     // with equal bins elect one that adds their count (one shared-memory atomic per distinct bin and warp)
@@ -188,21 +232,8 @@ select_compact_kernel(bf16* __restrict__ pool, const float* __restrict__ scores,
   for (int w = 0; w < SC_THREADS / 32; ++w) eq_total += wsum[w];
   __syncthreads();
 
-  const long long kbase = ((long long)layer * 2 + 0) * num_blocks;
-  const long long vbase = ((long long)layer * 2 + 1) * num_blocks;
-  const int* bt = block_tables + (long long)seq * max_blocks;
-  auto row_ptr = [&](long long base, int tok) -> bf16* {
-    const int blk = bt[tok / block_size];
-    if (blk < 0 || blk >= num_blocks) {
-      report(status, ST_BAD_INDEX);
-      return nullptr;
-    }
-    return pool + (((base + blk) * Hkv + h) * block_size + tok % block_size) * D;
-  };
-
-  // ---- destination of every row, once for the whole request: thread t owns rows [t * RPT, (t + 1) * RPT).
-  // Two block-wide exclusive scans (ties, then kept rows); afterwards the copy loop needs one barrier per chunk.
-  int* dstpos = reinterpret_cast<int*>(keys);            // the keys are no longer needed once a row's flags are known
+  // ---- the kept rows in order: thread t owns rows [t * RPT, (t + 1) * RPT).  Two block-wide exclusive scans (ties,
+  // then kept rows).
   const int RPT = (S + SC_THREADS - 1) / SC_THREADS;
   const int r_lo = min(S, tid * RPT), r_hi = min(S, r_lo + RPT);
   auto block_exclusive = [&](int local) -> int {         // exclusive prefix of `local` over the threads of the CTA
@@ -234,45 +265,72 @@ select_compact_kernel(bf16* __restrict__ pool, const float* __restrict__ scores,
     }
   }
   int pos = block_exclusive(kept_mine);
-  {
-    int e = eq_before;
-    for (int r = r_lo; r < r_hi; ++r) {
-      const uint32_t key = keys[r];
-      const bool tie = key == thr;
-      const bool keep = (key > thr) || (tie && (eq_total - e) <= need_eq);
-      e += tie;
-      dstpos[r] = keep ? pos : -1;                        // (row r's key is not read again)
-      pos += keep;
-    }
+  int* out = kept + (((long long)seq * L + layer) * Hkv + h) * s_stride;
+  int e = eq_before;
+  for (int r = r_lo; r < r_hi; ++r) {
+    const uint32_t key = keys[r];
+    const bool tie = key == thr;
+    if ((key > thr) || (tie && (eq_total - e) <= need_eq)) out[pos++] = r;
+    e += tie;
   }
-  __syncthreads();
+}
 
-  // ---- move rows, 128 at a time: read the whole chunk, barrier, write it.  A row only ever moves towards the
-  // front, so the rows a chunk writes lie before the rows any LATER chunk reads: no barrier is needed between the
-  // writes of one chunk and the reads of the next.
-  constexpr int PIECES = D / 8;              // 16-byte pieces per row (K or V)
-  constexpr int PER_THREAD = (SC_CHUNK * 2 * PIECES) / SC_THREADS;
-  for (int c0 = 0; c0 < S; c0 += SC_CHUNK) {
-    uint4 regs[PER_THREAD];
-#pragma unroll
-    for (int j = 0; j < PER_THREAD; ++j) {
-      const int piece = tid + j * SC_THREADS;
-      const int r = c0 + piece / (2 * PIECES), part = piece % (2 * PIECES);
-      regs[j] = make_uint4(0, 0, 0, 0);
-      if (r < S && dstpos[r] >= 0 && dstpos[r] != r) {
-        const bf16* src = row_ptr(part < PIECES ? kbase : vbase, r);
-        if (src != nullptr) regs[j] = reinterpret_cast<const uint4*>(src)[part % PIECES];
+// One CTA: 64 columns (128 bytes) of K or V of one (kv head, layer, request); eight lanes read a row's part.  Lane j of
+// such a group looks up the addresses of the group's j-th row of the chunk, the others get them by shuffle: two block
+// table look-ups per row instead of one per 16-byte piece.
+constexpr int MV_THREADS = 256;
+constexpr int MV_ROWS = 8;                       // rows per group of eight lanes and chunk
+constexpr int MV_CHUNK = MV_THREADS / 8 * MV_ROWS;
+constexpr uint32_t MV_NONE = 0xffffffffu;
+
+template <int D>
+__global__ void __launch_bounds__(MV_THREADS)
+move_rows_kernel(bf16* __restrict__ pool, const int* __restrict__ kept, const int* __restrict__ block_tables,
+                 const int* __restrict__ kv_lens, const int* __restrict__ n_kepts, int L, int num_blocks, int block_size,
+                 int Hkv, int max_blocks, int s_stride, uint32_t* status) {
+  constexpr int COLS = D / 64;
+  const int part = blockIdx.x % (2 * COLS), h = blockIdx.x / (2 * COLS), layer = blockIdx.y, seq = blockIdx.z;
+  const int S = kv_lens[seq];
+  int k = n_kepts[seq];
+  if (k >= S || S <= 0) return;
+  if (k < 1) k = 1;
+  const int lane = threadIdx.x & 7, grp = threadIdx.x >> 3;
+  const int* rows = kept + (((long long)seq * L + layer) * Hkv + h) * s_stride;
+  const int* bt = block_tables + (long long)seq * max_blocks;
+  // rows of a plane are numbered (block * Hkv + head) * block_size + row: 32 bits count 512 GB of 64-wide rows
+  bf16* base = pool + ((long long)layer * 2 + part / COLS) * num_blocks * Hkv * block_size * D + (part % COLS) * 64 + lane * 8;
+  auto number = [&](int tok) -> uint32_t {
+    const int blk = bt[tok / block_size];
+    if (blk < 0 || blk >= num_blocks) {
+      report(status, ST_BAD_INDEX);
+      return MV_NONE;
+    }
+    return (uint32_t(blk) * Hkv + h) * block_size + tok % block_size;
+  };
+  for (int c0 = 0; c0 < k; c0 += MV_CHUNK) {
+    uint32_t src = MV_NONE, dst = MV_NONE;
+    const int j = c0 + grp * MV_ROWS + lane;
+    if (j < k) {
+      const int r = rows[j];
+      if (r != j) {                              // a row that stays is neither read nor written
+        src = number(r);
+        dst = number(j);
       }
     }
+    uint4 v[MV_ROWS];
+#pragma unroll
+    for (int u = 0; u < MV_ROWS; ++u) {
+      const uint32_t from = __shfl_sync(0xffffffffu, src, u, 8);
+      v[u] = make_uint4(0, 0, 0, 0);
+      if (from != MV_NONE) v[u] = *reinterpret_cast<const uint4*>(base + (long long)from * D);
+    }
+    // every row of this chunk has been read (and of the chunks before) when the first one is written; rows only move
+    // towards the front, so what is written here lies before the rows of every later chunk
     __syncthreads();
 #pragma unroll
-    for (int j = 0; j < PER_THREAD; ++j) {
-      const int piece = tid + j * SC_THREADS;
-      const int r = c0 + piece / (2 * PIECES), part = piece % (2 * PIECES);
-      if (r < S && dstpos[r] >= 0 && dstpos[r] != r) {
-        bf16* dst = row_ptr(part < PIECES ? kbase : vbase, dstpos[r]);
-        if (dst != nullptr) reinterpret_cast<uint4*>(dst)[part % PIECES] = regs[j];
-      }
+    for (int u = 0; u < MV_ROWS; ++u) {
+      const uint32_t to = __shfl_sync(0xffffffffu, dst, u, 8);
+      if (to != MV_NONE) *reinterpret_cast<uint4*>(base + (long long)to * D) = v[u];
     }
   }
 }
@@ -283,25 +341,25 @@ void launch_knorm_scores(const void* pool, const int* block_tables, const int* k
   if (n_seq == 0 || max_len == 0) return;
   if (Hkv > 32 || D % 8 != 0) throw std::runtime_error("knorm scores: at most 32 KV heads, head_dim a multiple of 8");
   dim3 grid((max_len + KN_ROWS - 1) / KN_ROWS, L, n_seq);
-  knorm_score_kernel<<<grid, 256, 0, stream>>>((const bf16*)pool, block_tables, kv_lens, scores, L, num_blocks,
-                                               block_size, Hkv, D, max_blocks, s_stride, mode, status);
+  auto kern = (D == 128 && Hkv % 8 == 0) ? knorm_score_kernel<true> : knorm_score_kernel<false>;
+  kern<<<grid, 256, 0, stream>>>((const bf16*)pool, block_tables, kv_lens, scores, L, num_blocks, block_size, Hkv, D,
+                                 max_blocks, s_stride, mode, status);
 }
 
 void launch_select_compact(void* pool, const float* scores, const int* block_tables, const int* kv_lens,
-                           const int* n_kepts, int n_seq, int L, int num_blocks, int block_size, int Hkv, int D,
+                           const int* n_kepts, int* kept, int n_seq, int L, int num_blocks, int block_size, int Hkv, int D,
                            int max_blocks, int s_stride, uint32_t* status, cudaStream_t stream) {
   if (n_seq == 0) return;
-  dim3 grid(Hkv, L, n_seq);
-  const int smem = (s_stride + 256 + 8 + SC_CHUNK + 16) * 4;
+  const int smem = (s_stride + 256 + 8 + SC_THREADS / 32) * 4;
   if (smem > 220 * 1024) throw std::runtime_error("select_compact: request too long for one CTA's shared memory");
-  auto launch = [&](auto kern) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    kern<<<grid, SC_THREADS, smem, stream>>>((bf16*)pool, scores, block_tables, kv_lens, n_kepts, L, num_blocks,
-                                             block_size, Hkv, max_blocks, s_stride, status);
-  };
-  if (D == 128) launch(select_compact_kernel<128>);
-  else if (D == 64) launch(select_compact_kernel<64>);
-  else throw std::runtime_error("select_compact: head_dim must be 64 or 128");
+  if (D != 64 && D != 128) throw std::runtime_error("select_compact: head_dim must be 64 or 128");
+  if ((long long)num_blocks * Hkv * block_size >= (long long)MV_NONE)
+    throw std::runtime_error("select_compact: too many rows in one plane of the pool");
+  cudaFuncSetAttribute(select_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  select_rows_kernel<<<dim3(Hkv, L, n_seq), SC_THREADS, smem, stream>>>(scores, kv_lens, n_kepts, kept, L, Hkv, s_stride);
+  auto move = D == 128 ? move_rows_kernel<128> : move_rows_kernel<64>;
+  move<<<dim3(Hkv * 2 * (D / 64), L, n_seq), MV_THREADS, 0, stream>>>((bf16*)pool, kept, block_tables, kv_lens, n_kepts, L,
+                                                                      num_blocks, block_size, Hkv, max_blocks, s_stride, status);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) throw std::runtime_error(std::string("select_compact launch: ") + cudaGetErrorString(e));
 }

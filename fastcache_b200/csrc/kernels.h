@@ -83,7 +83,7 @@ void set_ea_tensor_cores(bool on);
 void launch_position_scores(float* scores, const int* kv_lens, int n_seq, int units_per_seq, int stride, int n_sink,
                             cudaStream_t stream);
 void launch_select_compact(void* pool, const float* scores, const int* block_tables, const int* kv_lens,
-                           const int* n_kepts, int n_seq, int L, int num_blocks, int block_size, int Hkv, int D,
+                           const int* n_kepts, int* kept, int n_seq, int L, int num_blocks, int block_size, int Hkv, int D,
                            int max_blocks, int s_stride, uint32_t* status, cudaStream_t stream);
 }  // namespace fc
 
