@@ -10,19 +10,24 @@
 // each of the G heads (the MLP weights are shared by all heads, so short segments still fill
 // the 128-row tensor-core tile; the host picks G from the segment lengths).
 //
-//   warps 2-5 (128 workers)  gather the A operand k-block by k-block with cp.async into the
-//                            128-byte-swizzled layout tcgen05 expects (up to three k-blocks
-//                            in flight), run the epilogues (tcgen05.ld, bias, ReLU, bf16) and
-//                            scatter the result rows
-//   warp 0                   streams W1 / W2 / W3 k-blocks with TMA into the same stage ring
-//   warp 1                   issues tcgen05.mma: GEMM1 over f*2 k-blocks (A gathered), GEMM2 and
-//                            GEMM3 with the activation tile as the A operand; the epilogue writes
-//                            that tile into the A halves of the two stages whose W halves carry
-//                            the matching W2 / W3 k-blocks (those halves are idle then), so the
-//                            CTA needs 96 KiB and two CTAs share an SM; accumulators live in TMEM
-// The intermediates never leave the SM.  In-place safety: an output row index never
-// exceeds the index of any input row of the same head it depends on, tiles are processed in
-// ascending order by one CTA, and a tile is read completely (GEMM1 is done) before it is written.
+//   warps 6-9  gather the A operand of GEMM1 k-block by k-block with cp.async into the 128-byte-swizzled layout
+//              tcgen05 expects (a ring of four k-blocks that runs on from tile to tile)
+//   warp 0     streams W1 / W2 / W3 k-blocks with TMA into a ring of three
+//   warp 1     issues tcgen05.mma: GEMM1 over f*2 k-blocks (A gathered), GEMM2 and GEMM3 with the activation tile
+//              as the A operand FROM TENSOR MEMORY
+//   warps 2-5  epilogues: tcgen05.ld, bias, ReLU, bf16; the activation tile goes back over the accumulator it came
+//              from as packed bf16 (tcgen05.st), the result rows are scattered to the pool
+// The intermediates never leave the SM.  112 KB of shared memory and 256 TMEM columns: two CTAs share an SM.
+//
+// What bounds it: rows are read once and a quarter (1 / f) of them written; the floor is that traffic.  A tile is a
+// dependent chain (gather -> GEMM1 -> epilogue -> GEMM2 -> epilogue -> GEMM3 -> scatter), so the copies of the next tile
+// have to be in flight while it runs: gathering warps of their own do that (with the epilogue's threads gathering,
+// an SM had no read outstanding for most of a tile), and the activation tile in tensor memory is what pays for the
+// deeper ring.  LLaVA-1.5 shape, 15 requests of 576 + 64 rows, 32 layers x 32 heads,
+// factor 4 (6.3 GB): 4.11 ms with the epilogue's threads gathering into three shared stages, 2.17 ms so.
+// In-place safety: an output row index never exceeds the index of any input row of the same head it depends on, tiles
+// are processed in ascending order by one CTA, and a tile is read completely (GEMM1 is done) before it is written.
+// What the gathering warps read ahead lies behind every row that is still to be written for an earlier tile.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -41,8 +46,9 @@ namespace fc {
 using bf16 = __nv_bfloat16;
 
 constexpr int CCM_D = 128;
-constexpr int CCM_STAGES = 3;
-constexpr int CCM_THREADS = 192;
+constexpr int CCM_A_STAGES = 4;        // gathered k-blocks
+constexpr int CCM_W_STAGES = 3;        // weight k-blocks
+constexpr int CCM_THREADS = 320;
 constexpr int CCM_TILE = 128;          // output rows per tile
 constexpr int CCM_KB_BYTES = CCM_TILE * 64 * 2;   // one [128 x 64] bf16 sub-tile
 
@@ -72,13 +78,13 @@ __device__ __forceinline__ int ccm_seg_out(int n, int f, int min_len) {
 __global__ void __launch_bounds__(CCM_THREADS, 2)
 ccm_fused_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_constant__ CUtensorMap tm_w2,
                  const __grid_constant__ CUtensorMap tm_w3, const CcmParams p) {
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  // stage s: A sub-tile at s * 2 * KB, W sub-tile right after
-  uint64_t* a_full = reinterpret_cast<uint64_t*>(smem + CCM_STAGES * 2 * CCM_KB_BYTES);
-  uint64_t* w_full = a_full + CCM_STAGES;
-  uint64_t* empty = w_full + CCM_STAGES;
-  uint64_t* acc_full = empty + CCM_STAGES;      // [1]
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint8_t* s_w = smem + CCM_A_STAGES * CCM_KB_BYTES;
+  uint64_t* a_full = reinterpret_cast<uint64_t*>(s_w + CCM_W_STAGES * CCM_KB_BYTES);
+  uint64_t* a_empty = a_full + CCM_A_STAGES;
+  uint64_t* w_full = a_empty + CCM_A_STAGES;
+  uint64_t* w_empty = w_full + CCM_W_STAGES;
+  uint64_t* acc_full = w_empty + CCM_W_STAGES;  // [1]
   uint64_t* h_ready = acc_full + 1;             // [1]
   uint64_t* acc_free = h_ready + 1;             // [1]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_free + 1);
@@ -94,15 +100,19 @@ ccm_fused_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_constan
   const int nk_tile = nk1 + 4;                  // + 2 for W2 + 2 for W3
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < CCM_STAGES; ++s) {
+    for (int s = 0; s < CCM_A_STAGES; ++s) {
       mbar_init(&a_full[s], 128);
+      mbar_init(&a_empty[s], 1);
+    }
+    for (int s = 0; s < CCM_W_STAGES; ++s) {
       mbar_init(&w_full[s], 1);
-      mbar_init(&empty[s], 1);
+      mbar_init(&w_empty[s], 1);
     }
     mbar_init(acc_full, 1);
     mbar_init(h_ready, 128);
     mbar_init(acc_free, 128);
-    *s_abort = 0;
+    *s_abort = (smem_u32(smem) & 1023u) != 0u;  // the swizzled tiles need 1024-byte alignment: nothing runs without it
+    if (*s_abort) report(p.status, ST_BAD_INDEX);
     fence_barrier_init();
     tma_prefetch_desc(&tm_w1);
     tma_prefetch_desc(&tm_w2);
@@ -129,7 +139,7 @@ ccm_fused_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_constan
     const int sp = seg_len[s] / f;
     seg_tiles[s] = (seg_len[s] > 0 && sp >= p.min_seq_len) ? (sp + RJ - 1) >> rj_shift : 0;
   }
-  const int total_tiles = seg_tiles[0] + seg_tiles[1];
+  const int total_tiles = *s_abort ? 0 : seg_tiles[0] + seg_tiles[1];
 
   const int* bt = p.block_tables + (long long)seq * p.max_blocks;
   const long long plane = (((long long)layer * 2 + kv) * p.num_blocks);
@@ -158,31 +168,38 @@ ccm_fused_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_constan
     // ------------------------------------------------------------- weight producer (TMA)
     if (lane == 0) {
       int it = 0;
-      for (int tile = 0; tile < total_tiles && !*s_abort; ++tile) {
+      bool ok = true;
+      for (int tile = 0; tile < total_tiles && ok; ++tile) {
         const int seg = tile < seg_tiles[0] ? 0 : 1;
         const int bank = (seg == 0 ? 2 : 0) + kv;             // (tk, tv, ik, iv)
         const int wrow = (wlayer * 4 + bank) * CCM_D;
         for (int i = 0; i < nk_tile; ++i, ++it) {
-          const int stage = it % CCM_STAGES;
-          if (!mbar_wait(&empty[stage], ((it / CCM_STAGES) & 1) ^ 1, p.status, ST_TIMEOUT_EMPTY)) {
+          const int stage = it % CCM_W_STAGES;
+          if (*s_abort || !mbar_wait(&w_empty[stage], ((it / CCM_W_STAGES) & 1) ^ 1, p.status, ST_TIMEOUT_EMPTY)) {
             *s_abort = 1;
+            ok = false;
             break;
           }
-          uint8_t* sw = smem + stage * 2 * CCM_KB_BYTES + CCM_KB_BYTES;
+          uint8_t* sw = s_w + stage * CCM_KB_BYTES;
           mbar_expect_tx(&w_full[stage], CCM_KB_BYTES);
           if (i < nk1) tma_load_2d(sw, &tm_w1, &w_full[stage], i * 64, wrow);
           else if (i < nk1 + 2) tma_load_2d(sw, &tm_w2, &w_full[stage], (i - nk1) * 64, wrow);
           else tma_load_2d(sw, &tm_w3, &w_full[stage], (i - nk1 - 2) * 64, wrow);
         }
       }
+      // unwind: copies that are in flight land before the CTA may exit
+      if (!ok)
+        for (int n = max(0, it - CCM_W_STAGES); n < it; ++n)
+          mbar_wait(&w_full[n % CCM_W_STAGES], (n / CCM_W_STAGES) & 1, nullptr, 0);
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------------- MMA issuer
+    // accumulators: GEMM1 and GEMM3 in columns [0, 128), GEMM2 in [128, 256).  The activation tile of GEMM2 is in
+    // the first 64 columns of the former, that of GEMM3 in the first 64 of the latter.
     if (lane == 0) {
       constexpr uint32_t idesc = make_idesc_bf16(128, 128);
-      int it = 0;
+      int ia = 0, iw = 0;
       uint32_t h_phase = 0, free_phase = 0;
-      uint32_t a_uses[CCM_STAGES] = {0, 0, 0};
       bool ok = true;
       for (int tile = 0; tile < total_tiles && ok; ++tile) {
         // the previous tile's last epilogue must have drained accumulator 0
@@ -201,42 +218,99 @@ ccm_fused_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_constan
             if (!ok) break;
             tc_fence_after();
           }
-          for (int i = 0; i < nk && ok; ++i, ++it) {
-            const int stage = it % CCM_STAGES;
-            const uint32_t ph = (it / CCM_STAGES) & 1;
-            ok = mbar_wait(&w_full[stage], ph, p.status, ST_TIMEOUT_FULL);
-            if (ok && g == 0) {
-              // a_full[stage] completes a phase only when the stage carries a gathered operand,
-              // so its parity is counted per stage, not derived from the ring position
-              ok = mbar_wait(&a_full[stage], a_uses[stage] & 1u, p.status, ST_TIMEOUT_FULL);
-              ++a_uses[stage];
-            }
+          for (int i = 0; i < nk && ok; ++i, ++iw) {
+            const int ws = iw % CCM_W_STAGES, as = ia % CCM_A_STAGES;
+            ok = mbar_wait(&w_full[ws], (iw / CCM_W_STAGES) & 1, p.status, ST_TIMEOUT_FULL);
+            if (ok && g == 0) ok = mbar_wait(&a_full[as], (ia / CCM_A_STAGES) & 1, p.status, ST_TIMEOUT_FULL);
             if (!ok) break;
             tc_fence_after();
-            // the A half of the stage holds the gathered rows (GEMM1) or the activation sub-tile that the
-            // epilogue wrote for this k-block (GEMM2, GEMM3)
-            const uint32_t sa = smem_u32(smem + stage * 2 * CCM_KB_BYTES);
-            const uint64_t da = make_sdesc_sw128(sa);
-            const uint64_t db = make_sdesc_sw128(sa + CCM_KB_BYTES);
+            const uint64_t db = make_sdesc_sw128(smem_u32(s_w + ws * CCM_KB_BYTES));
+            if (g == 0) {
+              const uint64_t da = make_sdesc_sw128(smem_u32(smem + as * CCM_KB_BYTES));
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
-              tc_mma_f16(d_tmem, da + uint64_t(2 * k), db + uint64_t(2 * k), idesc, (i > 0 || k > 0) ? 1u : 0u);
-            tc_commit(&empty[stage]);
+              for (int k = 0; k < 4; ++k)
+                tc_mma_f16(d_tmem, da + uint64_t(2 * k), db + uint64_t(2 * k), idesc, (i > 0 || k > 0) ? 1u : 0u);
+              tc_commit(&a_empty[as]);
+              ++ia;
+            } else {
+              const uint32_t a_tmem = tmem_base + (g == 1 ? 0u : 128u) + uint32_t(i * 32);   // 64 packed columns of K
+#pragma unroll
+              for (int k = 0; k < 4; ++k)
+                tc_mma_f16_ts(d_tmem, a_tmem + uint32_t(8 * k), db + uint64_t(2 * k), idesc, (i > 0 || k > 0) ? 1u : 0u);
+            }
+            tc_commit(&w_empty[ws]);
           }
           if (ok) tc_commit(acc_full);
         }
       }
       if (!ok) *s_abort = 1;
     }
+  } else if (warp >= 6) {
+    // ---------------------------------------------------------------------- gather of GEMM1's A operand
+    // Thread gt copies 16-byte piece gt & 7 of rows (gt >> 3) + 16 q of every k-block; the eight threads of a row look up
+    // one row each and pass it on.  A stage is handed to the MMA warp once its copies, CCM_A_STAGES - 1 k-blocks back,
+    // have landed.
+    const int gt = threadIdx.x - 192;              // 0..127
+    const int ch = gt & 7, r0 = gt >> 3;
+    const uint32_t s_dst = smem_u32(smem) + r0 * 128 + ((ch ^ (r0 & 7)) << 4);     // (16 q keeps the low bits of the row)
+    constexpr uint32_t NO_ROW = 0xffffffffu;
+    const bf16* base = p.pool + ch * 8;
+    int it = 0;
+    bool ok = true;
+    for (int tile = 0; tile < total_tiles && ok; ++tile) {
+      const int seg = tile < seg_tiles[0] ? 0 : 1;
+      const int j0 = (seg == 0 ? tile : tile - seg_tiles[0]) << rj_shift;
+      const int sp = seg_len[seg] / f;
+      const int my_r = r0 + 16 * ch;               // the row this thread looks up: head my_r >> rj_shift, output row my_j
+      const int my_j = j0 + (my_r & (RJ - 1));
+      for (int tok = 0; tok < f && ok; ++tok) {
+        uint32_t mine = NO_ROW;                    // pool row (block rows of all planes counted through)
+        if (my_j < sp) {
+          const int t = seg_in[seg] + my_j * f + tok;
+          const int blk = bt[t / p.block_size];
+          if (blk < 0 || blk >= p.num_blocks) report(p.status, ST_BAD_INDEX);
+          else mine = uint32_t(((plane + blk) * p.Hkv + h0 + (my_r >> rj_shift)) * p.block_size + t % p.block_size);
+        }
+        uint32_t row[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) row[q] = __shfl_sync(0xffffffffu, mine, q, 8);
+        for (int half = 0; half < CCM_D / 64; ++half, ++it) {
+          const int stage = it % CCM_A_STAGES;
+          if (*s_abort || !mbar_wait(&a_empty[stage], ((it / CCM_A_STAGES) & 1) ^ 1, p.status, ST_TIMEOUT_EMPTY)) {
+            ok = false;
+            break;
+          }
+          const uint32_t sa = s_dst + stage * CCM_KB_BYTES;
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const bool live = row[q] != NO_ROW;
+            cp_async16(sa + q * 16 * 128, base + (live ? size_t(row[q]) * CCM_D + half * 64 : size_t(0)), live);
+          }
+          cp_async_commit();
+          if (it >= CCM_A_STAGES - 1) {
+            cp_async_wait<CCM_A_STAGES - 1>();
+            fence_proxy_async();
+            mbar_arrive(&a_full[(it + 1) % CCM_A_STAGES]);      // k-block it - (CCM_A_STAGES - 1)
+          }
+        }
+        // the shuffles above count on whole warps: a thread that gave up takes the others with it
+        ok = __all_sync(0xffffffffu, ok);
+      }
+    }
+    cp_async_wait<0>();
+    if (ok) {
+      fence_proxy_async();
+      for (int n = max(0, it - (CCM_A_STAGES - 1)); n < it; ++n) mbar_arrive(&a_full[n % CCM_A_STAGES]);
+    } else {
+      *s_abort = 1;
+    }
   } else {
-    // --------------------------------------------------- workers: gather, epilogues, scatter
+    // ---------------------------------------------------------------------- epilogues, scatter, rows that only move
     const int wt = threadIdx.x - 64;               // 0..127
     const int lane_group = warp & 3;
     const int row = lane_group * 32 + lane;        // TMEM lane == tile row owned by this thread
-    int it = 0;
     uint32_t acc_phase = 0;
-    bool ok = true;
-    int tile = 0;
+    bool ok = !*s_abort;
     for (int seg = 0; seg < 2 && ok; ++seg) {
       const int n = seg_len[seg];
       if (n <= 0) continue;
@@ -269,48 +343,10 @@ ccm_fused_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_constan
       const bf16* b1 = p.b1 + ((long long)wlayer * 4 + bank) * CCM_D;
       const bf16* b2 = p.b2 + ((long long)wlayer * 4 + bank) * CCM_D;
       const bf16* b3 = p.b3 + ((long long)wlayer * 4 + bank) * CCM_D;
-      for (int t = 0; t < seg_tiles[seg] && ok; ++t, ++tile) {
+      for (int t = 0; t < seg_tiles[seg] && ok; ++t) {
         const int j0 = t << rj_shift;
-        // ---- gather the A operand of GEMM1, one [128 x 64] k-block per stage; the copies of up to three
-        //      k-blocks are in flight, a stage is handed to the MMA warp when its own group has landed
-        for (int i = 0; i < nk1 && ok; ++i, ++it) {
-          const int stage = it % CCM_STAGES;
-          if (*s_abort || !mbar_wait(&empty[stage], ((it / CCM_STAGES) & 1) ^ 1, p.status, ST_TIMEOUT_EMPTY)) {
-            ok = false;
-            break;
-          }
-          const uint32_t sa = smem_u32(smem + stage * 2 * CCM_KB_BYTES);
-          const int tok_in_group = i / (CCM_D / 64), half = i % (CCM_D / 64);
-#pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            const int c = wt + q * 128;              // 1024 chunks of 16 bytes: (tile row r, chunk ch)
-            const int r = c >> 3, ch = c & 7;
-            const int j = j0 + (r & (RJ - 1));       // tile row r = head (r >> rj_shift), output row j of that head
-            const bf16* src = p.pool;
-            bool live = j < sp;
-            if (live) {
-              const bf16* rp = row_ptr(h0 + (r >> rj_shift), in0 + j * f + tok_in_group);
-              if (rp == nullptr) live = false;
-              else src = rp + half * 64 + ch * 8;
-            }
-            cp_async16(sa + r * 128 + ((ch ^ (r & 7)) << 4), src, live);
-          }
-          cp_async_commit();
-          if (i >= 2) {
-            cp_async_wait<2>();
-            fence_proxy_async();
-            mbar_arrive(&a_full[(it - 2) % CCM_STAGES]);
-          }
-        }
-        cp_async_wait<0>();
-        if (!ok) break;
-        // the last two k-blocks (GEMM1 always has at least two)
-        fence_proxy_async();
-        mbar_arrive(&a_full[(it - 2) % CCM_STAGES]);
-        mbar_arrive(&a_full[(it - 1) % CCM_STAGES]);
-        const int it_h = it;     // ring position of the first W2 k-block: its stage takes the first activation sub-tile
-        it += 4;     // the W2 / W3 stages carry no gathered operand (the MMA warp counts a_full uses per stage)
-        // ---- epilogues 1 and 2: bias + ReLU, activation tile to shared memory for the next GEMM
+        // ---- epilogues 1 and 2: bias + ReLU, activation tile as packed bf16 over the accumulator's first 64 columns
+        //      (a thread has read columns 0 ... 2 c + 31 of its row when it writes columns c ... c + 15)
         for (int g = 0; g < 2 && ok; ++g) {
           if (!mbar_wait(acc_full, acc_phase, p.status, ST_TIMEOUT_ACC_FULL)) {
             ok = false;
@@ -320,34 +356,28 @@ ccm_fused_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_constan
           tc_fence_after();
           const bf16* bias = g == 0 ? b1 : b2;
           const uint32_t t_addr = tmem_base + (uint32_t(lane_group * 32) << 16) + (g == 1 ? 128u : 0u);
-          // activation sub-tile i (columns 64 i .. 64 i + 63) goes to the A half of the stage whose W half
-          // carries k-block i of the next GEMM; every earlier use of those halves is complete (acc_full)
-          uint8_t* const h_dst0 = smem + ((it_h + 2 * g) % CCM_STAGES) * 2 * CCM_KB_BYTES;
-          uint8_t* const h_dst1 = smem + ((it_h + 2 * g + 1) % CCM_STAGES) * 2 * CCM_KB_BYTES;
 #pragma unroll 1
           for (int c4 = 0; c4 < 4; ++c4) {
             uint32_t rr[32];
             tmem_ld_32x32(t_addr + uint32_t(c4 * 32), rr);
             tmem_ld_wait();
-            uint8_t* const h_row = (c4 < 2 ? h_dst0 : h_dst1) + row * 128;
+            uint32_t u[16];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
               const uint4 bv = *reinterpret_cast<const uint4*>(bias + c4 * 32 + q * 8);
               const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
-              uint32_t u[4];
 #pragma unroll
               for (int e = 0; e < 4; ++e) {
                 // a bf16 is the upper half of the fp32 with the same value
                 const float a = fmaxf(__uint_as_float(rr[q * 8 + e * 2]) + __uint_as_float(bw[e] << 16), 0.f);
                 const float b = fmaxf(__uint_as_float(rr[q * 8 + e * 2 + 1]) + __uint_as_float(bw[e] & 0xffff0000u), 0.f);
-                u[e] = pack_bf16(a, b);
+                u[q * 4 + e] = pack_bf16(a, b);
               }
-              const int chunk = (c4 & 1) * 4 + q;      // 16-byte chunk of the 128-byte sub-tile row
-              *reinterpret_cast<uint4*>(h_row + ((chunk ^ (row & 7)) << 4)) = make_uint4(u[0], u[1], u[2], u[3]);
             }
+            tmem_st_32x16(t_addr + uint32_t(c4 * 16), u);
           }
+          tmem_st_wait();
           tc_fence_before();
-          fence_proxy_async();
           mbar_arrive(h_ready);
         }
         if (!ok) break;
@@ -434,6 +464,8 @@ void launch_ccm_fused(void* pool, const int* block_tables, const int* kv_lens, c
   for (int g = G; g > 1; g >>= 1) --rj_shift;
   if (D != CCM_D) throw std::runtime_error("fused CCM kernel: head_dim must be 128");
   if (factor < 1 || factor > 8) throw std::runtime_error("fused CCM kernel: factor must be in [1, 8]");
+  if ((unsigned long long)(layer_end * 2ll) * num_blocks * Hkv * block_size >= 0xffffffffull)
+    throw std::runtime_error("fused CCM kernel: the pool has more rows than 32 bits count");
   if (factor > 8) throw std::runtime_error("remainder move handles fewer than 8 rows");
   CcmParams p{};
   p.pool = (bf16*)pool;
@@ -460,7 +492,7 @@ void launch_ccm_fused(void* pool, const int* block_tables, const int* kv_lens, c
   const CUtensorMap t1 = make_tmap_bf16_2d(w1, wrows, (uint64_t)D * factor, (uint64_t)D * factor, 128, 64);
   const CUtensorMap t2 = make_tmap_bf16_2d(w2, wrows, D, D, 128, 64);
   const CUtensorMap t3 = make_tmap_bf16_2d(w3, wrows, D, D, 128, 64);
-  const int smem = CCM_STAGES * 2 * CCM_KB_BYTES + 256 + 1024;
+  const int smem = (CCM_A_STAGES + CCM_W_STAGES) * CCM_KB_BYTES + 256;
   cudaFuncSetAttribute(ccm_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   dim3 grid(Hkv / G, (layer_end - layer_start) * 2, n_seq);
   ccm_fused_kernel<<<grid, CCM_THREADS, smem, stream>>>(t1, t2, t3, p);
