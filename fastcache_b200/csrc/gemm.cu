@@ -9,20 +9,23 @@
 //   warp 1   MMA issuer: tcgen05.mma (cta_group::1, kind::f16, M = 128, N = BN,
 //            K = 16) x 4 per stage; tcgen05.commit releases the stage and, after the
 //            last K block, publishes the accumulator
-//   warps 2-5 epilogue: tcgen05.ld of the 128 x BN fp32 accumulator (one TMEM lane
-//            per thread), bias / activation, bf16 stores
+//   warps 2-5 epilogue: tcgen05.ld of the 128 x BN fp32 accumulator (one TMEM lane per thread), bias / activation,
+//            bf16 stores from registers
+//   STAGED   two such groups of four warps.  A group takes every other slab of 64 output columns, packs it into 16 KB
+//            of shared memory of its own (128-byte swizzle) and one thread hands it to TMA (cp.async.bulk.tensor
+//            store, which clips at the edges of the matrix).
 // Two accumulators (2 x BN TMEM columns) let the epilogue of one tile overlap the
 // main loop of the next.
 //
-// Output addressing is (i, j) -> C + i * ldc_i + j * ldc_j, so the same kernel
-// serves the "swapped" decode form in which the weight matrix is the 128-row
-// operand and the (small) token batch is the N operand: W is then streamed from
-// HBM exactly once per step and the result is written transposed.
-//
-// Split-K (decode shapes with few output tiles): each split stores its fp32
-// partial tile to scratch; a per-tile arrival counter elects the last split, which
-// sums the partials in split order (deterministic), applies the epilogue and
-// resets the counter.
+// What bounds it: the tensor pipe where K is a few thousand.  With K near 1000 (vision towers: K = 1024 and 1152) the
+// main loop of a 128 x 256 tile takes about 4500 clocks, and four warps that store 16 bytes per lane to 32 different
+// rows take longer than that for one accumulator: each store instruction touches 32 cache lines, and one warp per
+// scheduler has nothing to hide its tcgen05.ld and MUFU latencies with.  Hence STAGED: 15 images through the CLIP tower,
+// 95 products of 8655 rows: 5.69 ms with the stores from registers, 4.49 ms so; SigLIP, 5 slices of 961 rows: 5.73 ms
+// against 4.72 ms.  At K = 4096 and more the main loop hides the plain epilogue, and the second group only costs: 26120
+// rows through four 8B layers took 39.8 ms with it off and 40.8 ms with it on, so the line is at K = 2048.  With no more
+// than two tiles per CTA nothing hides the last epilogue whatever K is, and STAGED is the faster one again (SigLIP's
+// 4805 x 1152 x 4304).
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -43,19 +46,16 @@ namespace fc {
 
 constexpr int BM = 128;
 constexpr int BK = 64;
-constexpr int GEMM_THREADS = 192;
+constexpr int STAGED_K = 2048;                    // see above
+constexpr int SLAB = 64;                          // output columns an epilogue group stores at a time
+constexpr int SLAB_BYTES = BM * SLAB * 2;
 
 struct GemmParams {
   int M, N, K;
   __nv_bfloat16* C;
-  long long ldc_i, ldc_j;
+  long long ldc;
   const __nv_bfloat16* bias;
-  int bias_on_i;
   int act;
-  int splits;
-  int kb_per_split;
-  float* scratch;
-  int* counters;
   uint32_t* status;
   int num_m, num_n, group_m;
   int total_work;
@@ -63,7 +63,7 @@ struct GemmParams {
   // other forms (GemmForm)
   float* wide;            // GF_WIDE: columns [wide0, wide0 + wide_n) also go here in fp32, [M, wide_n]
   int wide0, wide_n;
-  float* acc;             // GF_ACC: fp32 output, pitch ldc_i, replaced or added to
+  float* acc;             // GF_ACC: fp32 output, pitch ldc, replaced or added to
   int acc_add;
   const int* plan;        // GF_GROUPED: rows sorted by group, see gemm_bf16_grouped
   int groups, group_rows; // groups, rows of W per group
@@ -114,12 +114,15 @@ __device__ __forceinline__ void apply_act_chunk(float (&v)[32], int act) {
   }
 }
 
-template <int BN, int STAGES>
+constexpr int gemm_threads(bool staged) { return staged ? 320 : 192; }
+
+template <int BN, int STAGES, bool STAGED>
 struct SmemLayout {
   static constexpr int A_BYTES = BM * BK * 2;
   static constexpr int B_BYTES = BN * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int BAR_OFF = STAGES * STAGE_BYTES;
+  static constexpr int SLAB_OFF = STAGES * STAGE_BYTES;      // one slab per epilogue group
+  static constexpr int BAR_OFF = SLAB_OFF + (STAGED ? 2 * SLAB_BYTES : 0);
   static constexpr int TOTAL = BAR_OFF + 256 + 1024;  // + barriers + alignment slack
 };
 
@@ -127,11 +130,11 @@ struct SmemLayout {
 enum Glu : int { GLU_NONE = 0, GLU_SILU = 1, GLU_GELU_TANH = 2, GLU_CLAMPED = 3 };   // GLU_GELU_TANH takes a bias [gate | up]
 enum GemmForm : int { GF_PLAIN = 0, GF_WIDE = 1, GF_ACC = 2, GF_GROUPED = 3, GF_XIELU = 4 };
 
-template <int BN, int STAGES, bool TRANS_OUT, int GLU = GLU_NONE, int FORM = GF_PLAIN>
-__global__ void __launch_bounds__(GEMM_THREADS, 1)
+template <int BN, int STAGES, int GLU = GLU_NONE, int FORM = GF_PLAIN, bool STAGED = false>
+__global__ void __launch_bounds__(gemm_threads(STAGED), 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
-                 const GemmParams p) {
-  using L = SmemLayout<BN, STAGES>;
+                 const __grid_constant__ CUtensorMap tma_c, const GemmParams p) {
+  using L = SmemLayout<BN, STAGES, STAGED>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
@@ -139,7 +142,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   uint64_t* acc_full = empty_bar + STAGES;
   uint64_t* acc_empty = acc_full + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
-  volatile int* s_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);  // [0] abort, [1] is_last
+  volatile int* s_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);  // [0] abort
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -153,10 +156,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&acc_full[a], 1);
-      mbar_init(&acc_empty[a], 128);
+      mbar_init(&acc_empty[a], STAGED ? 256 : 128);
     }
     s_flag[0] = 0;
-    s_flag[1] = 0;
     fence_barrier_init();
     tma_prefetch_desc(&tma_a);
     tma_prefetch_desc(&tma_b);
@@ -189,9 +191,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     }
   };
 
-  auto decode_work = [&](int w, int& m_blk, int& n_blk, int& kb0, int& kb1, int& tile, int& split) {
-    split = w % p.splits;
-    tile = w / p.splits;
+  auto decode_work = [&](int tile, int& m_blk, int& n_blk) {
     const int per_group = p.group_m * p.num_n;
     const int g = tile / per_group;
     const int first_m = g * p.group_m;
@@ -199,8 +199,6 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     const int local = tile - g * per_group;
     m_blk = first_m + local % gm;
     n_blk = local / gm;
-    kb0 = split * p.kb_per_split;
-    kb1 = min(num_kb, kb0 + p.kb_per_split);
   };
 
   if (warp == 0) {
@@ -211,10 +209,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       int issued = 0;
       bool ok = true;
       for (int w = blockIdx.x; w < total_work && ok; w += gridDim.x) {
-        int m_blk, n_blk, kb0, kb1, tile, split, row0, row_end, w0;
-        decode_work(w, m_blk, n_blk, kb0, kb1, tile, split);
+        int m_blk, n_blk, row0, row_end, w0;
+        decode_work(w, m_blk, n_blk);
         tile_rows(m_blk, row0, row_end, w0);
-        for (int kb = kb0; kb < kb1; ++kb) {
+        for (int kb = 0; kb < num_kb; ++kb) {
           if (s_flag[0] || !mbar_wait(&empty_bar[stage], phase ^ 1, p.status, ST_TIMEOUT_EMPTY)) {
             s_flag[0] = 1;
             ok = false;
@@ -261,15 +259,13 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       uint32_t acc_phase = 0;
       bool ok = true;
       for (int w = blockIdx.x; w < total_work && ok; w += gridDim.x) {
-        int m_blk, n_blk, kb0, kb1, tile, split;
-        decode_work(w, m_blk, n_blk, kb0, kb1, tile, split);
         if (s_flag[0] || !mbar_wait(&acc_empty[acc], acc_phase ^ 1, p.status, ST_TIMEOUT_ACC_EMPTY)) {
           s_flag[0] = 1;
           break;
         }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + uint32_t(acc * BN);
-        for (int kb = kb0; kb < kb1; ++kb) {
+        for (int kb = 0; kb < num_kb; ++kb) {
           if (s_flag[0] || !mbar_wait(&full_bar[stage], phase, p.status, ST_TIMEOUT_FULL)) {
             s_flag[0] = 1;
             ok = false;
@@ -282,7 +278,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k) {
             // +32 bytes per K = 16 step inside the 128-byte swizzle row (address field is >> 4)
-            tc_mma_f16(d_tmem, da + uint64_t(2 * k), db + uint64_t(2 * k), idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+            tc_mma_f16(d_tmem, da + uint64_t(2 * k), db + uint64_t(2 * k), idesc, (kb > 0 || k > 0) ? 1u : 0u);
           }
           tc_commit(&empty_bar[stage]);
           if (++stage == STAGES) {
@@ -300,13 +296,101 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     // ---------------------------------------------------------------- epilogue
     const int lane_group = warp & 3;                 // TMEM lanes this warp may read
     const int row = lane_group * 32 + lane;          // row of the 128 x BN tile
-    const int ep_tid = (warp - 2) * 32 + lane;       // 0..127
+    const int group = STAGED ? (warp - 2) >> 2 : 0;  // takes the slabs group, group + 2, ...
+    const bool leader = warp == 2 + 4 * group && lane == 0;
+    uint8_t* const slab = smem + L::SLAB_OFF + group * SLAB_BYTES;
+    auto group_bar = [&] { asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory"); };
+    constexpr int GROUPS = STAGED ? 2 : 1;
     int acc = 0;
     uint32_t acc_phase = 0;
+
+    // bias and activation of 32 values, columns col ... col + 31
+    auto finish = [&](float (&v)[32], int col, bool whole) {
+      if (p.bias != nullptr) {
+        if (whole && (reinterpret_cast<uintptr_t>(p.bias + col) & 15) == 0) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const uint4 bv = *reinterpret_cast<const uint4*>(p.bias + col + q * 8);
+            const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {      // a bf16 is the upper half of the fp32 with the same value
+              v[q * 8 + e * 2] += __uint_as_float(bw[e] << 16);
+              v[q * 8 + e * 2 + 1] += __uint_as_float(bw[e] & 0xffff0000u);
+            }
+          }
+        } else {
+#pragma unroll
+          for (int t = 0; t < 32; ++t)
+            if (col + t < p.N) v[t] += __bfloat162float(p.bias[col + t]);
+        }
+      }
+      if constexpr (FORM == GF_XIELU) {
+        const float a = __ldg(p.coef), b = __ldg(p.coef + 1);
+#pragma unroll
+        for (int t = 0; t < 32; ++t) v[t] = xielu_t<__nv_bfloat16>(v[t], a, b);
+      } else {
+        apply_act_chunk(v, p.act);
+      }
+    };
+    // out = act(gate) * up of 32 columns col ... col + 31 of the output, packed
+    auto gated = [&](const uint32_t (&rg)[32], const uint32_t (&ru)[32], int col, uint32_t (&u)[16]) {
+#pragma unroll
+      for (int t = 0; t < 32; t += 2) {
+        float g0 = __uint_as_float(rg[t]), g1 = __uint_as_float(rg[t + 1]);
+        float u0 = __uint_as_float(ru[t]), u1 = __uint_as_float(ru[t + 1]);
+        float a, b;
+        if constexpr (GLU == GLU_GELU_TANH) {
+          if (p.bias != nullptr) {            // pairs of a bias that starts at a multiple of 16 bytes
+            const uint32_t bg = *reinterpret_cast<const uint32_t*>(p.bias + col + t);
+            const uint32_t bu = *reinterpret_cast<const uint32_t*>(p.bias + p.up_row0 + col + t);
+            g0 += __uint_as_float(bg << 16);
+            g1 += __uint_as_float(bg & 0xffff0000u);
+            u0 += __uint_as_float(bu << 16);
+            u1 += __uint_as_float(bu & 0xffff0000u);
+          }
+          // 0.5 z (1 + tanh y) = z / (1 + exp(-2 y)), y = sqrt(2 / pi) (z + 0.044715 z^3)
+          a = __fdividef(g0, 1.f + __expf(-1.5957691216057308f * (g0 + 0.044715f * g0 * g0 * g0))) * u0;
+          b = __fdividef(g1, 1.f + __expf(-1.5957691216057308f * (g1 + 0.044715f * g1 * g1 * g1))) * u1;
+        } else if constexpr (GLU == GLU_CLAMPED) {
+          g0 = fminf(g0, p.limit);
+          g1 = fminf(g1, p.limit);
+          a = __fdividef(g0, 1.f + __expf(-1.702f * g0)) * (fminf(fmaxf(u0, -p.limit), p.limit) + 1.f);
+          b = __fdividef(g1, 1.f + __expf(-1.702f * g1)) * (fminf(fmaxf(u1, -p.limit), p.limit) + 1.f);
+        } else {
+          a = g0 / (1.f + __expf(-g0)) * u0;
+          b = g1 / (1.f + __expf(-g1)) * u1;
+        }
+        u[t / 2] = pack_bf16(a, b);
+      }
+    };
+    // 32 packed columns (half 0 or 1 of the slab) into this thread's row
+    auto park = [&](const uint32_t (&u)[16], int half) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        *reinterpret_cast<uint4*>(slab + row * 128 + (((half * 4 + q) ^ (row & 7)) << 4)) =
+            make_uint4(u[4 * q], u[4 * q + 1], u[4 * q + 2], u[4 * q + 3]);
+    };
+    // the slab's last store has been read out of shared memory when this returns
+    auto slab_free = [&] {
+      if (leader) tma_store_wait_read();
+      group_bar();
+    };
+    auto slab_out = [&](int col, int row0) {
+      fence_proxy_async();
+      group_bar();
+      if (leader && col < p.N) {
+        tma_store_2d(slab, &tma_c, col, row0);
+        tma_store_commit();
+      }
+    };
+
     for (int w = blockIdx.x; w < total_work; w += gridDim.x) {
-      int m_blk, n_blk, kb0, kb1, tile, split;
-      decode_work(w, m_blk, n_blk, kb0, kb1, tile, split);
-      if (s_flag[0] || !mbar_wait(&acc_full[acc], acc_phase, p.status, ST_TIMEOUT_ACC_FULL)) {
+      int m_blk, n_blk;
+      decode_work(w, m_blk, n_blk);
+      bool ok = !s_flag[0] && mbar_wait(&acc_full[acc], acc_phase, p.status, ST_TIMEOUT_ACC_FULL);
+      // a staged group goes on or gives up as one: its threads meet at barriers below
+      if constexpr (STAGED) ok = barrier_all(1 + group, 128, ok);
+      if (!ok) {
         s_flag[0] = 1;
         break;
       }
@@ -315,71 +399,106 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       int row0, row_end, w0;
       tile_rows(m_blk, row0, row_end, w0);
       const int gi = row0 + row;
-      const int j0 = n_blk * BN;
+      auto acc_read = [&] {                  // accumulator fully read by this thread: hand it back before the stores
+        tc_fence_before();
+        mbar_arrive(&acc_empty[acc]);
+      };
 
-      auto finish_chunk = [&](float (&v)[32], int c) {
-        // v: 32 consecutive columns of row `gi`, starting at column j0 + 32 c
-        const int jb = j0 + c * 32;
-        if (gi >= row_end) return;
-        if constexpr (FORM == GF_ACC) {
-          float* dst = p.acc + (long long)gi * p.ldc_i + jb;
-          if (jb + 32 <= p.N && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-            float4 o[8];
+      if constexpr (GLU != GLU_NONE) {
+        // accumulator columns [0, BN/2) = gate, [BN/2, BN) = up; out[:, n_blk * BN/2 + j] = act(gate_j) * up_j
+        const int jo = n_blk * (BN / 2);
+#pragma unroll 1
+        for (int sl = group; sl < BN / 2 / SLAB; sl += GROUPS) {
+          if constexpr (STAGED) slab_free();
+#pragma unroll 1
+          for (int half = 0; half < 2; ++half) {
+            __syncwarp();                    // a tensor-memory load is a warp instruction
+            const int c = sl * SLAB + half * 32;
+            uint32_t rg[32], ru[32], u[16];
+            tmem_ld_32x32(t_addr + uint32_t(c), rg);
+            tmem_ld_32x32(t_addr + uint32_t(BN / 2 + c), ru);
+            tmem_ld_wait();
+            if (half == 1 && sl + GROUPS >= BN / 2 / SLAB) acc_read();
+            gated(rg, ru, jo + c, u);
+            if (STAGED) {
+              park(u, half);
+            } else if (gi < row_end) {
+              __nv_bfloat16* dst = p.C + (long long)gi * p.ldc + jo + c;
 #pragma unroll
-            for (int q = 0; q < 8; ++q)
-              o[q] = p.acc_add ? *reinterpret_cast<const float4*>(dst + q * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-            for (int q = 0; q < 8; ++q)
-              *reinterpret_cast<float4*>(dst + q * 4) =
-                  make_float4(o[q].x + v[q * 4], o[q].y + v[q * 4 + 1], o[q].z + v[q * 4 + 2], o[q].w + v[q * 4 + 3]);
-          } else {
-#pragma unroll
-            for (int t = 0; t < 32; ++t)
-              if (jb + t < p.N) dst[t] = p.acc_add ? dst[t] + v[t] : v[t];
-          }
-          return;
-        }
-        if constexpr (FORM == GF_WIDE) {
-          if (jb < p.wide0 + p.wide_n && jb + 32 > p.wide0) {
-#pragma unroll
-            for (int t = 0; t < 32; ++t) {
-              const int o = jb + t - p.wide0;
-              if (o >= 0 && o < p.wide_n) p.wide[(long long)gi * p.wide_n + o] = v[t];
+              for (int q = 0; q < 4; ++q)
+                *reinterpret_cast<uint4*>(dst + q * 8) = make_uint4(u[4 * q], u[4 * q + 1], u[4 * q + 2], u[4 * q + 3]);
             }
           }
+          if constexpr (STAGED) slab_out(jo + sl * SLAB, row0);
         }
-        float bi = (p.bias != nullptr && p.bias_on_i) ? __bfloat162float(p.bias[gi]) : 0.f;
-        if constexpr (!TRANS_OUT) {
-          __nv_bfloat16* dst = p.C + (long long)gi * p.ldc_i + jb;
-          const bool vec_ok = (jb + 32 <= p.N) && ((reinterpret_cast<uintptr_t>(dst) & 15) == 0);
-          if (vec_ok) {
-            if (p.bias != nullptr) {
-              if (p.bias_on_i) {
+      } else if constexpr (STAGED) {
+#pragma unroll 1
+        for (int sl = group; sl < BN / SLAB; sl += GROUPS) {
+          const int col = n_blk * BN + sl * SLAB;
+          uint32_t r[2][32];
+          tmem_ld_32x32(t_addr + uint32_t(sl * SLAB), r[0]);
+          tmem_ld_32x32(t_addr + uint32_t(sl * SLAB + 32), r[1]);
+          tmem_ld_wait();
+          if (sl + GROUPS >= BN / SLAB) acc_read();
+          slab_free();
 #pragma unroll
-                for (int t = 0; t < 32; ++t) v[t] += bi;
-              } else if ((reinterpret_cast<uintptr_t>(p.bias + jb) & 15) == 0) {
+          for (int half = 0; half < 2; ++half) {
+            float v[32];
+            uint32_t u[16];
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                  const uint4 bv = *reinterpret_cast<const uint4*>(p.bias + jb + q * 8);
-                  const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
+            for (int t = 0; t < 32; ++t) v[t] = __uint_as_float(r[half][t]);
+            finish(v, col + half * 32, col + SLAB <= p.N);
 #pragma unroll
-                  for (int e = 0; e < 4; ++e) {      // a bf16 is the upper half of the fp32 with the same value
-                    v[q * 8 + e * 2] += __uint_as_float(bw[e] << 16);
-                    v[q * 8 + e * 2 + 1] += __uint_as_float(bw[e] & 0xffff0000u);
-                  }
-                }
-              } else {
+            for (int t = 0; t < 16; ++t) u[t] = pack_bf16(v[2 * t], v[2 * t + 1]);
+            park(u, half);
+          }
+          slab_out(col, row0);
+        }
+      } else {
+#pragma unroll 1
+        for (int c = 0; c < BN / 32; ++c) {
+          __syncwarp();                      // a tensor-memory load is a warp instruction
+          uint32_t r[32];
+          tmem_ld_32x32(t_addr + uint32_t(c * 32), r);
+          tmem_ld_wait();
+          float v[32];
 #pragma unroll
-                for (int t = 0; t < 32; ++t) v[t] += __bfloat162float(p.bias[jb + t]);
+          for (int t = 0; t < 32; ++t) v[t] = __uint_as_float(r[t]);
+          if (c == BN / 32 - 1) acc_read();
+          // v: 32 consecutive columns of row `gi`
+          const int jb = n_blk * BN + c * 32;
+          if (gi >= row_end) continue;
+          if constexpr (FORM == GF_ACC) {
+            float* dst = p.acc + (long long)gi * p.ldc + jb;
+            if (jb + 32 <= p.N && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+              float4 o[8];
+#pragma unroll
+              for (int q = 0; q < 8; ++q)
+                o[q] = p.acc_add ? *reinterpret_cast<const float4*>(dst + q * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+              for (int q = 0; q < 8; ++q)
+                *reinterpret_cast<float4*>(dst + q * 4) =
+                    make_float4(o[q].x + v[q * 4], o[q].y + v[q * 4 + 1], o[q].z + v[q * 4 + 2], o[q].w + v[q * 4 + 3]);
+            } else {
+#pragma unroll
+              for (int t = 0; t < 32; ++t)
+                if (jb + t < p.N) dst[t] = p.acc_add ? dst[t] + v[t] : v[t];
+            }
+            continue;
+          }
+          if constexpr (FORM == GF_WIDE) {
+            if (jb < p.wide0 + p.wide_n && jb + 32 > p.wide0) {
+#pragma unroll
+              for (int t = 0; t < 32; ++t) {
+                const int o = jb + t - p.wide0;
+                if (o >= 0 && o < p.wide_n) p.wide[(long long)gi * p.wide_n + o] = v[t];
               }
             }
-            if constexpr (FORM == GF_XIELU) {
-              const float a = __ldg(p.coef), b = __ldg(p.coef + 1);
-#pragma unroll
-              for (int t = 0; t < 32; ++t) v[t] = xielu_t<__nv_bfloat16>(v[t], a, b);
-            } else {
-              apply_act_chunk(v, p.act);
-            }
+          }
+          __nv_bfloat16* dst = p.C + (long long)gi * p.ldc + jb;
+          const bool whole = jb + 32 <= p.N;
+          finish(v, jb, whole);
+          if (whole && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
               uint32_t u[4];
@@ -389,137 +508,16 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
             }
           } else {
 #pragma unroll
-            for (int t = 0; t < 32; ++t) {
-              if (jb + t < p.N) {
-                float a = v[t] + bi;
-                if (p.bias != nullptr && !p.bias_on_i) a += __bfloat162float(p.bias[jb + t]);
-                if constexpr (FORM == GF_XIELU) a = xielu_t<__nv_bfloat16>(a, __ldg(p.coef), __ldg(p.coef + 1));
-                else a = apply_act(a, p.act);
-                dst[t] = __float2bfloat16(a);
-              }
-            }
-          }
-        } else {
-#pragma unroll
-          for (int t = 0; t < 32; ++t) {
-            if (jb + t < p.N) {
-              float a = v[t] + bi;
-              if (p.bias != nullptr && !p.bias_on_i) a += __bfloat162float(p.bias[jb + t]);
-              p.C[(long long)gi * p.ldc_i + (long long)(jb + t) * p.ldc_j] = __float2bfloat16(apply_act(a, p.act));
-            }
+            for (int t = 0; t < 32; ++t)
+              if (jb + t < p.N) dst[t] = __float2bfloat16(v[t]);
           }
         }
-      };
-
-      if constexpr (GLU != GLU_NONE) {
-        // accumulator columns [0, BN/2) = gate, [BN/2, BN) = up; out[:, n_blk * BN/2 + j] = silu(gate_j) * up_j
-        const int jo = n_blk * (BN / 2);
-#pragma unroll 1
-        for (int c = 0; c < BN / 64; ++c) {
-          uint32_t rg[32], ru[32];
-          tmem_ld_32x32(t_addr + uint32_t(c * 32), rg);
-          tmem_ld_32x32(t_addr + uint32_t(BN / 2 + c * 32), ru);
-          tmem_ld_wait();
-          if (c == BN / 64 - 1) {
-            tc_fence_before();
-            mbar_arrive(&acc_empty[acc]);
-          }
-          if (gi < row_end) {
-            __nv_bfloat16* dst = p.C + (long long)gi * p.ldc_i + jo + c * 32;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              uint32_t u[4];
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const int t = q * 8 + e * 2;
-                float g0 = __uint_as_float(rg[t]), g1 = __uint_as_float(rg[t + 1]);
-                float u0 = __uint_as_float(ru[t]), u1 = __uint_as_float(ru[t + 1]);
-                float a, b;
-                if constexpr (GLU == GLU_GELU_TANH) {
-                  if (p.bias != nullptr) {            // pairs of a bias that starts at a multiple of 16 bytes
-                    const uint32_t bg = *reinterpret_cast<const uint32_t*>(p.bias + jo + c * 32 + t);
-                    const uint32_t bu = *reinterpret_cast<const uint32_t*>(p.bias + p.up_row0 + jo + c * 32 + t);
-                    g0 += __uint_as_float(bg << 16);
-                    g1 += __uint_as_float(bg & 0xffff0000u);
-                    u0 += __uint_as_float(bu << 16);
-                    u1 += __uint_as_float(bu & 0xffff0000u);
-                  }
-                  // 0.5 z (1 + tanh y) = z / (1 + exp(-2 y)), y = sqrt(2 / pi) (z + 0.044715 z^3)
-                  a = __fdividef(g0, 1.f + __expf(-1.5957691216057308f * (g0 + 0.044715f * g0 * g0 * g0))) * u0;
-                  b = __fdividef(g1, 1.f + __expf(-1.5957691216057308f * (g1 + 0.044715f * g1 * g1 * g1))) * u1;
-                } else if constexpr (GLU == GLU_CLAMPED) {
-                  g0 = fminf(g0, p.limit);
-                  g1 = fminf(g1, p.limit);
-                  a = __fdividef(g0, 1.f + __expf(-1.702f * g0)) * (fminf(fmaxf(u0, -p.limit), p.limit) + 1.f);
-                  b = __fdividef(g1, 1.f + __expf(-1.702f * g1)) * (fminf(fmaxf(u1, -p.limit), p.limit) + 1.f);
-                } else {
-                  a = g0 / (1.f + __expf(-g0)) * u0;
-                  b = g1 / (1.f + __expf(-g1)) * u1;
-                }
-                u[e] = pack_bf16(a, b);
-              }
-              *reinterpret_cast<uint4*>(dst + q * 8) = make_uint4(u[0], u[1], u[2], u[3]);
-            }
-          }
-        }
-      } else if (p.splits == 1) {
-#pragma unroll 1
-        for (int c = 0; c < BN / 32; ++c) {
-          uint32_t r[32];
-          tmem_ld_32x32(t_addr + uint32_t(c * 32), r);
-          tmem_ld_wait();
-          float v[32];
-#pragma unroll
-          for (int t = 0; t < 32; ++t) v[t] = __uint_as_float(r[t]);
-          if (c == BN / 32 - 1) {
-            // accumulator fully read: hand it back before the global stores
-            tc_fence_before();
-            mbar_arrive(&acc_empty[acc]);
-          }
-          finish_chunk(v, c);
-        }
-      } else {
-        // split-K: park the fp32 partial, the last split to arrive reduces
-        float* part = p.scratch + ((long long)tile * p.splits + split) * (BM * BN);
-#pragma unroll 1
-        for (int c = 0; c < BN / 32; ++c) {
-          uint32_t r[32];
-          tmem_ld_32x32(t_addr + uint32_t(c * 32), r);
-          tmem_ld_wait();
-#pragma unroll
-          for (int t = 0; t < 32; ++t) part[(c * 32 + t) * BM + row] = __uint_as_float(r[t]);
-        }
-        tc_fence_before();
-        mbar_arrive(&acc_empty[acc]);
-        __threadfence();
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        if (ep_tid == 0) {
-          const int old = atomicAdd(&p.counters[tile], 1);
-          s_flag[1] = (old == p.splits - 1) ? 1 : 0;
-        }
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        if (s_flag[1]) {
-          __threadfence();
-          const float* base = p.scratch + (long long)tile * p.splits * (BM * BN);
-#pragma unroll 1
-          for (int c = 0; c < BN / 32; ++c) {
-            float v[32];
-#pragma unroll
-            for (int t = 0; t < 32; ++t) v[t] = 0.f;
-            for (int s = 0; s < p.splits; ++s) {
-              const float* ps = base + (long long)s * (BM * BN);
-#pragma unroll
-              for (int t = 0; t < 32; ++t) v[t] += __ldcg(&ps[(c * 32 + t) * BM + row]);
-            }
-            finish_chunk(v, c);
-          }
-          if (ep_tid == 0) p.counters[tile] = 0;
-        }
-        asm volatile("bar.sync 1, 128;" ::: "memory");
       }
+      __syncwarp();
       acc ^= 1;
       if (acc == 0) acc_phase ^= 1;
     }
+    if (STAGED && leader) tma_store_wait_all();
   }
 
   tc_fence_before();
@@ -582,11 +580,11 @@ CUtensorMap make_tmap_bf16_3d(const void* base, uint64_t n0, uint64_t n1, uint64
   return m;
 }
 
-template <int BN, int STAGES, bool TRANS, int GLU = GLU_NONE, int FORM = GF_PLAIN>
-static void launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int grid,
-                       cudaStream_t stream) {
-  using L = SmemLayout<BN, STAGES>;
-  auto kern = gemm_bf16_kernel<BN, STAGES, TRANS, GLU, FORM>;
+template <int BN, int STAGES, int GLU, int FORM, bool STAGED>
+static void launch_form(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const GemmParams& p, int grid,
+                        cudaStream_t stream) {
+  using L = SmemLayout<BN, STAGES, STAGED>;
+  auto kern = gemm_bf16_kernel<BN, STAGES, GLU, FORM, STAGED>;
   // the attribute belongs to the (function, device) pair: remember it per device, not per process
   static std::atomic<uint64_t> configured{0};
   int dev = 0;
@@ -597,9 +595,24 @@ static void launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const GemmP
     if (e != cudaSuccess) throw std::runtime_error(std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
     configured.fetch_or(bit, std::memory_order_relaxed);
   }
-  kern<<<grid, GEMM_THREADS, L::TOTAL, stream>>>(ta, tb, p);
+  kern<<<grid, gemm_threads(STAGED), L::TOTAL, stream>>>(ta, tb, tc, p);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) throw std::runtime_error(std::string("gemm launch: ") + cudaGetErrorString(e));
+}
+
+// The staged epilogue for a short main loop, or a CTA's last tile being half of its work, and an output that TMA can
+// describe; grouped rows (a tile may end inside
+// another group's rows) and the fp32 forms have the other one only.
+template <int BN, int STAGES, int GLU = GLU_NONE, int FORM = GF_PLAIN>
+static void launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int grid, cudaStream_t stream) {
+  if constexpr (FORM == GF_PLAIN || FORM == GF_XIELU) {
+    if ((p.K <= STAGED_K || p.total_work <= 2 * grid) && p.ldc % 8 == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0) {
+      const CUtensorMap tc = make_tmap_bf16_2d(p.C, p.M, p.N, p.ldc, BM, SLAB);
+      launch_form<BN, STAGES, GLU, FORM, true>(ta, tb, tc, p, grid, stream);
+      return;
+    }
+  }
+  launch_form<BN, STAGES, GLU, FORM, false>(ta, tb, ta, p, grid, stream);        // (the last map is not read)
 }
 
 static int g_num_sms = 0;
@@ -629,9 +642,6 @@ void gemm_bf16(const void* x, const void* w, void* c, const void* bias, int M, i
   p.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
   p.act = act;
   p.status = ws.status;
-  p.scratch = ws.scratch;
-  p.counters = ws.counters;
-  const int num_kb = (K + BK - 1) / BK;
   const bool swapped = (M <= 256);
   if (!swapped && gemm_pairs_mode() && act != ACT_GEGLU_TANH &&
       gemm_bf16_2cta(x, w, c, bias, M, N, K, ldx, ldw, ldc, act, sm_limit, ws.status, stream))
@@ -640,11 +650,7 @@ void gemm_bf16(const void* x, const void* w, void* c, const void* bias, int M, i
     // tokens are the 128-row operand
     p.M = M;
     p.N = N;
-    p.ldc_i = ldc;
-    p.ldc_j = 1;
-    p.bias_on_i = 0;
-    p.splits = 1;
-    p.kb_per_split = num_kb;
+    p.ldc = ldc;
     p.num_m = (M + BM - 1) / BM;
     p.group_m = 16;
     CUtensorMap ta = make_tmap_bf16_2d(x, M, K, ldx, BM, BK);
@@ -661,22 +667,22 @@ void gemm_bf16(const void* x, const void* w, void* c, const void* bias, int M, i
       p.num_n = width / (BN / 2);
       p.total_work = p.num_m * p.num_n;
       CUtensorMap tb = make_tmap_bf16_2d(w, N, K, ldw, BN / 2, BK);
-      if (act == ACT_SWIGLU) launch_one<BN, 4, false, GLU_SILU>(ta, tb, p, std::min(p.total_work, sms), stream);
-      else launch_one<BN, 4, false, GLU_GELU_TANH>(ta, tb, p, std::min(p.total_work, sms), stream);
+      if (act == ACT_SWIGLU) launch_one<BN, 4, GLU_SILU>(ta, tb, p, std::min(p.total_work, sms), stream);
+      else launch_one<BN, 4, GLU_GELU_TANH>(ta, tb, p, std::min(p.total_work, sms), stream);
       return;
     }
-    if (N >= 256 || N % 256 == 0) {
+    if (N >= 256) {
       constexpr int BN = 256;
       p.num_n = (N + BN - 1) / BN;
       p.total_work = p.num_m * p.num_n;
       CUtensorMap tb = make_tmap_bf16_2d(w, N, K, ldw, BN, BK);
-      launch_one<BN, 4, false>(ta, tb, p, std::min(p.total_work, sms), stream);
+      launch_one<BN, 4>(ta, tb, p, std::min(p.total_work, sms), stream);
     } else {
       constexpr int BN = 128;
       p.num_n = (N + BN - 1) / BN;
       p.total_work = p.num_m * p.num_n;
       CUtensorMap tb = make_tmap_bf16_2d(w, N, K, ldw, BN, BK);
-      launch_one<BN, 6, false>(ta, tb, p, std::min(p.total_work, sms), stream);
+      launch_one<BN, 6>(ta, tb, p, std::min(p.total_work, sms), stream);
     }
     return;
   }
@@ -696,11 +702,8 @@ static GemmParams prefill_params(void* c, int M, int N, int K, long long ldc, co
   p.N = N;
   p.K = K;
   p.C = reinterpret_cast<__nv_bfloat16*>(c);
-  p.ldc_i = ldc;
-  p.ldc_j = 1;
+  p.ldc = ldc;
   p.status = ws.status;
-  p.splits = 1;
-  p.kb_per_split = (K + BK - 1) / BK;
   p.num_m = (M + BM - 1) / BM;
   p.group_m = 16;
   return p;
@@ -718,14 +721,14 @@ void gemm_bf16_wide(const void* x, const void* w, void* c, int M, int N, int K, 
     constexpr int BN = 128;
     p.num_n = 1;
     p.total_work = p.num_m;
-    launch_one<BN, 6, false, GLU_NONE, GF_WIDE>(make_tmap_bf16_2d(x, M, K, ldx, BM, BK), make_tmap_bf16_2d(w, N, K, ldw, BN, BK), p,
+    launch_one<BN, 6, GLU_NONE, GF_WIDE>(make_tmap_bf16_2d(x, M, K, ldx, BM, BK), make_tmap_bf16_2d(w, N, K, ldw, BN, BK), p,
                                                 std::min(p.total_work, sms), stream);
     return;
   }
   constexpr int BN = 256;
   p.num_n = (N + BN - 1) / BN;
   p.total_work = p.num_m * p.num_n;
-  launch_one<BN, 4, false, GLU_NONE, GF_WIDE>(make_tmap_bf16_2d(x, M, K, ldx, BM, BK), make_tmap_bf16_2d(w, N, K, ldw, BN, BK),
+  launch_one<BN, 4, GLU_NONE, GF_WIDE>(make_tmap_bf16_2d(x, M, K, ldx, BM, BK), make_tmap_bf16_2d(w, N, K, ldw, BN, BK),
                                               p, std::min(p.total_work, sms), stream);
 }
 
@@ -739,7 +742,7 @@ void gemm_bf16_acc(const void* x, const void* w, float* y, int M, int N, int K, 
   p.acc_add = add ? 1 : 0;
   p.num_n = (N + BN - 1) / BN;
   p.total_work = p.num_m * p.num_n;
-  launch_one<BN, 4, false, GLU_NONE, GF_ACC>(make_tmap_bf16_2d(x, M, K, ldx, BM, BK), make_tmap_bf16_2d(w, N, K, ldw, BN, BK),
+  launch_one<BN, 4, GLU_NONE, GF_ACC>(make_tmap_bf16_2d(x, M, K, ldx, BM, BK), make_tmap_bf16_2d(w, N, K, ldw, BN, BK),
                                              p, std::min(p.total_work, sms), stream);
 }
 
@@ -754,7 +757,7 @@ void gemm_bf16_clamped_glu(const void* x, const void* w, void* c, int M, int wid
   p.up_row0 = width;
   p.num_n = width / (BN / 2);
   p.total_work = p.num_m * p.num_n;
-  launch_one<BN, 4, false, GLU_CLAMPED>(make_tmap_bf16_2d(x, M, K, ldx, BM, BK),
+  launch_one<BN, 4, GLU_CLAMPED>(make_tmap_bf16_2d(x, M, K, ldx, BM, BK),
                                         make_tmap_bf16_2d(w, 2 * width, K, ldw, BN / 2, BK), p,
                                         std::min(p.total_work, sm_limit > 0 ? sm_limit : gemm_num_sms()), stream);
 }
@@ -767,7 +770,7 @@ void gemm_bf16_xielu(const void* x, const void* w, void* c, const float* coef, i
   p.coef = coef;
   p.num_n = (N + BN - 1) / BN;
   p.total_work = p.num_m * p.num_n;
-  launch_one<BN, 4, false, GLU_NONE, GF_XIELU>(make_tmap_bf16_2d(x, M, K, ldx, BM, BK), make_tmap_bf16_2d(w, N, K, ldw, BN, BK), p,
+  launch_one<BN, 4, GLU_NONE, GF_XIELU>(make_tmap_bf16_2d(x, M, K, ldx, BM, BK), make_tmap_bf16_2d(w, N, K, ldw, BN, BK), p,
                                                std::min(p.total_work, sm_limit > 0 ? sm_limit : gemm_num_sms()), stream);
 }
 
@@ -792,17 +795,17 @@ void gemm_bf16_grouped(const void* x, const void* w, void* c, const int* plan, i
     p.num_n = width / (BN / 2);
     const CUtensorMap tb = make_tmap_bf16_2d(w, (uint64_t)groups * N, K, K, BN / 2, BK);
     const int grid = std::min(max_tiles * p.num_n, sms);
-    if (glu_kind == 0) launch_one<BN, 4, false, GLU_SILU, GF_GROUPED>(ta, tb, p, grid, stream);
-    else launch_one<BN, 4, false, GLU_CLAMPED, GF_GROUPED>(ta, tb, p, grid, stream);
+    if (glu_kind == 0) launch_one<BN, 4, GLU_SILU, GF_GROUPED>(ta, tb, p, grid, stream);
+    else launch_one<BN, 4, GLU_CLAMPED, GF_GROUPED>(ta, tb, p, grid, stream);
   } else if (N >= 256) {
     constexpr int BN = 256;
     p.num_n = (N + BN - 1) / BN;
-    launch_one<BN, 4, false, GLU_NONE, GF_GROUPED>(ta, make_tmap_bf16_2d(w, (uint64_t)groups * N, K, K, BN, BK), p,
+    launch_one<BN, 4, GLU_NONE, GF_GROUPED>(ta, make_tmap_bf16_2d(w, (uint64_t)groups * N, K, K, BN, BK), p,
                                                    std::min(max_tiles * p.num_n, sms), stream);
   } else {
     constexpr int BN = 128;
     p.num_n = (N + BN - 1) / BN;
-    launch_one<BN, 6, false, GLU_NONE, GF_GROUPED>(ta, make_tmap_bf16_2d(w, (uint64_t)groups * N, K, K, BN, BK), p,
+    launch_one<BN, 6, GLU_NONE, GF_GROUPED>(ta, make_tmap_bf16_2d(w, (uint64_t)groups * N, K, K, BN, BK), p,
                                                    std::min(max_tiles * p.num_n, sms), stream);
   }
 }
