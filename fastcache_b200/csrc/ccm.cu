@@ -24,7 +24,8 @@
 // have to be in flight while it runs: gathering warps of their own do that (with the epilogue's threads gathering,
 // an SM had no read outstanding for most of a tile), and the activation tile in tensor memory is what pays for the
 // deeper ring.  LLaVA-1.5 shape, 15 requests of 576 + 64 rows, 32 layers x 32 heads,
-// factor 4 (6.3 GB): 4.11 ms with the epilogue's threads gathering into three shared stages, 2.17 ms so.
+// factor 4 (6.3 GB): 4.11 ms with the epilogue's threads gathering into three shared stages, 2.17 ms so, 1.96 ms with
+// the first GEMM of a tile under the scatter of the one before and a full ring announced at once.
 // In-place safety: an output row index never exceeds the index of any input row of the same head it depends on, tiles
 // are processed in ascending order by one CTA, and a tile is read completely (GEMM1 is done) before it is written.
 // What the gathering warps read ahead lies behind every row that is still to be written for an earlier tile.
@@ -84,10 +85,9 @@ ccm_fused_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_constan
   uint64_t* a_empty = a_full + CCM_A_STAGES;
   uint64_t* w_full = a_empty + CCM_A_STAGES;
   uint64_t* w_empty = w_full + CCM_W_STAGES;
-  uint64_t* acc_full = w_empty + CCM_W_STAGES;  // [1]
-  uint64_t* h_ready = acc_full + 1;             // [1]
-  uint64_t* acc_free = h_ready + 1;             // [1]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_free + 1);
+  uint64_t* acc_full = w_empty + CCM_W_STAGES;  // [2]: GEMM1; GEMM2 and GEMM3 in turn
+  uint64_t* h_ready = acc_full + 2;             // [1]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(h_ready + 1);
   volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -108,9 +108,9 @@ ccm_fused_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_constan
       mbar_init(&w_full[s], 1);
       mbar_init(&w_empty[s], 1);
     }
-    mbar_init(acc_full, 1);
+    mbar_init(&acc_full[0], 1);
+    mbar_init(&acc_full[1], 1);
     mbar_init(h_ready, 128);
-    mbar_init(acc_free, 128);
     *s_abort = (smem_u32(smem) & 1023u) != 0u;  // the swizzled tiles need 1024-byte alignment: nothing runs without it
     if (*s_abort) report(p.status, ST_BAD_INDEX);
     fence_barrier_init();
@@ -194,24 +194,19 @@ ccm_fused_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_constan
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------------- MMA issuer
-    // accumulators: GEMM1 and GEMM3 in columns [0, 128), GEMM2 in [128, 256).  The activation tile of GEMM2 is in
-    // the first 64 columns of the former, that of GEMM3 in the first 64 of the latter.
+    // accumulators: GEMM1 in columns [0, 128), GEMM2 and GEMM3 in [128, 256).  Both activation tiles are packed into
+    // [0, 64), so GEMM1 of the next tile may start as soon as GEMM3 is through and runs while this tile's rows are
+    // scattered.  Products are executed in the order they are issued; h_ready of the next tile says that the second
+    // accumulator has been read.
     if (lane == 0) {
       constexpr uint32_t idesc = make_idesc_bf16(128, 128);
       int ia = 0, iw = 0;
-      uint32_t h_phase = 0, free_phase = 0;
+      uint32_t h_phase = 0;
       bool ok = true;
       for (int tile = 0; tile < total_tiles && ok; ++tile) {
-        // the previous tile's last epilogue must have drained accumulator 0
-        if (tile > 0) {
-          ok = mbar_wait(acc_free, free_phase, p.status, ST_TIMEOUT_ACC_EMPTY);
-          free_phase ^= 1;
-          if (!ok) break;
-          tc_fence_after();
-        }
         for (int g = 0; g < 3 && ok; ++g) {
           const int nk = g == 0 ? nk1 : 2;
-          const uint32_t d_tmem = tmem_base + (g == 1 ? 128u : 0u);
+          const uint32_t d_tmem = tmem_base + (g == 0 ? 0u : 128u);
           if (g > 0) {
             ok = mbar_wait(h_ready, h_phase, p.status, ST_TIMEOUT_ACC_FULL);
             h_phase ^= 1;
@@ -233,14 +228,14 @@ ccm_fused_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_constan
               tc_commit(&a_empty[as]);
               ++ia;
             } else {
-              const uint32_t a_tmem = tmem_base + (g == 1 ? 0u : 128u) + uint32_t(i * 32);   // 64 packed columns of K
+              const uint32_t a_tmem = tmem_base + uint32_t(i * 32);   // 64 values of K, two to a column
 #pragma unroll
               for (int k = 0; k < 4; ++k)
                 tc_mma_f16_ts(d_tmem, a_tmem + uint32_t(8 * k), db + uint64_t(2 * k), idesc, (i > 0 || k > 0) ? 1u : 0u);
             }
             tc_commit(&w_empty[ws]);
           }
-          if (ok) tc_commit(acc_full);
+          if (ok) tc_commit(&acc_full[g == 0 ? 0 : 1]);
         }
       }
       if (!ok) *s_abort = 1;
@@ -248,37 +243,48 @@ ccm_fused_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_constan
   } else if (warp >= 6) {
     // ---------------------------------------------------------------------- gather of GEMM1's A operand
     // Thread gt copies 16-byte piece gt & 7 of rows (gt >> 3) + 16 q of every k-block; the eight threads of a row look up
-    // one row each and pass it on.  A stage is handed to the MMA warp once its copies, CCM_A_STAGES - 1 k-blocks back,
-    // have landed.
+    // one row each, a row of the group ahead, and pass it on.  A stage is handed to the MMA warp when its copies have
+    // landed: while stages are free CCM_A_STAGES - 1 k-blocks later, and all of them when the ring is full, so that the
+    // next tile's first k-blocks are announced before they are wanted.
     const int gt = threadIdx.x - 192;              // 0..127
     const int ch = gt & 7, r0 = gt >> 3;
     const uint32_t s_dst = smem_u32(smem) + r0 * 128 + ((ch ^ (r0 & 7)) << 4);     // (16 q keeps the low bits of the row)
     constexpr uint32_t NO_ROW = 0xffffffffu;
     const bf16* base = p.pool + ch * 8;
-    int it = 0;
-    bool ok = true;
-    for (int tile = 0; tile < total_tiles && ok; ++tile) {
+    const int my_r = r0 + 16 * ch;                 // the tile row this thread looks up: head my_r >> rj_shift
+    auto lookup = [&](int tile, int tok) -> uint32_t {       // pool row (block rows of all planes counted through)
       const int seg = tile < seg_tiles[0] ? 0 : 1;
-      const int j0 = (seg == 0 ? tile : tile - seg_tiles[0]) << rj_shift;
-      const int sp = seg_len[seg] / f;
-      const int my_r = r0 + 16 * ch;               // the row this thread looks up: head my_r >> rj_shift, output row my_j
-      const int my_j = j0 + (my_r & (RJ - 1));
+      const int j = ((seg == 0 ? tile : tile - seg_tiles[0]) << rj_shift) + (my_r & (RJ - 1));
+      if (j >= seg_len[seg] / f) return NO_ROW;
+      const int t = seg_in[seg] + j * f + tok;
+      const int blk = bt[t / p.block_size];
+      if (blk < 0 || blk >= p.num_blocks) {
+        report(p.status, ST_BAD_INDEX);
+        return NO_ROW;
+      }
+      return uint32_t(((plane + blk) * p.Hkv + h0 + (my_r >> rj_shift)) * p.block_size + t % p.block_size);
+    };
+    int it = 0, told = 0;                          // k-blocks asked for, and announced
+    bool ok = true;
+    uint32_t next = total_tiles > 0 ? lookup(0, 0) : NO_ROW;
+    for (int tile = 0; tile < total_tiles && ok; ++tile) {
       for (int tok = 0; tok < f && ok; ++tok) {
-        uint32_t mine = NO_ROW;                    // pool row (block rows of all planes counted through)
-        if (my_j < sp) {
-          const int t = seg_in[seg] + my_j * f + tok;
-          const int blk = bt[t / p.block_size];
-          if (blk < 0 || blk >= p.num_blocks) report(p.status, ST_BAD_INDEX);
-          else mine = uint32_t(((plane + blk) * p.Hkv + h0 + (my_r >> rj_shift)) * p.block_size + t % p.block_size);
-        }
         uint32_t row[8];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) row[q] = __shfl_sync(0xffffffffu, mine, q, 8);
+        for (int q = 0; q < 8; ++q) row[q] = __shfl_sync(0xffffffffu, next, q, 8);
+        if (tok + 1 < f) next = lookup(tile, tok + 1);
+        else if (tile + 1 < total_tiles) next = lookup(tile + 1, 0);
         for (int half = 0; half < CCM_D / 64; ++half, ++it) {
           const int stage = it % CCM_A_STAGES;
-          if (*s_abort || !mbar_wait(&a_empty[stage], ((it / CCM_A_STAGES) & 1) ^ 1, p.status, ST_TIMEOUT_EMPTY)) {
-            ok = false;
-            break;
+          const uint32_t ph = ((it / CCM_A_STAGES) & 1) ^ 1;
+          if (!mbar_try_wait(&a_empty[stage], ph)) {
+            cp_async_wait<0>();
+            fence_proxy_async();
+            for (; told < it; ++told) mbar_arrive(&a_full[told % CCM_A_STAGES]);
+            if (*s_abort || !mbar_wait(&a_empty[stage], ph, p.status, ST_TIMEOUT_EMPTY)) {
+              ok = false;
+              break;
+            }
           }
           const uint32_t sa = s_dst + stage * CCM_KB_BYTES;
 #pragma unroll
@@ -287,10 +293,10 @@ ccm_fused_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_constan
             cp_async16(sa + q * 16 * 128, base + (live ? size_t(row[q]) * CCM_D + half * 64 : size_t(0)), live);
           }
           cp_async_commit();
-          if (it >= CCM_A_STAGES - 1) {
+          if (it - told >= CCM_A_STAGES - 1) {
             cp_async_wait<CCM_A_STAGES - 1>();
             fence_proxy_async();
-            mbar_arrive(&a_full[(it + 1) % CCM_A_STAGES]);      // k-block it - (CCM_A_STAGES - 1)
+            mbar_arrive(&a_full[told++ % CCM_A_STAGES]);
           }
         }
         // the shuffles above count on whole warps: a thread that gave up takes the others with it
@@ -300,7 +306,7 @@ ccm_fused_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_constan
     cp_async_wait<0>();
     if (ok) {
       fence_proxy_async();
-      for (int n = max(0, it - (CCM_A_STAGES - 1)); n < it; ++n) mbar_arrive(&a_full[n % CCM_A_STAGES]);
+      for (; told < it; ++told) mbar_arrive(&a_full[told % CCM_A_STAGES]);
     } else {
       *s_abort = 1;
     }
@@ -309,7 +315,7 @@ ccm_fused_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_constan
     const int wt = threadIdx.x - 64;               // 0..127
     const int lane_group = warp & 3;
     const int row = lane_group * 32 + lane;        // TMEM lane == tile row owned by this thread
-    uint32_t acc_phase = 0;
+    uint32_t tile_phase = 0;
     bool ok = !*s_abort;
     for (int seg = 0; seg < 2 && ok; ++seg) {
       const int n = seg_len[seg];
@@ -345,17 +351,17 @@ ccm_fused_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_constan
       const bf16* b3 = p.b3 + ((long long)wlayer * 4 + bank) * CCM_D;
       for (int t = 0; t < seg_tiles[seg] && ok; ++t) {
         const int j0 = t << rj_shift;
-        // ---- epilogues 1 and 2: bias + ReLU, activation tile as packed bf16 over the accumulator's first 64 columns
-        //      (a thread has read columns 0 ... 2 c + 31 of its row when it writes columns c ... c + 15)
+        // ---- epilogues 1 and 2: bias + ReLU, activation tile as packed bf16 to columns [0, 64): over the accumulator of
+        //      GEMM1 (a thread has read columns 0 ... 2 c + 31 of its row when it writes columns c ... c + 15), and over
+        //      the first activation tile, which GEMM2 is done with
         for (int g = 0; g < 2 && ok; ++g) {
-          if (!mbar_wait(acc_full, acc_phase, p.status, ST_TIMEOUT_ACC_FULL)) {
+          if (!mbar_wait(&acc_full[g], g == 0 ? tile_phase : 0u, p.status, ST_TIMEOUT_ACC_FULL)) {
             ok = false;
             break;
           }
-          acc_phase ^= 1;
           tc_fence_after();
           const bf16* bias = g == 0 ? b1 : b2;
-          const uint32_t t_addr = tmem_base + (uint32_t(lane_group * 32) << 16) + (g == 1 ? 128u : 0u);
+          const uint32_t h_addr = tmem_base + (uint32_t(lane_group * 32) << 16), t_addr = h_addr + (g == 1 ? 128u : 0u);
 #pragma unroll 1
           for (int c4 = 0; c4 < 4; ++c4) {
             uint32_t rr[32];
@@ -374,7 +380,7 @@ ccm_fused_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_constan
                 u[q * 4 + e] = pack_bf16(a, b);
               }
             }
-            tmem_st_32x16(t_addr + uint32_t(c4 * 16), u);
+            tmem_st_32x16(h_addr + uint32_t(c4 * 16), u);
           }
           tmem_st_wait();
           tc_fence_before();
@@ -382,16 +388,16 @@ ccm_fused_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_constan
         }
         if (!ok) break;
         // ---- epilogue 3: bias, bf16, scatter the rows of this tile
-        if (!mbar_wait(acc_full, acc_phase, p.status, ST_TIMEOUT_ACC_FULL)) {
+        if (!mbar_wait(&acc_full[1], 1u, p.status, ST_TIMEOUT_ACC_FULL)) {
           ok = false;
           break;
         }
-        acc_phase ^= 1;
+        tile_phase ^= 1;
         tc_fence_after();
         {
           const int j = j0 + (row & (RJ - 1));
           bf16* dst = (j < sp) ? dst_ptr(h0 + (row >> rj_shift), out0 + j) : nullptr;
-          const uint32_t t_addr = tmem_base + (uint32_t(lane_group * 32) << 16);
+          const uint32_t t_addr = tmem_base + (uint32_t(lane_group * 32) << 16) + 128u;
 #pragma unroll 1
           for (int c4 = 0; c4 < 4; ++c4) {
             uint32_t rr[32];
@@ -413,8 +419,7 @@ ccm_fused_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_constan
             }
           }
         }
-        tc_fence_before();
-        mbar_arrive(acc_free);
+        tc_fence_before();                       // (h_ready of the next tile follows)
       }
       if (!ok) break;
       // ---- remainder rows of the segment move behind the compressed rows (fewer than f rows)
