@@ -122,6 +122,26 @@ Tensor gemm(const Tensor& x, const Tensor& w, const c10::optional<Tensor>& bias,
   return out;
 }
 
+// residual + x @ w.T + bias in one kernel, or nothing (undefined) where the sizes or layouts are not that kernel's
+c10::optional<Tensor> gemm_residual(const Tensor& x, const Tensor& w, const Tensor& bias, const Tensor& residual) {
+  for (const Tensor* t : {&x, &w, &bias, &residual}) check_bf16(*t, "operand");
+  TORCH_CHECK(x.dim() == 2 && w.dim() == 2 && residual.dim() == 2 && x.size(1) == w.size(1), "gemm expects 2-D operands with one inner size");
+  const int64_t M = x.size(0), K = x.size(1), N = w.size(0);
+  TORCH_CHECK(residual.size(0) == M && residual.size(1) == N && bias.numel() == N && bias.is_contiguous(), "bad bias or residual");
+  TORCH_CHECK(x.stride(1) == 1 && w.stride(1) == 1 && residual.stride(1) == 1, "operands must be row-major (unit inner stride)");
+  TORCH_CHECK(K % 8 == 0 && x.stride(0) % 8 == 0 && w.stride(0) % 8 == 0, "K and the row pitches must be multiples of 8 elements");
+  c10::cuda::CUDAGuard guard(x.device());
+  Tensor out = torch::empty({M, N}, x.options());
+  auto& ws = workspace(x.get_device());
+  fc::GemmWorkspace gw;
+  gw.status = ws.raw.status;
+  cudaStream_t stream = at::cuda::getCurrentCUDAStream();
+  if (!fc::gemm_bf16_residual(x.data_ptr(), w.data_ptr(), out.data_ptr(), bias.data_ptr(), residual.data_ptr(), int(M), int(N),
+                              int(K), x.stride(0), w.stride(0), out.stride(0), residual.stride(0), gw, sm_limit_for(stream), stream))
+    return c10::nullopt;
+  return out;
+}
+
 // Launches the GEMM of x @ w.T.  Decode-size inputs may leave fp32 partial sums in the workspace
 // instead of a finished result: returns the number of K splits (1 = `out` holds the result).
 static int gemm_maybe_partial(const Tensor& x, const Tensor& w, Tensor& out, DeviceWorkspace& ws,
@@ -494,6 +514,7 @@ void set_fused_epilogues(bool on) { g_fused_epilogues = on ? 1 : 0; }
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm", &gemm, "y = act(x @ w.T + bias) on tcgen05", py::arg("x"), py::arg("w"), py::arg("bias") = py::none(),
         py::arg("act") = 0, py::arg("out") = py::none());
+  m.def("gemm_residual", &gemm_residual);
   m.def("linear_add_rms_norm", &linear_add_rms_norm);
   m.def("linear_silu_mul", &linear_silu_mul);
   m.def("rms_norm", &rms_norm);

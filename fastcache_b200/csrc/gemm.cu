@@ -128,12 +128,12 @@ struct SmemLayout {
 
 // GLU: gated epilogue, out = act(gate) * up of w = [gate; up]
 enum Glu : int { GLU_NONE = 0, GLU_SILU = 1, GLU_GELU_TANH = 2, GLU_CLAMPED = 3 };   // GLU_GELU_TANH takes a bias [gate | up]
-enum GemmForm : int { GF_PLAIN = 0, GF_WIDE = 1, GF_ACC = 2, GF_GROUPED = 3, GF_XIELU = 4 };
+enum GemmForm : int { GF_PLAIN = 0, GF_WIDE = 1, GF_ACC = 2, GF_GROUPED = 3, GF_XIELU = 4, GF_RESIDUAL = 5 };
 
 template <int BN, int STAGES, int GLU = GLU_NONE, int FORM = GF_PLAIN, bool STAGED = false>
 __global__ void __launch_bounds__(gemm_threads(STAGED), 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
-                 const __grid_constant__ CUtensorMap tma_c, const GemmParams p) {
+                 const __grid_constant__ CUtensorMap tma_c, const __grid_constant__ CUtensorMap tma_r, const GemmParams p) {
   using L = SmemLayout<BN, STAGES, STAGED>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -141,7 +141,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   uint64_t* empty_bar = full_bar + STAGES;
   uint64_t* acc_full = empty_bar + STAGES;
   uint64_t* acc_empty = acc_full + 2;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  uint64_t* res_full = acc_empty + 2;              // GF_RESIDUAL, one per epilogue group
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(res_full + 2);
   volatile int* s_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);  // [0] abort
 
   const int warp = threadIdx.x >> 5;
@@ -157,6 +158,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     for (int a = 0; a < 2; ++a) {
       mbar_init(&acc_full[a], 1);
       mbar_init(&acc_empty[a], STAGED ? 256 : 128);
+      mbar_init(&res_full[a], 1);
     }
     s_flag[0] = 0;
     fence_barrier_init();
@@ -302,7 +304,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     auto group_bar = [&] { asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory"); };
     constexpr int GROUPS = STAGED ? 2 : 1;
     int acc = 0;
-    uint32_t acc_phase = 0;
+    uint32_t acc_phase = 0, res_phase = 0;
 
     // bias and activation of 32 values, columns col ... col + 31
     auto finish = [&](float (&v)[32], int col, bool whole) {
@@ -435,12 +437,26 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
 #pragma unroll 1
         for (int sl = group; sl < BN / SLAB; sl += GROUPS) {
           const int col = n_blk * BN + sl * SLAB;
+          if constexpr (FORM == GF_RESIDUAL) {           // what is added arrives in the slab while the accumulator is read
+            slab_free();
+            if (leader && col < p.N) {
+              mbar_expect_tx(&res_full[group], SLAB_BYTES);
+              tma_load_2d(slab, &tma_r, &res_full[group], col, row0);
+            }
+          }
           uint32_t r[2][32];
           tmem_ld_32x32(t_addr + uint32_t(sl * SLAB), r[0]);
           tmem_ld_32x32(t_addr + uint32_t(sl * SLAB + 32), r[1]);
           tmem_ld_wait();
           if (sl + GROUPS >= BN / SLAB) acc_read();
-          slab_free();
+          if constexpr (FORM == GF_RESIDUAL) {
+            if (col < p.N) {
+              if (!mbar_wait(&res_full[group], res_phase, p.status, ST_TIMEOUT_FULL)) s_flag[0] = 1;   // (reported; no barrier is skipped)
+              res_phase ^= 1;
+            }
+          } else {
+            slab_free();
+          }
 #pragma unroll
           for (int half = 0; half < 2; ++half) {
             float v[32];
@@ -448,6 +464,18 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
 #pragma unroll
             for (int t = 0; t < 32; ++t) v[t] = __uint_as_float(r[half][t]);
             finish(v, col + half * 32, col + SLAB <= p.N);
+            if constexpr (FORM == GF_RESIDUAL) {
+#pragma unroll
+              for (int q = 0; q < 4; ++q) {
+                const uint4 a = *reinterpret_cast<const uint4*>(slab + row * 128 + (((half * 4 + q) ^ (row & 7)) << 4));
+                const uint32_t w[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                  v[q * 8 + 2 * e] += __uint_as_float(w[e] << 16);
+                  v[q * 8 + 2 * e + 1] += __uint_as_float(w[e] & 0xffff0000u);
+                }
+              }
+            }
 #pragma unroll
             for (int t = 0; t < 16; ++t) u[t] = pack_bf16(v[2 * t], v[2 * t + 1]);
             park(u, half);
@@ -581,8 +609,8 @@ CUtensorMap make_tmap_bf16_3d(const void* base, uint64_t n0, uint64_t n1, uint64
 }
 
 template <int BN, int STAGES, int GLU, int FORM, bool STAGED>
-static void launch_form(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const GemmParams& p, int grid,
-                        cudaStream_t stream) {
+static void launch_form(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const CUtensorMap& tr,
+                        const GemmParams& p, int grid, cudaStream_t stream) {
   using L = SmemLayout<BN, STAGES, STAGED>;
   auto kern = gemm_bf16_kernel<BN, STAGES, GLU, FORM, STAGED>;
   // the attribute belongs to the (function, device) pair: remember it per device, not per process
@@ -595,7 +623,7 @@ static void launch_form(const CUtensorMap& ta, const CUtensorMap& tb, const CUte
     if (e != cudaSuccess) throw std::runtime_error(std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
     configured.fetch_or(bit, std::memory_order_relaxed);
   }
-  kern<<<grid, gemm_threads(STAGED), L::TOTAL, stream>>>(ta, tb, tc, p);
+  kern<<<grid, gemm_threads(STAGED), L::TOTAL, stream>>>(ta, tb, tc, tr, p);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) throw std::runtime_error(std::string("gemm launch: ") + cudaGetErrorString(e));
 }
@@ -608,11 +636,11 @@ static void launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const GemmP
   if constexpr (FORM == GF_PLAIN || FORM == GF_XIELU) {
     if ((p.K <= STAGED_K || p.total_work <= 2 * grid) && p.ldc % 8 == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0) {
       const CUtensorMap tc = make_tmap_bf16_2d(p.C, p.M, p.N, p.ldc, BM, SLAB);
-      launch_form<BN, STAGES, GLU, FORM, true>(ta, tb, tc, p, grid, stream);
+      launch_form<BN, STAGES, GLU, FORM, true>(ta, tb, tc, ta, p, grid, stream);
       return;
     }
   }
-  launch_form<BN, STAGES, GLU, FORM, false>(ta, tb, ta, p, grid, stream);        // (the last map is not read)
+  launch_form<BN, STAGES, GLU, FORM, false>(ta, tb, ta, ta, p, grid, stream);    // (the last two maps are not read)
 }
 
 static int g_num_sms = 0;
@@ -707,6 +735,24 @@ static GemmParams prefill_params(void* c, int M, int N, int K, long long ldc, co
   p.num_m = (M + BM - 1) / BM;
   p.group_m = 16;
   return p;
+}
+
+// C = residual + X W^T + bias with one rounding.  False (nothing launched) where the staged form cannot run: decode sizes,
+// narrow outputs, and outputs or residuals that TMA cannot describe.
+bool gemm_bf16_residual(const void* x, const void* w, void* c, const void* bias, const void* residual, int M, int N, int K,
+                        long long ldx, long long ldw, long long ldc, long long ldr, const GemmWorkspace& ws, int sm_limit,
+                        cudaStream_t stream) {
+  constexpr int BN = 256;
+  auto fits = [](const void* p, long long ld) { return ld % 8 == 0 && (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+  if (M <= 256 || N < BN || K <= 0 || !fits(c, ldc) || !fits(residual, ldr)) return false;
+  GemmParams p = prefill_params(c, M, N, K, ldc, ws);
+  p.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
+  p.num_n = (N + BN - 1) / BN;
+  p.total_work = p.num_m * p.num_n;
+  launch_form<BN, 4, GLU_NONE, GF_RESIDUAL, true>(
+      make_tmap_bf16_2d(x, M, K, ldx, BM, BK), make_tmap_bf16_2d(w, N, K, ldw, BN, BK), make_tmap_bf16_2d(c, M, N, ldc, BM, SLAB),
+      make_tmap_bf16_2d(residual, M, N, ldr, BM, SLAB), p, std::min(p.total_work, sm_limit > 0 ? sm_limit : gemm_num_sms()), stream);
+  return true;
 }
 
 void gemm_bf16_wide(const void* x, const void* w, void* c, int M, int N, int K, long long ldx, long long ldw, long long ldc,

@@ -44,8 +44,12 @@ class VLinear(nn.Module):
         self.weight = _param(out_f, in_f)
         self.bias = _param(out_f) if bias else None
 
-    def forward(self, x: torch.Tensor, act: str = "none") -> torch.Tensor:
-        return ops.linear(x, self.weight, self.bias, act)
+    def forward(self, x: torch.Tensor, act: str = "none", residual: Optional[torch.Tensor] = None) -> torch.Tensor:
+        """With `residual` (and no activation) the sum of both, added in the epilogue."""
+        if residual is not None and self.bias is not None and act == "none":
+            return ops.linear_add(x, self.weight, self.bias, residual)
+        y = ops.linear(x, self.weight, self.bias, act)
+        return y if residual is None else residual + y
 
 
 class VLayerNorm(nn.Module):
@@ -71,13 +75,13 @@ class VisionAttention(nn.Module):
         self._qkv_w = torch.cat([self.q_proj.weight, self.k_proj.weight, self.v_proj.weight], dim=0).contiguous()
         self._qkv_b = torch.cat([self.q_proj.bias, self.k_proj.bias, self.v_proj.bias], dim=0).contiguous()
 
-    def forward(self, x: torch.Tensor, key_mask: Optional[torch.Tensor] = None) -> torch.Tensor:
+    def forward(self, x: torch.Tensor, key_mask: Optional[torch.Tensor] = None, residual: Optional[torch.Tensor] = None) -> torch.Tensor:
         B, S, C = x.shape
         if self._qkv_w is None:
             self.fuse()
         qkv = ops.linear(x.reshape(B * S, C), self._qkv_w, self._qkv_b).view(B, S, 3, self.heads, self.head_dim)
         o = ops.dense_attention(qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2], self.head_dim ** -0.5, key_mask)
-        return self.out_proj(o.reshape(B * S, C)).view(B, S, C)
+        return self.out_proj(o.reshape(B * S, C), residual=None if residual is None else residual.reshape(B * S, C)).view(B, S, C)
 
 
 class VisionMLP(nn.Module):
@@ -85,8 +89,8 @@ class VisionMLP(nn.Module):
         super().__init__()
         self.fc1, self.fc2, self.act = VLinear(dim, inter), VLinear(inter, dim), act
 
-    def forward(self, x: torch.Tensor) -> torch.Tensor:
-        return self.fc2(self.fc1(x, self.act))
+    def forward(self, x: torch.Tensor, residual: Optional[torch.Tensor] = None) -> torch.Tensor:
+        return self.fc2(self.fc1(x, self.act), residual=residual)
 
 
 class VisionLayer(nn.Module):
@@ -98,8 +102,12 @@ class VisionLayer(nn.Module):
 
     def forward(self, x: torch.Tensor, key_mask: Optional[torch.Tensor] = None) -> torch.Tensor:
         B, S, C = x.shape
-        x = x + self.self_attn(self.layer_norm1(x), key_mask)
-        return x + self.mlp(self.layer_norm2(x).reshape(B * S, C)).view(B, S, C)
+        attn, mlp = self.self_attn, self.mlp
+        if attn._forward_hooks or attn.out_proj._forward_hooks or mlp._forward_hooks or mlp.fc2._forward_hooks:
+            x = x + attn(self.layer_norm1(x), key_mask)             # whoever watches a block sees its own output
+            return x + mlp(self.layer_norm2(x).reshape(B * S, C)).view(B, S, C)
+        x = attn(self.layer_norm1(x), key_mask, residual=x)
+        return mlp(self.layer_norm2(x).reshape(B * S, C), residual=x.reshape(B * S, C)).view(B, S, C)
 
 
 class _Encoder(nn.Module):

@@ -76,6 +76,18 @@ def linear(x, weight, bias=None, act: str = "none", out: Optional[torch.Tensor] 
     return y
 
 
+def linear_add(x, weight, bias, residual):
+    """residual + x @ weight.T + bias, [T, N]; the prompt-size CUDA GEMM adds in its epilogue."""
+    if x.is_cuda:
+        from ..parallel.fused import get_fused_comm
+        if get_fused_comm() is None and residual.dtype == x.dtype and x.stride(-1) == 1 and residual.stride(-1) == 1:
+            y = ext().gemm_residual(x, weight, bias, residual)
+            if y is not None:
+                _n()
+                return y
+    return residual + linear(x, weight, bias)
+
+
 def linear_add_rms_norm(x, weight, bias, residual, norm_weight, eps) -> Tuple[torch.Tensor, torch.Tensor]:
     """residual += x @ weight.T (+ bias); returns (RMSNorm(residual), residual).  On CUDA the split-K
     partial sums of a decode-size GEMM are reduced inside the norm kernel (two launches in all)."""

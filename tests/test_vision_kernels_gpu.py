@@ -1,0 +1,68 @@
+"""Prompt-size GEMM epilogues and dense attention at the edges of their tiles."""
+import pytest
+import torch
+
+from fastcache_b200 import ops
+from fastcache_b200.ops import reference as ref
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _normal(*shape, seed=0, scale=1.0):
+    return (torch.randn(*shape, generator=torch.Generator().manual_seed(seed)) * scale).to(torch.bfloat16).to(DEV)
+
+
+def _clean():
+    assert ops.ext().read_status(torch.cuda.current_device()) == 0
+
+
+def _close(got, want, K):
+    # one rounding to bf16, and a sum of K products in 32 bits of terms whose mean square is that of the result / K
+    bound = 2.0 ** -8 * want.abs() + K * 2.0 ** -24 * want.pow(2).mean().sqrt() + 1e-6
+    assert ((got.double() - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("M", [257, 384, 1000])
+@pytest.mark.parametrize("N,K", [(256, 64), (264, 1024), (328, 2048), (1152, 4304), (3000, 136)])
+def test_staged_epilogue_at_ragged_sizes(M, N, K):
+    x, w, b, r = _normal(M, K, seed=1), _normal(N, K, seed=2, scale=K ** -0.5), _normal(N, seed=3), _normal(M, N, seed=4)
+    sums = x.double() @ w.double().T + b.double()
+    _close(ops.linear(x, w, b), sums, K)
+    _close(ops.linear_add(x, w, b, r), sums + r.double(), K)
+    wide = torch.full((M, N + 24), 7.0, dtype=torch.bfloat16, device=DEV)          # what lies beside the output stays
+    ops.linear(x, w, b, out=wide[:, 8:N + 8])
+    _close(wide[:, 8:N + 8], sums, K)
+    assert (wide[:, :8] == 7).all() and (wide[:, N + 8:] == 7).all()
+    odd = torch.full((M, N + 5), 7.0, dtype=torch.bfloat16, device=DEV)            # a pitch that only the plain epilogue takes
+    ops.linear(x, w, b, out=odd[:, :N])
+    _close(odd[:, :N], sums, K)
+    assert (odd[:, N:] == 7).all()
+    _clean()
+
+
+def test_added_residual_of_few_rows_and_other_pitches():
+    x, w, b = _normal(300, 256, seed=1), _normal(512, 256, seed=2, scale=0.06), _normal(512, seed=3)
+    sums = x.double() @ w.double().T + b.double()
+    for rows, r in ((20, _normal(20, 512, seed=4)), (300, _normal(300, 520, seed=5)[:, :512]), (300, _normal(300, 515, seed=6)[:, :512])):
+        got = ops.linear_add(x[:rows], w, b, r)
+        want = sums[:rows] + r.double()
+        assert ((got.double() - want).abs() <= 2.0 ** -7 * (sums[:rows].abs() + want.abs()) + 1e-5).all()      # two roundings at most
+
+
+@pytest.mark.parametrize("D", [8, 40, 64, 72, 80, 96, 128])
+@pytest.mark.parametrize("Sq,Sk", [(1, 1), (127, 63), (128, 64), (129, 65), (256, 127), (257, 128), (130, 129), (64, 400)])
+def test_dense_attention_at_tile_edges(D, Sq, Sk):
+    B, H = 2, 3
+    q, k, v = (_normal(B, n, H, D, seed=i) for i, n in enumerate((Sq, Sk, Sk)))
+    hole = torch.rand(B, Sk, generator=torch.Generator().manual_seed(9)) < 0.7
+    hole[:, Sk // 2] = True
+    hole[1, :] = hole[1, :] & (torch.arange(Sk) >= Sk // 2)                         # a first tile without a key
+    for mask in (None, hole.to(DEV)):
+        got = ops.dense_attention(q, k, v, D ** -0.5, mask, impl=2)
+        want = ref.dense_attention(q.float(), k.float(), v.float(), D ** -0.5, mask)
+        # P and the result in bf16: 2^-8 of the largest value each
+        assert (got.float() - want).abs().max() <= 2 * 2.0 ** -8 * v.float().abs().max()
+    nothing = torch.zeros(B, Sk, dtype=torch.bool, device=DEV)
+    assert torch.equal(ops.dense_attention(q, k, v, D ** -0.5, nothing, impl=2), torch.zeros_like(q))
+    _clean()
