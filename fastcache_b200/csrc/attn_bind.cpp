@@ -142,25 +142,16 @@ Tensor dense_attention(const Tensor& q, const Tensor& k, const Tensor& v, double
                      fc::dense_attention_tc_supported(int(B), int(Sq), int(Sk), int(H), int(D), qs, ks, vs);
   TORCH_CHECK(impl != 2 || tc_ok || B == 0 || Sq == 0, "dense attention: the tcgen05 kernel cannot take these strides");
   auto stream = at::cuda::getCurrentCUDAStream();
-  if (impl != 1 && tc_ok) {
-    const uint8_t* mask = nullptr;
-    Tensor mask_p;
-    const int64_t ld = (Sk + 127) / 128 * 128;
-    if (has_mask) {
-      mask_p = torch::zeros({B, ld}, key_mask->options().dtype(torch::kUInt8));
-      mask_p.narrow(1, 0, Sk).copy_(*key_mask);
-      mask = reinterpret_cast<const uint8_t*>(mask_p.data_ptr());
-    }
-    fc::launch_dense_attention_tc(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), mask, int(ld), int(B),
-                                  int(Sq), int(Sk), int(H), int(D), qs, ks, vs, float(scale),
-                                  status_ptr(q.get_device()), stream);
-    return out;
-  }
   const uint8_t* mask = nullptr;
   Tensor mask_c;
   if (has_mask) {
     mask_c = key_mask->contiguous();
     mask = reinterpret_cast<const uint8_t*>(mask_c.data_ptr());
+  }
+  if (impl != 1 && tc_ok) {
+    fc::launch_dense_attention_tc(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), mask, int(B), int(Sq), int(Sk),
+                                  int(H), int(D), qs, ks, vs, float(scale), status_ptr(q.get_device()), stream);
+    return out;
   }
   fc::launch_dense_attention(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), mask, int(B), int(Sq),
                              int(Sk), int(H), int(D), qs, ks, vs, float(scale), stream);

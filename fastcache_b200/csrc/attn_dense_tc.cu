@@ -2,14 +2,21 @@
 //
 // out[b, s, h, :] = softmax(q[b, s, h, :] . k[b, :, h, :]^T * scale  (+ key mask)) v[b, :, h, :]
 //
-// Same structure as the causal prefill kernel (attn_prefill_tc2.cu): one CTA owns 256 query rows of one head
-// of one batch element (tiles A and B of 128 rows, in ping-pong) and walks the keys in tiles of 128 rows; S, P
-// and O live in tensor memory:
-//     S_A [0,128)  S_B [128,256)  O_A [256,256+DP)  O_B [256+DP,256+2DP)
-//   warp 0       TMA: both Q tiles once, then K and V tiles into 2-stage rings (128-byte swizzle)
-//   warp 1       tcgen05.mma issuer: S_X = Q_X K^T from shared memory, O_X += P_X V with P_X read from tensor
-//                memory (packed bf16 over the first 64 columns of S_X) and V as an MN-major operand
-//   warps 2-5    softmax of tile A, warps 6-9 of tile B, one query row per thread, O rescaled lazily
+// One CTA owns 128 query rows of one head of one batch element and walks the keys in tiles of 128 rows; two CTAs share an
+// SM (256 columns of tensor memory and at most 98 KB of shared memory each), so one tile's products run under the
+// other's softmax, and 128-row units leave less of the last wave empty than pairs of them.  S, P and O live in tensor
+// memory:  S [0, 128), then P as packed bf16 over its first 64 columns;  O [128, 128 + DP)
+//   warp 0       TMA: the Q tile once, then K and V tiles (128-byte swizzle; two stages each for DP = 64, one for
+//                DP = 128, where the copy of the next tile has the whole softmax to arrive)
+//   warp 1       tcgen05.mma issuer: S = Q K^T from shared memory, O += P V with P read from tensor memory and V as an
+//                MN-major operand
+//   warps 2-5    softmax, one query row per thread, O rescaled lazily
+//
+// What bounds it: MUFU (one exp2 per score, 1024 clocks per tile and SM) and, above that, the chain S -> softmax -> P -> PV
+// -> next S of a tile, of which an SM has two.  5 x 961 rows, 16 heads of 72, ragged key mask: 80 us with two query tiles
+// per CTA, one CTA per SM (320 CTAs on 148 SMs) and the mask padded by two launches of its own, 69 us so.  15 x 577 rows,
+// 16 heads of 64: 63 us both ways.  Two threads per row, 64 columns each, were slower (69 us, 73 us): they have to
+// meet for the maximum of a row.
 //
 // The operands are [B, S, H, D] views with arbitrary strides (the packed qkv output of one GEMM is read in place),
 // described to TMA as 4-D tensors (D, H, S, B).  The head dimension is padded to DP = 64 or 128 columns by the
@@ -34,10 +41,9 @@ namespace fc {
 
 using bf16 = __nv_bfloat16;
 
-constexpr int DT_BM = 128;             // rows per query tile (two tiles per CTA)
+constexpr int DT_BM = 128;             // query rows per CTA
 constexpr int DT_BN = 128;
-constexpr int DT_THREADS = 320;
-constexpr int DT_THREADS_SINGLE = 192;
+constexpr int DT_THREADS = 192;
 constexpr int DT_SUB_BYTES = 128 * 64 * 2;              // one [128 x 64] sub-tile
 constexpr float DT_RESCALE_THRESHOLD = 8.f;             // log2 units
 
@@ -67,61 +73,60 @@ __device__ __forceinline__ void dt_tma_load_4d(void* smem, const CUtensorMap* m,
 
 struct DenseTcParams {
   bf16* out;                 // [B, Sq, H, D] contiguous
-  const uint8_t* key_mask;   // [B, mask_ld] (1 = attend), rows padded with zeros to a multiple of 128; or null
-  int mask_ld;
+  const uint8_t* key_mask;   // [B, Sk] (0 = do not attend), or null
   int Sq, Sk, H, D;
   float scale_log2;
   uint32_t* status;
 };
 
-// PAIR: two query tiles per CTA in ping-pong, one CTA per SM (512 columns of tensor memory).  Otherwise one query
-// tile per CTA, half the tensor memory and (for DP = 64) half the shared memory, so that two CTAs share an SM:
-// the start-up and the epilogue of one overlap the key loop of the other, and a sequence of 577 rows costs five
-// tiles instead of three pairs.
-template <int DP, bool PAIR>
-__global__ void __launch_bounds__(PAIR ? DT_THREADS : DT_THREADS_SINGLE, PAIR ? 1 : 2)
+template <int DP>
+struct DtSmem {
+  static constexpr int TILE_BYTES = DP / 64 * DT_SUB_BYTES;
+  static constexpr int STAGES = DP == 64 ? 2 : 1;                       // of K and of V
+  static constexpr int BAR_OFF = (1 + 2 * STAGES) * TILE_BYTES;
+  static constexpr int TOTAL = BAR_OFF + 128 + 1024;
+};
+
+template <int DP>
+__global__ void __launch_bounds__(DT_THREADS, 2)
 dense_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                      const __grid_constant__ CUtensorMap tm_v, const DenseTcParams p) {
-  constexpr int SUBS = DP / 64;
-  constexpr int TILE_BYTES = SUBS * DT_SUB_BYTES;
-  constexpr int NQ = PAIR ? 2 : 1;                     // query tiles per CTA
-  constexpr uint32_t O_BASE = PAIR ? 256u : 128u;      // first column of O_A
-  constexpr uint32_t TMEM_COLS = PAIR ? 512u : 256u;
+  using L = DtSmem<DP>;
+  constexpr int TILE_BYTES = L::TILE_BYTES, STAGES = L::STAGES;
+  constexpr uint32_t O_BASE = 128u;                    // first column of O
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* s_q = smem;                                // 2 tiles
-  uint8_t* s_k = s_q + NQ * TILE_BYTES;               // 2 stages
-  uint8_t* s_v = s_k + 2 * TILE_BYTES;                // 2 stages
-  uint64_t* bars = reinterpret_cast<uint64_t*>(s_v + 2 * TILE_BYTES);
+  uint8_t* s_q = smem;
+  uint8_t* s_k = s_q + TILE_BYTES;
+  uint8_t* s_v = s_k + STAGES * TILE_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
   uint64_t* q_full = bars;            // [1]
   uint64_t* k_full = bars + 1;        // [2]
   uint64_t* k_empty = bars + 3;       // [2]
   uint64_t* v_full = bars + 5;        // [2]
   uint64_t* v_empty = bars + 7;       // [2]
-  uint64_t* s_full = bars + 9;        // [2] per query tile
-  uint64_t* p_ready = bars + 11;      // [2] per query tile (128 arrivals)
-  uint64_t* o_done = bars + 13;       // [2] per query tile
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
+  uint64_t* s_full = bars + 9;        // [1]
+  uint64_t* p_ready = bars + 10;      // [1] (128 arrivals)
+  uint64_t* o_done = bars + 11;       // [1]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
   volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int b = blockIdx.z, h = blockIdx.y;
-  const int q0 = blockIdx.x * (NQ * DT_BM);
-  const bool act_b = PAIR && q0 + DT_BM < p.Sq;
+  const int q0 = blockIdx.x * DT_BM;
   const int n_tiles = (p.Sk + DT_BN - 1) / DT_BN;
-  const int n_a = n_tiles, n_b = act_b ? n_tiles : 0;
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
-    for (int s = 0; s < 2; ++s) {
+    for (int s = 0; s < STAGES; ++s) {
       mbar_init(&k_full[s], 1);
       mbar_init(&k_empty[s], 1);
       mbar_init(&v_full[s], 1);
       mbar_init(&v_empty[s], 1);
-      mbar_init(&s_full[s], 1);
-      mbar_init(&p_ready[s], 128);
-      mbar_init(&o_done[s], 1);
     }
+    mbar_init(s_full, 1);
+    mbar_init(p_ready, 128);
+    mbar_init(o_done, 1);
     *s_abort = 0;
     fence_barrier_init();
     tma_prefetch_desc(&tm_q);
@@ -129,7 +134,7 @@ dense_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     tma_prefetch_desc(&tm_v);
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, TMEM_COLS);
+    tmem_alloc(tmem_slot, 256);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -140,133 +145,114 @@ dense_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA loader
     if (lane == 0) {
-      mbar_expect_tx(q_full, (act_b ? 2 : 1) * TILE_BYTES);
-      for (int x = 0; x < (act_b ? 2 : 1); ++x)
-        for (int sub = 0; sub < SUBS; ++sub)
-          dt_tma_load_4d(s_q + x * TILE_BYTES + sub * DT_SUB_BYTES, &tm_q, q_full, sub * 64, h, q0 + x * DT_BM, b);
-      for (int j = 0; j < n_tiles && !*s_abort; ++j) {
-        const int st = j & 1;
-        const uint32_t ph = ((j >> 1) & 1) ^ 1;
-        for (int which = 0; which < 2; ++which) {
-          uint64_t* full = which == 0 ? &k_full[st] : &v_full[st];
-          uint64_t* empty = which == 0 ? &k_empty[st] : &v_empty[st];
-          if (!mbar_wait(empty, ph, p.status, ST_TIMEOUT_EMPTY)) {
-            *s_abort = 1;
-            break;
-          }
-          uint8_t* dst = (which == 0 ? s_k : s_v) + st * TILE_BYTES;
-          const CUtensorMap* tm = which == 0 ? &tm_k : &tm_v;
-          mbar_expect_tx(full, TILE_BYTES);           // rows and columns outside the tensor count as copied zeros
-          for (int sub = 0; sub < SUBS; ++sub)
-            dt_tma_load_4d(dst + sub * DT_SUB_BYTES, tm, full, sub * 64, h, j * DT_BN, b);
-        }
+      auto load = [&](uint8_t* dst, const CUtensorMap* tm, uint64_t* full, int row) {
+        mbar_expect_tx(full, TILE_BYTES);             // rows and columns outside the tensor count as copied zeros
+        for (int sub = 0; sub < DP / 64; ++sub)
+          dt_tma_load_4d(dst + sub * DT_SUB_BYTES, tm, full, sub * 64, h, row, b);
+      };
+      load(s_q, &tm_q, q_full, q0);
+      int nk = 0, nv = 0;
+      for (int j = 0; j < n_tiles; ++j) {
+        const int st = j % STAGES;
+        const uint32_t ph = ((j / STAGES) & 1) ^ 1;
+        if (*s_abort || !mbar_wait(&k_empty[st], ph, p.status, ST_TIMEOUT_EMPTY)) break;
+        load(s_k + st * TILE_BYTES, &tm_k, &k_full[st], j * DT_BN);
+        ++nk;
+        if (*s_abort || !mbar_wait(&v_empty[st], ph, p.status, ST_TIMEOUT_EMPTY)) break;
+        load(s_v + st * TILE_BYTES, &tm_v, &v_full[st], j * DT_BN);
+        ++nv;
+      }
+      if (nv < n_tiles) {
+        // unwind: what was asked for lands before the CTA may exit
+        *s_abort = 1;
+        mbar_wait(q_full, 0, nullptr, 0);
+        for (int j = max(0, nk - STAGES); j < nk; ++j) mbar_wait(&k_full[j % STAGES], (j / STAGES) & 1, nullptr, 0);
+        for (int j = max(0, nv - STAGES); j < nv; ++j) mbar_wait(&v_full[j % STAGES], (j / STAGES) & 1, nullptr, 0);
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     if (lane == 0) {
       constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, false, false);
-      constexpr uint32_t idesc_o = make_idesc_bf16(128, DP, false, true);      // B (= V) is MN-major
+      // B (= V) is MN-major; of the DP columns that the copy pads to, only the 16-column groups that hold some of D
+      const int d16 = (p.D + 15) / 16;
+      const uint32_t idesc_o = make_idesc_bf16(128, d16 * 16, false, true);
+      const uint32_t qa = smem_u32(s_q);
       bool ok = mbar_wait(q_full, 0, p.status, ST_TIMEOUT_FULL);
-      auto issue_s = [&](int x, int j) {
-        const int st = j & 1;
-        const uint32_t qa = smem_u32(s_q + x * TILE_BYTES), ka = smem_u32(s_k + st * TILE_BYTES);
+      auto issue_s = [&](int j) {
+        const int st = j % STAGES;
+        if (!mbar_wait(&k_full[st], (j / STAGES) & 1, p.status, ST_TIMEOUT_FULL)) return false;
+        tc_fence_after();
+        const uint32_t ka = smem_u32(s_k + st * TILE_BYTES);
 #pragma unroll
         for (int kk = 0; kk < DP / 16; ++kk) {
           const uint32_t off = uint32_t(kk >> 2) * DT_SUB_BYTES + uint32_t(kk & 3) * 32;
-          tc_mma_f16(tmem_base + uint32_t(x * 128), dt_sdesc(qa + off, 16, 1024), dt_sdesc(ka + off, 16, 1024),
-                     idesc_s, kk > 0 ? 1u : 0u);
+          if (kk < d16)
+            tc_mma_f16(tmem_base, dt_sdesc(qa + off, 16, 1024), dt_sdesc(ka + off, 16, 1024), idesc_s, kk > 0 ? 1u : 0u);
         }
-        tc_commit(&s_full[x]);
+        tc_commit(s_full);
+        tc_commit(&k_empty[st]);
+        return true;
       };
-      auto issue_pv = [&](int x, int j) {
-        const int st = j & 1;
+      if (ok) ok = issue_s(0);
+      for (int j = 0; j < n_tiles && ok; ++j) {
+        const int st = j % STAGES;
+        ok = mbar_wait(p_ready, uint32_t(j) & 1u, p.status, ST_TIMEOUT_FULL) &&
+             mbar_wait(&v_full[st], uint32_t(j / STAGES) & 1u, p.status, ST_TIMEOUT_FULL);
+        if (!ok) break;
+        tc_fence_after();
         const uint32_t va = smem_u32(s_v + st * TILE_BYTES);
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk) {
           const uint64_t db = dt_sdesc(va + uint32_t(kk) * 2048, DT_SUB_BYTES, 1024);
-          tc_mma_f16_ts(tmem_base + O_BASE + uint32_t(x * DP), tmem_base + uint32_t(x * 128) + uint32_t(kk * 8), db,
-                        idesc_o, (j > 0 || kk > 0) ? 1u : 0u);
+          tc_mma_f16_ts(tmem_base + O_BASE, tmem_base + uint32_t(kk * 8), db, idesc_o, (j > 0 || kk > 0) ? 1u : 0u);
         }
-        tc_commit(&o_done[x]);
-      };
-      if (ok) ok = mbar_wait(&k_full[0], 0, p.status, ST_TIMEOUT_FULL);
-      if (ok) {
-        tc_fence_after();
-        issue_s(0, 0);
-        if (act_b) issue_s(1, 0);
-        tc_commit(&k_empty[0]);
-      }
-      for (int j = 0; j < n_tiles && ok; ++j) {
-        const int st = j & 1;
-        const bool more = j + 1 < n_tiles;
-        bool v_waited = false, k_waited = false;
-        for (int x = 0; x < 2 && ok; ++x) {
-          const int n_x = x == 0 ? n_a : n_b;
-          if (j >= n_x) continue;
-          ok = mbar_wait(&p_ready[x], uint32_t(j) & 1u, p.status, ST_TIMEOUT_FULL);
-          if (ok && !v_waited) {
-            ok = mbar_wait(&v_full[st], uint32_t(j >> 1) & 1u, p.status, ST_TIMEOUT_FULL);
-            v_waited = true;
-          }
-          if (!ok) break;
-          tc_fence_after();
-          issue_pv(x, j);
-          if (j + 1 < n_x) {
-            if (!k_waited) {
-              ok = mbar_wait(&k_full[st ^ 1], uint32_t((j + 1) >> 1) & 1u, p.status, ST_TIMEOUT_FULL);
-              k_waited = true;
-              if (!ok) break;
-              tc_fence_after();
-            }
-            issue_s(x, j + 1);
-          }
-        }
-        if (!ok) break;
+        tc_commit(o_done);
         tc_commit(&v_empty[st]);
-        if (more && k_waited) tc_commit(&k_empty[st ^ 1]);
+        if (j + 1 < n_tiles) ok = issue_s(j + 1);      // after PV(j), whose P lies where S(j + 1) goes
       }
       if (!ok) *s_abort = 1;
     }
   } else {
-    // ------------------------------------------------ softmax of one query tile (x = 0: A, 1: B)
-    const int x = (warp - 2) >> 2;
-    const int n_x = x == 0 ? n_a : n_b;
+    // ------------------------------------------------ softmax, one query row per thread
     const int lane_group = warp & 3;                         // TMEM lanes this warp may touch
     const int row = lane_group * 32 + lane;
     const uint32_t lane_addr = uint32_t(lane_group * 32) << 16;
-    const uint32_t ts = tmem_base + lane_addr + uint32_t(x * 128);           // S_x, then P_x
-    const uint32_t to = tmem_base + lane_addr + O_BASE + uint32_t(x * DP);   // O_x
-    const int qrow = q0 + x * DT_BM + row;
-    const uint8_t* mrow = p.key_mask != nullptr ? p.key_mask + (long long)b * p.mask_ld : nullptr;
+    const uint32_t ts = tmem_base + lane_addr;               // S, then P
+    const uint32_t to = tmem_base + lane_addr + O_BASE;      // O
+    const int qrow = q0 + row;
+    const uint8_t* mrow = p.key_mask != nullptr ? p.key_mask + (long long)b * p.Sk : nullptr;
     float m_ref = 0.f, l = 0.f;
     bool ok = true;
-    for (int j = 0; j < n_x && ok; ++j) {
-      if (*s_abort || !mbar_wait(&s_full[x], uint32_t(j) & 1u, p.status, ST_TIMEOUT_ACC_FULL)) {
-        ok = false;
-        break;
+    for (int j = 0; j < n_tiles && ok; ++j) {
+      // keys that are not there or not attended to, looked up before the wait for S: lane t asks for key 32 c + t, all
+      // lanes get the 32 answers
+      const int col0 = j * DT_BN;
+      const bool some = mrow != nullptr || col0 + DT_BN > p.Sk;
+      uint32_t seen[4];
+      if (some) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const int key = col0 + c * 32 + lane;
+          seen[c] = __ballot_sync(0xffffffffu, key < p.Sk && (mrow == nullptr || mrow[key] != 0));
+        }
       }
+      ok = __all_sync(0xffffffffu, !*s_abort && mbar_wait(s_full, uint32_t(j) & 1u, p.status, ST_TIMEOUT_ACC_FULL));
+      if (!ok) break;
       tc_fence_after();
       uint32_t s[128];
 #pragma unroll
       for (int c = 0; c < 4; ++c) tmem_ld_32x32(ts + uint32_t(c * 32), *reinterpret_cast<uint32_t(*)[32]>(&s[c * 32]));
       tmem_ld_wait();
-      const int col0 = j * DT_BN;
-      if (mrow != nullptr) {
-        // the same 128 bytes for every row of the tile: broadcast loads, served by L1 after the first warp
-        const uint4* m4 = reinterpret_cast<const uint4*>(mrow + col0);
+      if (some) {
 #pragma unroll
-        for (int g = 0; g < 8; ++g) {
-          const uint4 mv = __ldg(m4 + g);
-          const uint32_t w[4] = {mv.x, mv.y, mv.z, mv.w};
+        for (int c = 0; c < 4; ++c) {
+          if (seen[c] != 0xffffffffu) {
 #pragma unroll
-          for (int t = 0; t < 16; ++t)
-            if (((w[t >> 2] >> ((t & 3) * 8)) & 0xffu) == 0u) s[g * 16 + t] = 0xff800000u;      // -inf
+            for (int t = 0; t < 32; ++t)
+              if (((seen[c] >> t) & 1u) == 0u) s[c * 32 + t] = 0xff800000u;      // -inf
+          }
         }
-      } else if (col0 + DT_BN > p.Sk) {
-#pragma unroll
-        for (int t = 0; t < 128; ++t)
-          if (col0 + t >= p.Sk) s[t] = 0xff800000u;
       }
       // four independent chains each (a single one is 128 dependent operations per tile)
       float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
@@ -279,9 +265,9 @@ dense_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       mx *= p.scale_log2;
       if (j == 0) {
         m_ref = (mx == -INFINITY) ? 0.f : mx;
-      } else if (__any_sync(__activemask(), mx > m_ref + DT_RESCALE_THRESHOLD)) {
+      } else if (__any_sync(0xffffffffu, mx > m_ref + DT_RESCALE_THRESHOLD)) {
         // some row of this warp outgrew its reference: bring O (complete up to tile j - 1) to the new one
-        if (!mbar_wait(&o_done[x], uint32_t(j - 1) & 1u, p.status, ST_TIMEOUT_ACC_FULL)) {
+        if (!mbar_wait(o_done, uint32_t(j - 1) & 1u, p.status, ST_TIMEOUT_ACC_FULL)) {
           ok = false;
           break;
         }
@@ -318,11 +304,11 @@ dense_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       tmem_st_32x32(ts + 32u, *reinterpret_cast<uint32_t(*)[32]>(&u[32]));
       tmem_st_wait();
       tc_fence_before();
-      mbar_arrive(&p_ready[x]);
+      mbar_arrive(p_ready);
       l += rs;
     }
     if (!ok) *s_abort = 1;
-    if (ok && n_x > 0 && mbar_wait(&o_done[x], uint32_t(n_x - 1) & 1u, p.status, ST_TIMEOUT_ACC_FULL)) {
+    if (ok && mbar_wait(o_done, uint32_t(n_tiles - 1) & 1u, p.status, ST_TIMEOUT_ACC_FULL)) {
       tc_fence_after();
       const float inv = l > 0.f ? 1.f / l : 0.f;
       bf16* dst = p.out + (((long long)b * p.Sq + qrow) * p.H + h) * p.D;
@@ -352,7 +338,7 @@ dense_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, TMEM_COLS);
+    tmem_dealloc(tmem_base, 256);
   }
 }
 
@@ -399,11 +385,11 @@ bool dense_attention_tc_supported(int B, int Sq, int Sk, int H, int D, const lon
   return true;
 }
 
-template <int DP, bool PAIR>
+template <int DP>
 static void dt_launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const DenseTcParams& p,
                       dim3 grid, cudaStream_t stream) {
-  constexpr int smem = ((PAIR ? 2 : 1) + 4) * (DP / 64) * DT_SUB_BYTES + 256 + 1024;
-  auto kern = dense_attn_tc_kernel<DP, PAIR>;
+  constexpr int smem = DtSmem<DP>::TOTAL;
+  auto kern = dense_attn_tc_kernel<DP>;
   static std::atomic<uint64_t> configured{0};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -413,20 +399,18 @@ static void dt_launch(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
     if (e != cudaSuccess) throw std::runtime_error(std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
     configured.fetch_or(bit, std::memory_order_relaxed);
   }
-  kern<<<grid, PAIR ? DT_THREADS : DT_THREADS_SINGLE, smem, stream>>>(tq, tk, tv, p);
+  kern<<<grid, DT_THREADS, smem, stream>>>(tq, tk, tv, p);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) throw std::runtime_error(std::string("dense attention (tcgen05) launch: ") + cudaGetErrorString(e));
 }
 
 void launch_dense_attention_tc(const void* q, const void* k, const void* v, void* out, const uint8_t* key_mask,
-                               int mask_ld, int B, int Sq, int Sk, int H, int D, const long long* q_strides,
+                               int B, int Sq, int Sk, int H, int D, const long long* q_strides,
                                const long long* k_strides, const long long* v_strides, float scale,
                                uint32_t* status, cudaStream_t stream) {
   if (B == 0 || Sq == 0) return;
   if (!dense_attention_tc_supported(B, Sq, Sk, H, D, q_strides, k_strides, v_strides))
     throw std::runtime_error("dense attention (tcgen05): unsupported shape or strides");
-  if (key_mask != nullptr && (mask_ld % 128 != 0 || mask_ld < Sk || (reinterpret_cast<uintptr_t>(key_mask) & 15) != 0))
-    throw std::runtime_error("dense attention (tcgen05): the key mask must be padded to rows of a multiple of 128");
   // a dimension of extent 1 may carry any stride in the view; give TMA the one of a packed tensor
   auto fix = [&](const long long* s, int rows, long long* o) {
     o[1] = s[1];
@@ -440,7 +424,6 @@ void launch_dense_attention_tc(const void* q, const void* k, const void* v, void
   DenseTcParams p{};
   p.out = reinterpret_cast<bf16*>(out);
   p.key_mask = key_mask;
-  p.mask_ld = mask_ld;
   p.Sq = Sq;
   p.Sk = Sk;
   p.H = H;
@@ -450,12 +433,9 @@ void launch_dense_attention_tc(const void* q, const void* k, const void* v, void
   const CUtensorMap tq = dt_tmap(q, B, Sq, H, D, qs);
   const CUtensorMap tk = dt_tmap(k, B, Sk, H, D, ks);
   const CUtensorMap tv = dt_tmap(v, B, Sk, H, D, vs);
-  if (D <= 64) {
-    // 81 KB of shared memory and 256 columns per CTA: two CTAs per SM
-    dt_launch<64, false>(tq, tk, tv, p, dim3((Sq + DT_BM - 1) / DT_BM, H, B), stream);
-  } else {
-    dt_launch<128, true>(tq, tk, tv, p, dim3((Sq + 2 * DT_BM - 1) / (2 * DT_BM), H, B), stream);
-  }
+  const dim3 grid((Sq + DT_BM - 1) / DT_BM, H, B);
+  if (D <= 64) dt_launch<64>(tq, tk, tv, p, grid, stream);
+  else dt_launch<128>(tq, tk, tv, p, grid, stream);
 }
 
 }  // namespace fc
