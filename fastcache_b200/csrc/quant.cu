@@ -12,9 +12,10 @@
 //
 // What bounds it: at 2 + 1 bytes a value the copy rate allows ~16 instructions per value, and a division, a
 // rounding, two clamps and a conversion each are ~45: with those the kernel ran at a third of the copy rate.  The
-// codes are therefore taken from x * r, r ~ 1 / a, one multiplication, and the division is done only in a lane where
-// that quotient lies so close to the border between two codes that its error could matter (`encode8_fast`; a few
-// lanes in a thousand).  INT8, 1179648 rows of 128 values (458 MB): 199 us before, 133 us now.
+// codes are therefore taken from x * r, r ~ 1 / a, one multiply-add that rounds, and the division is done only for the
+// values whose quotient lies so close to the border between two codes that its error could matter.  INT8, 1179648 rows
+// of 128 values (458 MB): 199 us with the divisions, 133 us dividing all eight values of a lane that has an unsure one
+// (a fraction of a percent of the values, but half of the warps), 111 us so.
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
 #include <cuda_runtime.h>
@@ -97,8 +98,8 @@ __device__ __forceinline__ float decode(int q, float a, float z) {
 
 // Codes of eight values from the quotient t = x * r, r ~ 1 / a, in place of the division.  r is off by one unit in the
 // last place (2^-23) at most, t and the division that the codes are defined by by half of one, so t and fl(x / a) differ
-// by less than 2^-22 |t|: 6.1e-5 for the largest quotient, 255.  Returns false when some t is closer than 1e-4 (INT8,
-// INT4), 1e-6 (NF4, |t| <= 1) or 2^-20 |t| (FP8) to the border between two codes, or is no number: the caller then
+// by less than 2^-22 |t|: 6.1e-5 for the largest quotient, 255.  Returns a bit for each value whose t is closer than 1e-4
+// (INT8, INT4), 1e-6 (NF4, |t| <= 1) or 2^-20 |t| (FP8) to the border between two codes, or is no number: the caller then
 // divides, as it does where 1 / a would be subnormal.
 // `s_mid` (NF4 only): the 15 midpoints, with -inf before and +inf behind them.
 constexpr float QROUND = 12582912.f;      // 1.5 * 2^23: adding it rounds to an integer, half to even, in the low bits
@@ -107,34 +108,49 @@ constexpr float QNEAR = 0.5f - 1e-4f;
 __device__ __forceinline__ int nf4_code_fast(float t, const float* s_mid);
 
 template <int MODE>
-__device__ __forceinline__ bool encode8_fast(const float (&x)[8], float r, float z, const float* s_mid, int (&code)[8]) {
-  bool sure = true;
+__device__ __forceinline__ uint32_t encode8_fast(const uint4& raw, float r, float z, const float* s_mid, uint2& w) {
+  float x[8];
+  unpack8(raw, x);
+  uint32_t unsure = 0;
+  if (MODE == QUANT_INT8 || MODE == QUANT_INT8_ASYM || MODE == QUANT_INT4) {
+    // x r + QROUND rounds to an integer whose low byte is the code (two's complement; INT4 counts from 8); what the
+    // rounding took off is one more multiply-add
+    constexpr float OFFSET = MODE == QUANT_INT4 ? QROUND + 8.f : QROUND;
+    const float q = MODE == QUANT_INT4 ? r * 7.0f : r;
+    uint32_t m[8];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    if (MODE == QUANT_INT8 || MODE == QUANT_INT8_ASYM || MODE == QUANT_INT4) {
-      const float t = MODE == QUANT_INT8_ASYM ? (x[i] - z) * r : MODE == QUANT_INT4 ? x[i] * r * 7.0f : x[i] * r;
-      const float m = __fadd_rn(t, QROUND);
-      sure = sure && fabsf(__fsub_rn(t, __fsub_rn(m, QROUND))) < QNEAR;
-      code[i] = int(__float_as_uint(m) & 0xFFu);             // two's complement
-      if (MODE == QUANT_INT4) code[i] = (code[i] + 8) & 0xF;
-    } else if (MODE == QUANT_NF4) {
+    for (int i = 0; i < 8; ++i) {
+      const float y = MODE == QUANT_INT8_ASYM ? x[i] - z : x[i];
+      const float n = __fmaf_rn(y, q, OFFSET);
+      if (!(fabsf(__fmaf_rn(y, q, __fsub_rn(OFFSET, n))) < QNEAR)) unsure |= 1u << i;
+      m[i] = __float_as_uint(n);
+    }
+    w.x = __byte_perm(__byte_perm(m[0], m[1], 0x0040), __byte_perm(m[2], m[3], 0x0040), 0x5410);
+    w.y = __byte_perm(__byte_perm(m[4], m[5], 0x0040), __byte_perm(m[6], m[7], 0x0040), 0x5410);
+  } else if (MODE == QUANT_NF4) {
+    w = make_uint2(0, 0);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
       const float t = x[i] * r;
       const int c = nf4_code_fast(t, s_mid);
-      sure = sure && t - s_mid[c - 1] > 1e-6f && s_mid[c] - t > 1e-6f;
-      code[i] = c;
-    } else if ((i & 1) == 0) {
-      // both ends of the interval that holds the quotient have the same code
-      const __nv_fp8_interpretation_t kind = (MODE == QUANT_FP8_E4M3) ? __NV_E4M3 : __NV_E5M2;
-      const float t0 = x[i] * r, t1 = x[i + 1] * r;
-      constexpr float UP = 1.f + 0x1p-20f, DOWN = 1.f - 0x1p-20f;
-      const uint32_t u = __nv_cvt_float2_to_fp8x2(make_float2(t0 * UP, t1 * UP), __NV_SATFINITE, kind);
-      const uint32_t d = __nv_cvt_float2_to_fp8x2(make_float2(t0 * DOWN, t1 * DOWN), __NV_SATFINITE, kind);
-      sure = sure && u == d;
-      code[i] = int(u & 0xFFu);
-      code[i + 1] = int(u >> 8);
+      if (!(t - s_mid[c - 1] > 1e-6f && s_mid[c] - t > 1e-6f)) unsure |= 1u << i;
+      (i < 4 ? w.x : w.y) |= uint32_t(c) << (8 * (i & 3));
     }
+  } else {
+    // both ends of the interval that holds the quotient have the same code
+    const __nv_fp8_interpretation_t kind = (MODE == QUANT_FP8_E4M3) ? __NV_E4M3 : __NV_E5M2;
+    constexpr float UP = 1.f + 0x1p-20f, DOWN = 1.f - 0x1p-20f;
+    const float up = r * UP, down = r * DOWN;
+    uint32_t u[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      u[i] = __nv_cvt_float2_to_fp8x2(make_float2(x[2 * i] * up, x[2 * i + 1] * up), __NV_SATFINITE, kind);
+      if (u[i] != __nv_cvt_float2_to_fp8x2(make_float2(x[2 * i] * down, x[2 * i + 1] * down), __NV_SATFINITE, kind)) unsure |= 3u << (2 * i);
+    }
+    w.x = __byte_perm(u[0], u[1], 0x5410);
+    w.y = __byte_perm(u[2], u[3], 0x5410);
   }
-  return sure;
+  return unsure;
 }
 
 // group statistics of the values a warp holds -> (a, z) as `encode` wants them
@@ -149,12 +165,29 @@ __device__ __forceinline__ void group_params(float amax, float lo, float hi, flo
   else a = __fdiv_rn(fmaxf(amax, 1e-8f), MODE == QUANT_FP8_E4M3 ? 448.0f : 57344.0f);
 }
 
-// Lanes per group: a group of g values is g / 8 pieces of 16 bytes; W = the next power of two (at most 32) lanes
-// share one group, 32 / W groups sit side by side in a warp and QU such batches are in flight per iteration, so
-// every lane has QU independent 16-byte loads outstanding (a 128-value group uses 16 lanes: without this half of
-// every warp would idle and each lane would wait for one load at a time).  Groups longer than 256 values give a
-// lane several pieces (W = 32, up to QMAX_CHUNKS).
-constexpr int QU = 4;
+// the codes of the values in `which` (bits 0 ... 7) by division.  With bf16 inputs borders are met exactly and not only by
+// chance (a value of half the largest one lies between 63 and 64 in INT8, between 3 and 4 in INT4), a fraction of a
+// percent of all values: half of all warps come here with some lane, mostly for one value
+template <int MODE>
+__device__ __forceinline__ void encode_exact(uint32_t which, const uint4& raw, float a, float z, const float* s_mid, uint2& w) {
+  while (which != 0u) {
+    const int i = __ffs(which) - 1;
+    which &= which - 1;
+    const uint32_t pair = i < 4 ? (i < 2 ? raw.x : raw.y) : (i < 6 ? raw.z : raw.w);
+    const float x = __uint_as_float((i & 1) ? pair & 0xffff0000u : pair << 16);
+    const int e = (MODE == QUANT_NF4) ? nf4_code_fast(__fdiv_rn(x, a), s_mid) : encode<MODE>(x, a, z);
+    const int at = 8 * (i & 3);
+    const uint32_t old = i < 4 ? w.x : w.y, now = (old & ~(0xFFu << at)) | (uint32_t(e & 0xFF) << at);
+    if (i < 4) w.x = now;
+    else w.y = now;
+  }
+}
+
+// Lanes per group: a group of g values is g / 8 pieces of 16 bytes.  W lanes share one group, CH pieces each; 32 / W
+// groups sit side by side in a warp and QU such batches are in flight per iteration.  Two pieces per lane halve what a
+// group costs besides its values (the shuffles of the reduction, the scale and its reciprocal); only groups of up to 32
+// values have one.
+constexpr int quant_batches(int ch) { return ch > 2 ? 2 : 4; }
 
 template <int W>
 __device__ __forceinline__ float sub_max(float v) {
@@ -190,7 +223,7 @@ __device__ __forceinline__ int nf4_code_fast(float t, const float* s_mid) {
 // x [groups, g] bf16 (rows of D values cut into D / g groups).  FAKE: y = decode(encode(x)) in bf16, no codes.
 // Otherwise: codes as bytes (INT8, FP8: one per value; INT4 / NF4: one per two values), `scale` [groups] (the
 // scale, or the absmax for the 4-bit modes) and, for the asymmetric mode, `zero` [groups].
-template <int MODE, bool FAKE, int W>
+template <int MODE, bool FAKE, int W, int CH>
 __global__ void __launch_bounds__(256)
 quantize_kernel(const bf16* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ scale,
                 float* __restrict__ zero, bf16* __restrict__ y, long long groups, int g) {
@@ -208,7 +241,7 @@ quantize_kernel(const bf16* __restrict__ x, uint8_t* __restrict__ q, float* __re
   const int lane = threadIdx.x & 31;
   const int sub = lane / W, l = lane % W;
   constexpr int GPW = 32 / W;                                    // groups per warp and batch
-  constexpr int CH = (W == 32) ? QMAX_CHUNKS : 1;                // 16-byte pieces per lane and group
+  constexpr int QU = quant_batches(CH);
   const long long warp = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
   const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
   const int chunks = g >> 3;
@@ -263,29 +296,22 @@ quantize_kernel(const bf16* __restrict__ x, uint8_t* __restrict__ q, float* __re
 #pragma unroll
       for (int c = 0; c < CH; ++c) {
         if (l + W * c >= chunks) continue;
-        float v[8];
-        unpack8(raw[u][c], v);
-        int code[8];
-        if (!(a < 0x1p125f) || !encode8_fast<MODE>(v, r, z, s_mid, code)) {
-#pragma unroll
-          for (int i = 0; i < 8; ++i)
-            code[i] = (MODE == QUANT_NF4) ? nf4_code_fast(__fdiv_rn(v[i], a), s_mid) : encode<MODE>(v[i], a, z);
-        }
+        uint2 w;                                                 // eight codes, one byte each
+        const uint32_t unsure = encode8_fast<MODE>(raw[u][c], r, z, s_mid, w);
+        encode_exact<MODE>(a < 0x1p125f ? unsure : 0xFFu, raw[u][c], a, z, s_mid, w);
         if (FAKE) {
           float out[8];
 #pragma unroll
-          for (int i = 0; i < 8; ++i)
-            out[i] = FOUR_BIT ? s_tab[code[i]] * a : decode<MODE>((MODE == QUANT_INT8) ? int(int8_t(code[i])) : code[i], a, z);
+          for (int i = 0; i < 8; ++i) {
+            const int code = int(((i < 4 ? w.x : w.y) >> (8 * (i & 3))) & 0xFFu);
+            out[i] = FOUR_BIT ? s_tab[code] * a : decode<MODE>((MODE == QUANT_INT8) ? int(int8_t(code)) : code, a, z);
+          }
           store8(y + e + W * c * 8, out);
         } else if (FOUR_BIT) {
-          uint32_t w = 0;
-#pragma unroll
-          for (int i = 0; i < 4; ++i) w |= uint32_t((code[2 * i] & 0xF) | ((code[2 * i + 1] & 0xF) << 4)) << (8 * i);
-          *reinterpret_cast<uint32_t*>(q + ((e + W * c * 8) >> 1)) = w;
+          // bytes 0, 2, ... hold the low nibbles, 1, 3, ... the high ones
+          const uint32_t lo = (w.x | (w.x >> 4)) & 0x00FF00FFu, hi = (w.y | (w.y >> 4)) & 0x00FF00FFu;
+          *reinterpret_cast<uint32_t*>(q + ((e + W * c * 8) >> 1)) = __byte_perm(lo, hi, 0x6420);
         } else {
-          uint2 w;
-          w.x = __byte_perm(__byte_perm(code[0], code[1], 0x0040), __byte_perm(code[2], code[3], 0x0040), 0x5410);
-          w.y = __byte_perm(__byte_perm(code[4], code[5], 0x0040), __byte_perm(code[6], code[7], 0x0040), 0x5410);
           *reinterpret_cast<uint2*>(q + e + W * c * 8) = w;
         }
       }
@@ -337,21 +363,22 @@ static int quant_grid(long long work_items, int per_block) {
   return int(blocks < 1 ? 1 : (blocks > 148 * 16 ? 148 * 16 : blocks));
 }
 
-template <int MODE, int W>
+template <int MODE, int W, int CH>
 static void launch_quantize_w(const bf16* x, uint8_t* q, float* scale, float* zero, bf16* y, long long groups, int g,
                               cudaStream_t s) {
-  const int grid = quant_grid(groups, 8 * (32 / W) * QU);          // groups per block and iteration
-  if (y != nullptr) quantize_kernel<MODE, true, W><<<grid, 256, 0, s>>>(x, q, scale, zero, y, groups, g);
-  else quantize_kernel<MODE, false, W><<<grid, 256, 0, s>>>(x, q, scale, zero, y, groups, g);
+  const int grid = quant_grid(groups, 8 * (32 / W) * quant_batches(CH));          // groups per block and iteration
+  if (y != nullptr) quantize_kernel<MODE, true, W, CH><<<grid, 256, 0, s>>>(x, q, scale, zero, y, groups, g);
+  else quantize_kernel<MODE, false, W, CH><<<grid, 256, 0, s>>>(x, q, scale, zero, y, groups, g);
 }
 template <int MODE>
 static void launch_quantize_m(const bf16* x, uint8_t* q, float* scale, float* zero, bf16* y, long long groups, int g,
                               cudaStream_t s) {
   const int chunks = g >> 3;
-  if (chunks <= 4) launch_quantize_w<MODE, 4>(x, q, scale, zero, y, groups, g, s);
-  else if (chunks <= 8) launch_quantize_w<MODE, 8>(x, q, scale, zero, y, groups, g, s);
-  else if (chunks <= 16) launch_quantize_w<MODE, 16>(x, q, scale, zero, y, groups, g, s);
-  else launch_quantize_w<MODE, 32>(x, q, scale, zero, y, groups, g, s);
+  if (chunks <= 4) launch_quantize_w<MODE, 4, 1>(x, q, scale, zero, y, groups, g, s);
+  else if (chunks <= 8) launch_quantize_w<MODE, 4, 2>(x, q, scale, zero, y, groups, g, s);
+  else if (chunks <= 16) launch_quantize_w<MODE, 8, 2>(x, q, scale, zero, y, groups, g, s);
+  else if (chunks <= 32) launch_quantize_w<MODE, 16, 2>(x, q, scale, zero, y, groups, g, s);
+  else launch_quantize_w<MODE, 32, QMAX_CHUNKS>(x, q, scale, zero, y, groups, g, s);
 }
 
 void launch_quantize(const void* x, void* q, float* scale, float* zero, void* y_fake, long long groups, int g,
