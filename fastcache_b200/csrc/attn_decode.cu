@@ -1,7 +1,7 @@
 // Paged decode attention: one query row per request over its (possibly compressed) K/V in the pool.
 //
 // Grid (request, kv head, kv split).  A CTA streams 64-row K and V tiles of its
-// kv head through a 3-stage ring filled by TMA (cp.async.bulk.tensor 2-D boxes with
+// kv head through a ring of two or three stages filled by TMA (cp.async.bulk.tensor 2-D boxes with
 // the 128-byte swizzle, completion on an mbarrier): the pool is head-major inside a
 // block, so the rows of one head are a dense [rows, D] matrix and one elected thread
 // moves a whole tile with a handful of instructions.  Boxes never straddle a pool
@@ -41,8 +41,21 @@ namespace fc {
 using bf16 = __nv_bfloat16;
 
 constexpr int DEC_TILE = 64;      // kv rows per stage
-constexpr int DEC_STAGES = 3;
 constexpr int DEC_THREADS = 128;
+
+// K + V stages of a CTA: two, so that three CTAs share an SM, or three, so that two do.  Both keep 192 KB in flight; more
+// CTAs hide each other's start, query loads and final merge.  13 requests x 32 heads around 680 rows: 38.3 us with two
+// CTAs of three stages, 30.5 us with three of two; 128 x 8 around 1920 rows: 181.8 us and 174.2 us (158 us at the copy
+// rate).  Three stages stay where they save a wave: 64 x 8 around 1920 rows are two waves of 296 CTAs (106 us) and two of
+// 444 as well (115 us).
+constexpr int dec_ctas_per_sm(int stages) { return stages == 2 ? 3 : 2; }
+int dec_stages(long long ctas, int num_sms) {
+  auto cost = [&](int stages) {
+    const long long slots = (long long)dec_ctas_per_sm(stages) * num_sms;
+    return (ctas + slots - 1) / slots * dec_ctas_per_sm(stages);               // waves x the time of one
+  };
+  return cost(3) * 6 < cost(2) * 5 ? 3 : 2;
+}
 
 // byte offset of 16-byte chunk `chunk` of row `row` inside a TMA-swizzled tile:
 // sub-tiles of [64 rows x 128 bytes], chunk index XOR (row mod 8) inside the 128-byte row
@@ -104,7 +117,7 @@ __device__ __forceinline__ void decode_merge_last(const float* __restrict__ part
   if (threadIdx.x == 0) counters[b * Hkv + hk] = 0;
 }
 
-template <int D>
+template <int D, int DEC_STAGES>
 __global__ void __launch_bounds__(DEC_THREADS)
 decode_attn_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                    const bf16* __restrict__ q, int box_rows, const int* __restrict__ block_tables, const int* __restrict__ context_lens,
@@ -403,12 +416,14 @@ __global__ void decode_merge_kernel(const float* __restrict__ part_o, const floa
   }
 }
 
+// As many splits as fill the SMs once (rounded down: a few CTAs in a second wave cost as much as a full one) and at least
+// four tiles each.  24 requests x 8 heads around 1150 rows: 38.6 us with splits that overflow, 32.0 us so; 32 x 8 around
+// 100 rows, where the merge is what it costs: 18.0 us and 9.6 us.
 int decode_attn_pick_splits(int B, int Hkv, int max_ctx, int num_sms) {
   const int ctas = B * Hkv;
-  const int target = 2 * num_sms;
-  if (ctas >= target) return 1;
+  const int target = dec_ctas_per_sm(2) * num_sms;
   const int max_by_len = std::max(1, max_ctx / (4 * DEC_TILE));
-  return std::max(1, std::min({(target + ctas - 1) / ctas, max_by_len, DECODE_MAX_SPLITS}));
+  return std::max(1, std::min({target / std::max(1, ctas), max_by_len, DECODE_MAX_SPLITS}));
 }
 
 void launch_decode_attention(const void* q, const void* k_cache, const void* v_cache, const int* block_tables,
@@ -429,7 +444,8 @@ void launch_decode_attention(const void* q, const void* k_cache, const void* v_c
   if (box_rows < 8) throw std::runtime_error("decode attention: block_size must be a multiple of 8");
   const float scale_log2 = scale * 1.4426950408889634f;
   dim3 grid(B, Hkv, splits);
-  const int smem = DEC_STAGES * 2 * DEC_TILE * D * 2 + 64 + 1024;
+  const int stages = dec_stages((long long)B * Hkv * splits, gemm_num_sms());
+  const int smem = stages * 2 * DEC_TILE * D * 2 + 64 + 1024;
   const uint64_t rows = (uint64_t)num_blocks * Hkv * block_size;
   const CUtensorMap tk = make_tmap_bf16_2d(k_cache, rows, D, D, box_rows, 64);
   const CUtensorMap tv = make_tmap_bf16_2d(v_cache, rows, D, D, box_rows, 64);
@@ -440,8 +456,8 @@ void launch_decode_attention(const void* q, const void* k_cache, const void* v_c
                context_lens, (bf16*)out, part_o, part_lse, Hq, Hkv, block_size, max_blocks, num_blocks, splits,
                scale_log2, status, merge_counters, opt);
   };
-  if (D == 128) launch(decode_attn_kernel<128>);
-  else if (D == 64) launch(decode_attn_kernel<64>);
+  if (D == 128) launch(stages == 2 ? decode_attn_kernel<128, 2> : decode_attn_kernel<128, 3>);
+  else if (D == 64) launch(stages == 2 ? decode_attn_kernel<64, 2> : decode_attn_kernel<64, 3>);
   else throw std::runtime_error("decode attention: head_dim must be 64 or 128");
   // `merge_counters` (zero between launches, B * Hkv words): the last split of a (request, KV head) merges in the
   // attention kernel itself; without them a second kernel does
