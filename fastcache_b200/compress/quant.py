@@ -4,7 +4,7 @@ byte), FP8 casts and NF4 (nearest entry of the 16-value NormalFloat table).
 Parity: nanovllm/autocompress/methods.py:636-757, nanovllm/autocompress/kernels.py:388-422,
 utils_ccm/utils_compress.py:51-70, :144-154 (SimpleKVQuantizer / ImprovedKVQuantizer fake-quant).
 
-bf16 tensors on a CUDA device go through the kernels of csrc/quant.cu (one warp per group, one pass, codes and
+bf16 tensors on a CUDA device go through the kernels of csrc/quant.cu (up to 32 lanes per group, one pass, codes and
 scales bit-identical to the statements below); everything else runs the PyTorch statements.
 """
 from __future__ import annotations

@@ -322,6 +322,23 @@ Tensor layer_norm(const Tensor& x, const Tensor& w, const Tensor& b, double eps)
   return y;
 }
 
+// x [B, N, C] + table [side * side, C] at the buckets of `grids` [B, 2 + 2 n] int32 (h, w, row buckets, column buckets)
+Tensor add_grid_positions(const Tensor& x, const Tensor& table, const Tensor& grids, int64_t side) {
+  check_bf16(x, "x");
+  check_bf16(table, "table");
+  TORCH_CHECK(x.dim() == 3 && x.is_contiguous() && x.size(2) % 8 == 0 && table.is_contiguous() && table.dim() == 2 &&
+                  table.size(0) == side * side && table.size(1) == x.size(2), "bad features or table");
+  TORCH_CHECK(reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0 && reinterpret_cast<uintptr_t>(table.data_ptr()) % 16 == 0,
+              "features and table must be 16-byte aligned");
+  TORCH_CHECK(grids.is_cuda() && grids.scalar_type() == torch::kInt32 && grids.is_contiguous() && grids.dim() == 2 &&
+                  grids.size(0) == x.size(0) && grids.size(1) >= 4 && grids.size(1) % 2 == 0, "grids must be int32 [B, 2 + 2 n] on the device");
+  c10::cuda::CUDAGuard guard(x.device());
+  Tensor y = torch::empty_like(x);
+  fc::launch_add_grid_positions(x.data_ptr(), table.data_ptr(), grids.data_ptr<int>(), y.data_ptr(), int(x.size(0)), int(x.size(1)),
+                                int(x.size(2)), int(grids.size(1) / 2 - 1), int(side), at::cuda::getCurrentCUDAStream());
+  return y;
+}
+
 Tensor silu_and_mul(const Tensor& x) {
   check_bf16(x, "x");
   TORCH_CHECK(x.is_contiguous() && x.size(-1) % 16 == 0, "expects contiguous input with last dim % 16 == 0");
@@ -520,6 +537,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("rms_norm", &rms_norm);
   m.def("add_rms_norm", &add_rms_norm);
   m.def("layer_norm", &layer_norm);
+  m.def("add_grid_positions", &add_grid_positions);
   m.def("silu_and_mul", &silu_and_mul);
   m.def("embedding", &embedding);
   m.def("rope_qknorm_store", &rope_qknorm_store);

@@ -251,6 +251,32 @@ __global__ void embedding_kernel(const long long* __restrict__ ids, const bf16* 
   for (int c = threadIdx.x; c < chunks; c += blockDim.x) o[c] = src[c];
 }
 
+// y[b, i] = x[b, i] + table[row * side + column] for patch i of a grid of h x w patches, + table[0] past its h w patches.
+// grids [B, 2 + 2 n]: h, w, the bucket of each of the h rows (n places), that of each of the w columns (n places).
+// One warp per patch; bound by reading and writing x once.
+__global__ void __launch_bounds__(256)
+add_grid_positions_kernel(const bf16* __restrict__ x, const bf16* __restrict__ table, const int* __restrict__ grids,
+                          bf16* __restrict__ y, long long rows, int N, int C, int n, int side) {
+  const long long r = blockIdx.x * 8ll + (threadIdx.x >> 5);
+  if (r >= rows) return;
+  const int b = int(r / N), i = int(r - (long long)b * N);
+  const int* g = grids + (long long)b * (2 + 2 * n);
+  const int h = min(max(g[0], 0), n), w = min(max(g[1], 0), n);
+  int id = 0;
+  if (w > 0 && i < h * w) id = min(max(g[2 + i / w] * side + g[2 + n + i % w], 0), side * side - 1);
+  const uint4* xr = reinterpret_cast<const uint4*>(x + r * C);
+  const uint4* tr = reinterpret_cast<const uint4*>(table + (long long)id * C);
+  uint4* yr = reinterpret_cast<uint4*>(y + r * C);
+  for (int c = threadIdx.x & 31; c < (C >> 3); c += 32) {
+    float a[8], t[8];
+    unpack8(xr[c], a);
+    unpack8(tr[c], t);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) a[e] += t[e];
+    yr[c] = pack8(a);
+  }
+}
+
 // One warp per (token, head).  Heads [0, Hq) are queries (normed, rotated, written to q_out),
 // [Hq, Hq+Hkv) keys (normed, rotated, stored in the pool), the rest values (stored).
 __global__ void __launch_bounds__(128)
@@ -365,6 +391,16 @@ rope_qknorm_store_d128_kernel(const bf16* __restrict__ qkv, const long long* __r
   const long long g = active ? gid : 0;
   const int t = int(g / heads);
   const int h = int(g - (long long)t * heads);
+  // position -> angles is two round trips: both are under way while the partial sums arrive, and so are slot and weights
+  const long long slot_in = h >= Hq && slots != nullptr ? (long long)slots[t] : -1;
+  const float4* cs = reinterpret_cast<const float4*>(cos_sin + positions[t] * 128);
+  const float4 c0 = cs[2 * j], c1 = cs[2 * j + 1], s0 = cs[16 + 2 * j], s1 = cs[16 + 2 * j + 1];
+  const bf16* nw = h < Hq ? q_w : k_w;
+  uint4 gain_lo = make_uint4(0, 0, 0, 0), gain_hi = gain_lo;
+  if (nw != nullptr) {
+    gain_lo = reinterpret_cast<const uint4*>(nw)[j];
+    gain_hi = reinterpret_cast<const uint4*>(nw)[8 + j];
+  }
   uint4 ulo, uhi;
   if (partial != nullptr) {
     // qkv is still the split-K partial sums of its GEMM ([splits, T, heads * 128] fp32): reduce them here and
@@ -389,13 +425,10 @@ rope_qknorm_store_d128_kernel(const bf16* __restrict__ qkv, const long long* __r
     ulo = src[j];
     uhi = src[8 + j];
   }
-  long long slot = -1;
-  if (h >= Hq && slots != nullptr) {
-    slot = slots[t];
-    if (slot >= num_slots) {
-      report(status, ST_BAD_INDEX);
-      slot = -1;
-    }
+  long long slot = slot_in;
+  if (slot >= num_slots) {
+    report(status, ST_BAD_INDEX);
+    slot = -1;
   }
   float lo[8], hi[8];
   unpack8(ulo, lo);
@@ -418,12 +451,11 @@ rope_qknorm_store_d128_kernel(const bf16* __restrict__ qkv, const long long* __r
   }
   const bool is_q = h < Hq;
   if (!is_q && slot < 0) return;
-  const bf16* nw = is_q ? q_w : k_w;
   if (nw != nullptr) {
     const float inv = rsqrtf(ss / 128.f + eps);
     float wl[8], wh[8];
-    unpack8(reinterpret_cast<const uint4*>(nw)[j], wl);
-    unpack8(reinterpret_cast<const uint4*>(nw)[8 + j], wh);
+    unpack8(gain_lo, wl);
+    unpack8(gain_hi, wh);
     auto rn = [](float v) { return __bfloat162float(__float2bfloat16(v)); };
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -431,8 +463,6 @@ rope_qknorm_store_d128_kernel(const bf16* __restrict__ qkv, const long long* __r
       hi[i] = rn(rn(hi[i] * inv) * wh[i]);
     }
   }
-  const float4* cs = reinterpret_cast<const float4*>(cos_sin + positions[t] * 128);
-  const float4 c0 = cs[2 * j], c1 = cs[2 * j + 1], s0 = cs[16 + 2 * j], s1 = cs[16 + 2 * j + 1];
   const float c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
   const float s[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
   uint4 olo, ohi;
@@ -623,6 +653,13 @@ void launch_layer_norm(const void* x, const void* w, const void* b, void* y, lon
               : layer_norm_kernel<16>;
   constexpr int rows = NORM_THREADS / 32;
   kern<<<(unsigned)((T + rows - 1) / rows), NORM_THREADS, 0, s>>>((const bf16*)x, (const bf16*)w, (const bf16*)b, (bf16*)y, T, H, eps);
+}
+
+void launch_add_grid_positions(const void* x, const void* table, const int* grids, void* y, int B, int N, int C, int n, int side,
+                               cudaStream_t s) {
+  const long long rows = (long long)B * N;
+  if (rows == 0) return;
+  add_grid_positions_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, s>>>((const bf16*)x, (const bf16*)table, grids, (bf16*)y, rows, N, C, n, side);
 }
 
 void launch_silu_and_mul(const void* x, void* y, long long T, int I, cudaStream_t s) {

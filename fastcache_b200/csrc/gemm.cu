@@ -23,9 +23,9 @@
 // scheduler has nothing to hide its tcgen05.ld and MUFU latencies with.  Hence STAGED: 15 images through the CLIP tower,
 // 95 products of 8655 rows: 5.69 ms with the stores from registers, 4.49 ms so; SigLIP, 5 slices of 961 rows: 5.73 ms
 // against 4.72 ms.  At K = 4096 and more the main loop hides the plain epilogue, and the second group only costs: 26120
-// rows through four 8B layers took 39.8 ms with it off and 40.8 ms with it on, so the line is at K = 2048.  With no more
-// than two tiles per CTA nothing hides the last epilogue whatever K is, and STAGED is the faster one again (SigLIP's
-// 4805 x 1152 x 4304).
+// rows through four 8B layers took 39.8 ms with it off and 40.8 ms with it on, so the line is at K = 2048.  Three prompts
+// of 250 to 450 tokens through the same layers, at the power limit when they follow one another: 1.83 ms with the staged
+// epilogue and CTA pairs wherever they save time alone, 1.78 ms with neither beyond that line.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -39,6 +39,7 @@
 #include <unordered_map>
 
 #include "gemm.h"
+#include "gemm_epilogue.cuh"
 #include "hybrid.cuh"
 #include "ptx.cuh"
 
@@ -47,8 +48,6 @@ namespace fc {
 constexpr int BM = 128;
 constexpr int BK = 64;
 constexpr int STAGED_K = 2048;                    // see above
-constexpr int SLAB = 64;                          // output columns an epilogue group stores at a time
-constexpr int SLAB_BYTES = BM * SLAB * 2;
 
 struct GemmParams {
   int M, N, K;
@@ -70,49 +69,6 @@ struct GemmParams {
   float limit;            // GLU_CLAMPED
   const float* coef;      // GF_XIELU: its two factors
 };
-
-__device__ __forceinline__ float apply_act(float v, int act) {
-  switch (act) {
-    case ACT_RELU: return fmaxf(v, 0.f);
-    case ACT_GELU: return 0.5f * v * (1.f + erff(v * 0.70710678118654752f));
-    case ACT_GELU_TANH: {
-      float u = 0.7978845608028654f * (v + 0.044715f * v * v * v), th;
-      asm("tanh.approx.f32 %0, %1;" : "=f"(th) : "f"(u));
-      return 0.5f * v * (1.f + th);
-    }
-    case ACT_QUICK_GELU: return __fdividef(v, 1.f + __expf(-1.702f * v));
-    case ACT_SILU: return __fdividef(v, 1.f + __expf(-v));
-    default: return v;
-  }
-}
-
-// The activation of 32 values with the (uniform) selector tested once, not per element.
-__device__ __forceinline__ void apply_act_chunk(float (&v)[32], int act) {
-  switch (act) {
-    case ACT_NONE: break;
-    case ACT_RELU:
-#pragma unroll
-      for (int t = 0; t < 32; ++t) v[t] = apply_act(v[t], ACT_RELU);
-      break;
-    case ACT_GELU:
-#pragma unroll
-      for (int t = 0; t < 32; ++t) v[t] = apply_act(v[t], ACT_GELU);
-      break;
-    case ACT_GELU_TANH:
-#pragma unroll
-      for (int t = 0; t < 32; ++t) v[t] = apply_act(v[t], ACT_GELU_TANH);
-      break;
-    case ACT_QUICK_GELU:
-#pragma unroll
-      for (int t = 0; t < 32; ++t) v[t] = apply_act(v[t], ACT_QUICK_GELU);
-      break;
-    case ACT_SILU:
-#pragma unroll
-      for (int t = 0; t < 32; ++t) v[t] = apply_act(v[t], ACT_SILU);
-      break;
-    default: break;
-  }
-}
 
 constexpr int gemm_threads(bool staged) { return staged ? 320 : 192; }
 
@@ -308,24 +264,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
 
     // bias and activation of 32 values, columns col ... col + 31
     auto finish = [&](float (&v)[32], int col, bool whole) {
-      if (p.bias != nullptr) {
-        if (whole && (reinterpret_cast<uintptr_t>(p.bias + col) & 15) == 0) {
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const uint4 bv = *reinterpret_cast<const uint4*>(p.bias + col + q * 8);
-            const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {      // a bf16 is the upper half of the fp32 with the same value
-              v[q * 8 + e * 2] += __uint_as_float(bw[e] << 16);
-              v[q * 8 + e * 2 + 1] += __uint_as_float(bw[e] & 0xffff0000u);
-            }
-          }
-        } else {
-#pragma unroll
-          for (int t = 0; t < 32; ++t)
-            if (col + t < p.N) v[t] += __bfloat162float(p.bias[col + t]);
-        }
-      }
+      if (p.bias != nullptr) add_bias_chunk(v, p.bias, col, p.N, whole);
       if constexpr (FORM == GF_XIELU) {
         const float a = __ldg(p.coef), b = __ldg(p.coef + 1);
 #pragma unroll
@@ -334,43 +273,33 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         apply_act_chunk(v, p.act);
       }
     };
-    // out = act(gate) * up of 32 columns col ... col + 31 of the output, packed
-    auto gated = [&](const uint32_t (&rg)[32], const uint32_t (&ru)[32], int col, uint32_t (&u)[16]) {
-#pragma unroll
-      for (int t = 0; t < 32; t += 2) {
-        float g0 = __uint_as_float(rg[t]), g1 = __uint_as_float(rg[t + 1]);
-        float u0 = __uint_as_float(ru[t]), u1 = __uint_as_float(ru[t + 1]);
-        float a, b;
-        if constexpr (GLU == GLU_GELU_TANH) {
-          if (p.bias != nullptr) {            // pairs of a bias that starts at a multiple of 16 bytes
-            const uint32_t bg = *reinterpret_cast<const uint32_t*>(p.bias + col + t);
-            const uint32_t bu = *reinterpret_cast<const uint32_t*>(p.bias + p.up_row0 + col + t);
-            g0 += __uint_as_float(bg << 16);
-            g1 += __uint_as_float(bg & 0xffff0000u);
-            u0 += __uint_as_float(bu << 16);
-            u1 += __uint_as_float(bu & 0xffff0000u);
-          }
-          // 0.5 z (1 + tanh y) = z / (1 + exp(-2 y)), y = sqrt(2 / pi) (z + 0.044715 z^3)
-          a = __fdividef(g0, 1.f + __expf(-1.5957691216057308f * (g0 + 0.044715f * g0 * g0 * g0))) * u0;
-          b = __fdividef(g1, 1.f + __expf(-1.5957691216057308f * (g1 + 0.044715f * g1 * g1 * g1))) * u1;
-        } else if constexpr (GLU == GLU_CLAMPED) {
-          g0 = fminf(g0, p.limit);
-          g1 = fminf(g1, p.limit);
-          a = __fdividef(g0, 1.f + __expf(-1.702f * g0)) * (fminf(fmaxf(u0, -p.limit), p.limit) + 1.f);
-          b = __fdividef(g1, 1.f + __expf(-1.702f * g1)) * (fminf(fmaxf(u1, -p.limit), p.limit) + 1.f);
-        } else {
-          a = g0 / (1.f + __expf(-g0)) * u0;
-          b = g1 / (1.f + __expf(-g1)) * u1;
+    // out = act(gate) * up of columns col + t and col + t + 1 of the output, packed
+    auto gated = [&](const uint32_t (&rg)[32], const uint32_t (&ru)[32], int col, int t) -> uint32_t {
+      float g0 = __uint_as_float(rg[t]), g1 = __uint_as_float(rg[t + 1]);
+      float u0 = __uint_as_float(ru[t]), u1 = __uint_as_float(ru[t + 1]);
+      float a, b;
+      if constexpr (GLU == GLU_GELU_TANH) {
+        if (p.bias != nullptr) {            // pairs of a bias that starts at a multiple of 16 bytes
+          const uint32_t bg = *reinterpret_cast<const uint32_t*>(p.bias + col + t);
+          const uint32_t bu = *reinterpret_cast<const uint32_t*>(p.bias + p.up_row0 + col + t);
+          g0 += __uint_as_float(bg << 16);
+          g1 += __uint_as_float(bg & 0xffff0000u);
+          u0 += __uint_as_float(bu << 16);
+          u1 += __uint_as_float(bu & 0xffff0000u);
         }
-        u[t / 2] = pack_bf16(a, b);
+        // 0.5 z (1 + tanh y) = z / (1 + exp(-2 y)), y = sqrt(2 / pi) (z + 0.044715 z^3)
+        a = __fdividef(g0, 1.f + __expf(-1.5957691216057308f * (g0 + 0.044715f * g0 * g0 * g0))) * u0;
+        b = __fdividef(g1, 1.f + __expf(-1.5957691216057308f * (g1 + 0.044715f * g1 * g1 * g1))) * u1;
+      } else if constexpr (GLU == GLU_CLAMPED) {
+        g0 = fminf(g0, p.limit);
+        g1 = fminf(g1, p.limit);
+        a = __fdividef(g0, 1.f + __expf(-1.702f * g0)) * (fminf(fmaxf(u0, -p.limit), p.limit) + 1.f);
+        b = __fdividef(g1, 1.f + __expf(-1.702f * g1)) * (fminf(fmaxf(u1, -p.limit), p.limit) + 1.f);
+      } else {
+        a = g0 / (1.f + __expf(-g0)) * u0;
+        b = g1 / (1.f + __expf(-g1)) * u1;
       }
-    };
-    // 32 packed columns (half 0 or 1 of the slab) into this thread's row
-    auto park = [&](const uint32_t (&u)[16], int half) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        *reinterpret_cast<uint4*>(slab + row * 128 + (((half * 4 + q) ^ (row & 7)) << 4)) =
-            make_uint4(u[4 * q], u[4 * q + 1], u[4 * q + 2], u[4 * q + 3]);
+      return pack_bf16(a, b);
     };
     // the slab's last store has been read out of shared memory when this returns
     auto slab_free = [&] {
@@ -416,19 +345,27 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
           for (int half = 0; half < 2; ++half) {
             __syncwarp();                    // a tensor-memory load is a warp instruction
             const int c = sl * SLAB + half * 32;
-            uint32_t rg[32], ru[32], u[16];
+            uint32_t rg[32], ru[32];
             tmem_ld_32x32(t_addr + uint32_t(c), rg);
             tmem_ld_32x32(t_addr + uint32_t(BN / 2 + c), ru);
             tmem_ld_wait();
             if (half == 1 && sl + GROUPS >= BN / 2 / SLAB) acc_read();
-            gated(rg, ru, jo + c, u);
-            if (STAGED) {
-              park(u, half);
+            if constexpr (STAGED) {
+              uint32_t u[16];
+#pragma unroll
+              for (int t = 0; t < 16; ++t) u[t] = gated(rg, ru, jo + c, 2 * t);
+              slab_put(slab, row, half, u);
             } else if (gi < row_end) {
+              // each 16 bytes are stored as they are done: four stores at the end of the 32 columns made the whole
+              // product 7 % slower (1100 x 24576 x 4096: 175 us against 160 us)
               __nv_bfloat16* dst = p.C + (long long)gi * p.ldc + jo + c;
 #pragma unroll
-              for (int q = 0; q < 4; ++q)
-                *reinterpret_cast<uint4*>(dst + q * 8) = make_uint4(u[4 * q], u[4 * q + 1], u[4 * q + 2], u[4 * q + 3]);
+              for (int q = 0; q < 4; ++q) {
+                uint32_t u[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) u[e] = gated(rg, ru, jo + c, q * 8 + 2 * e);
+                *reinterpret_cast<uint4*>(dst + q * 8) = make_uint4(u[0], u[1], u[2], u[3]);
+              }
             }
           }
           if constexpr (STAGED) slab_out(jo + sl * SLAB, row0);
@@ -464,21 +401,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
 #pragma unroll
             for (int t = 0; t < 32; ++t) v[t] = __uint_as_float(r[half][t]);
             finish(v, col + half * 32, col + SLAB <= p.N);
-            if constexpr (FORM == GF_RESIDUAL) {
-#pragma unroll
-              for (int q = 0; q < 4; ++q) {
-                const uint4 a = *reinterpret_cast<const uint4*>(slab + row * 128 + (((half * 4 + q) ^ (row & 7)) << 4));
-                const uint32_t w[4] = {a.x, a.y, a.z, a.w};
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                  v[q * 8 + 2 * e] += __uint_as_float(w[e] << 16);
-                  v[q * 8 + 2 * e + 1] += __uint_as_float(w[e] & 0xffff0000u);
-                }
-              }
-            }
+            if constexpr (FORM == GF_RESIDUAL) slab_add(slab, row, half, v);
 #pragma unroll
             for (int t = 0; t < 16; ++t) u[t] = pack_bf16(v[2 * t], v[2 * t + 1]);
-            park(u, half);
+            slab_put(slab, row, half, u);
           }
           slab_out(col, row0);
         }
@@ -628,13 +554,12 @@ static void launch_form(const CUtensorMap& ta, const CUtensorMap& tb, const CUte
   if (e != cudaSuccess) throw std::runtime_error(std::string("gemm launch: ") + cudaGetErrorString(e));
 }
 
-// The staged epilogue for a short main loop, or a CTA's last tile being half of its work, and an output that TMA can
-// describe; grouped rows (a tile may end inside
+// The staged epilogue for a short main loop and an output that TMA can describe; grouped rows (a tile may end inside
 // another group's rows) and the fp32 forms have the other one only.
 template <int BN, int STAGES, int GLU = GLU_NONE, int FORM = GF_PLAIN>
 static void launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int grid, cudaStream_t stream) {
   if constexpr (FORM == GF_PLAIN || FORM == GF_XIELU) {
-    if ((p.K <= STAGED_K || p.total_work <= 2 * grid) && p.ldc % 8 == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0) {
+    if (p.K <= STAGED_K && p.ldc % 8 == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0) {
       const CUtensorMap tc = make_tmap_bf16_2d(p.C, p.M, p.N, p.ldc, BM, SLAB);
       launch_form<BN, STAGES, GLU, FORM, true>(ta, tb, tc, ta, p, grid, stream);
       return;
@@ -671,8 +596,8 @@ void gemm_bf16(const void* x, const void* w, void* c, const void* bias, int M, i
   p.act = act;
   p.status = ws.status;
   const bool swapped = (M <= 256);
-  if (!swapped && gemm_pairs_mode() && act != ACT_GEGLU_TANH &&
-      gemm_bf16_2cta(x, w, c, bias, M, N, K, ldx, ldw, ldc, act, sm_limit, ws.status, stream))
+  if (!swapped && act != ACT_GEGLU_TANH && (gemm_pairs_mode() || (K <= STAGED_K && sm_limit <= 0 && gemm_pairs_faster(M, N, K, sms))) &&
+      gemm_bf16_2cta(x, w, c, bias, nullptr, M, N, K, ldx, ldw, ldc, 0, act, sm_limit, ws.status, stream))
     return;
   if (!swapped) {
     // tokens are the 128-row operand
@@ -745,6 +670,9 @@ bool gemm_bf16_residual(const void* x, const void* w, void* c, const void* bias,
   constexpr int BN = 256;
   auto fits = [](const void* p, long long ld) { return ld % 8 == 0 && (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   if (M <= 256 || N < BN || K <= 0 || !fits(c, ldc) || !fits(residual, ldr)) return false;
+  if (sm_limit <= 0 && gemm_pairs_faster(M, N, K, gemm_num_sms()) &&
+      gemm_bf16_2cta(x, w, c, bias, residual, M, N, K, ldx, ldw, ldc, ldr, ACT_NONE, sm_limit, ws.status, stream))
+    return true;
   GemmParams p = prefill_params(c, M, N, K, ldc, ws);
   p.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
   p.num_n = (N + BN - 1) / BN;

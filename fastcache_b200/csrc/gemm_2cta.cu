@@ -12,17 +12,19 @@
 //            GPU's memory; every CTA fetches its own tiles), completion counted on the LEADER's (rank 0) barrier
 //   warp 1   leader only: tcgen05.mma.cta_group::2 (4 x K = 16 per stage); tcgen05.commit to both CTAs' barriers
 //            frees the stage in both and publishes the accumulator to both epilogues
-//   warps 2-5 epilogue in both CTAs: tcgen05.ld of the CTA's own 128 x 256 fp32 half, bias / activation / SwiGLU,
-//            16-byte bf16 stores; the 256 epilogue threads of the pair hand the accumulator back to the leader
+//   warps 2-9 epilogue in both CTAs, two groups of four as in the staged form of gemm.cu: tcgen05.ld of the CTA's own
+//            128 x 256 fp32 half, bias / activation / SwiGLU / residual, slabs of 64 columns through shared memory and
+//            TMA; the 512 epilogue threads of the pair hand the accumulator back to the leader
 // Two accumulators (2 x 256 TMEM columns per CTA) let the epilogue overlap the next tile's main loop.
 //
 // Every wait is bounded; both CTAs always reach the closing cluster barrier, so neither exits while its partner
 // may still signal one of its barriers.
 //
 // Measured (32768 x 6144 x 4096): tensor pipe 88.5 % active against 81.1 % for gemm.cu, but both kernels run into
-// the board's power limit (SM clock about 1.44 GHz) and take the same time within noise, so gemm_bf16 uses this
-// kernel only when asked to (FC_GEMM_PAIRS=1 / set_gemm_pairs(1)).  Asking for tiles 16 K blocks ahead to be
-// brought into L2 (cp.async.bulk.prefetch.tensor) made the K = 12288 shape 30 % slower and was taken out.
+// the board's power limit (SM clock about 1.44 GHz) and take the same time within noise, so sizes like that come here
+// only when asked to (FC_GEMM_PAIRS=1 / set_gemm_pairs(1)).  Asking for tiles 16 K blocks ahead to be brought into L2
+// (cp.async.bulk.prefetch.tensor) made the K = 12288 shape 30 % slower and was taken out.  Short products run at full
+// clock, where gemm.cu's four stages do not cover the latency of its 94 bytes per clock and SM: see gemm_pairs_faster.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -34,6 +36,7 @@
 #include <string>
 
 #include "gemm.h"
+#include "gemm_epilogue.cuh"
 #include "ptx.cuh"
 
 namespace fc {
@@ -45,17 +48,17 @@ constexpr int P2_BNH = 128;         // rows of B per CTA (256 per pair)
 constexpr int P2_BN = 256;
 constexpr int P2_BK = 64;
 constexpr int P2_STAGES = 6;
-constexpr int P2_THREADS = 192;
+constexpr long long PAIRS_MAX = 64 * 1024;
+constexpr int P2_THREADS = 320;
 constexpr int P2_A_BYTES = P2_BM * P2_BK * 2;
 constexpr int P2_B_BYTES = P2_BNH * P2_BK * 2;
 constexpr int P2_STAGE_BYTES = P2_A_BYTES + P2_B_BYTES;              // 32 KiB per CTA
-constexpr int P2_BAR_OFF = P2_STAGES * P2_STAGE_BYTES;
+constexpr int P2_SLAB_OFF = P2_STAGES * P2_STAGE_BYTES;
+constexpr int P2_BAR_OFF = P2_SLAB_OFF + 2 * SLAB_BYTES;
 constexpr int P2_SMEM = P2_BAR_OFF + 256 + 1024;
 
 struct Pair2Params {
   int M, N, K;
-  __nv_bfloat16* C;
-  long long ldc;
   const __nv_bfloat16* bias;
   int act;
   int num_m, num_n, group_m, total_work;
@@ -63,20 +66,7 @@ struct Pair2Params {
   uint32_t* status;
 };
 
-__device__ __forceinline__ float p2_act(float v, int act) {
-  switch (act) {
-    case ACT_RELU: return fmaxf(v, 0.f);
-    case ACT_GELU: return 0.5f * v * (1.f + erff(v * 0.70710678118654752f));
-    case ACT_GELU_TANH: {
-      float u = 0.7978845608028654f * (v + 0.044715f * v * v * v), th;
-      asm("tanh.approx.f32 %0, %1;" : "=f"(th) : "f"(u));
-      return 0.5f * v * (1.f + th);
-    }
-    case ACT_QUICK_GELU: return __fdividef(v, 1.f + __expf(-1.702f * v));
-    case ACT_SILU: return __fdividef(v, 1.f + __expf(-v));
-    default: return v;
-  }
-}
+enum PairForm : int { PF_PLAIN = 0, PF_SWIGLU = 1, PF_RESIDUAL = 2 };
 
 // 2-D tiled load whose completion is counted on a barrier of the pair's leader CTA (`bar_cluster_addr` is a
 // shared::cluster address); the destination is this CTA's own shared memory
@@ -106,18 +96,21 @@ __device__ __forceinline__ void p2_arrive_cluster(uint32_t bar_cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster_addr) : "memory");
 }
 
-template <bool SWIGLU>
+template <int FORM>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(P2_THREADS, 1)
 gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
+                      const __grid_constant__ CUtensorMap tma_c, const __grid_constant__ CUtensorMap tma_r,
                       const Pair2Params p) {
+  constexpr bool SWIGLU = FORM == PF_SWIGLU;
   extern __shared__ uint8_t smem_raw[];
   // the dynamic shared memory starts at the same offset in both CTAs, so the aligned base does too
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + P2_BAR_OFF);      // used in the leader
   uint64_t* empty_bar = full_bar + P2_STAGES;                               // one set per CTA
   uint64_t* acc_full = empty_bar + P2_STAGES;                               // [2], one set per CTA
-  uint64_t* acc_empty = acc_full + 2;                                       // [2], used in the leader (256 arrivals)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  uint64_t* acc_empty = acc_full + 2;                                       // [2], used in the leader (512 arrivals)
+  uint64_t* res_full = acc_empty + 2;                                       // [2], PF_RESIDUAL, one per epilogue group
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(res_full + 2);
   volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5;
@@ -133,7 +126,8 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&acc_full[a], 1);
-      mbar_init(&acc_empty[a], 256);
+      mbar_init(&acc_empty[a], 512);
+      mbar_init(&res_full[a], 1);
     }
     *s_abort = 0;
     fence_barrier_init();
@@ -253,111 +247,93 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
     // ---------------------------------------------------------------- epilogue (both CTAs)
     const int lane_group = warp & 3;
     const int row = lane_group * 32 + lane;
+    const int group = (warp - 2) >> 2;                        // takes the slabs group, group + 2, ...
+    const bool leader = warp == 2 + 4 * group && lane == 0;
+    uint8_t* const slab = smem + P2_SLAB_OFF + group * SLAB_BYTES;
+    const int width = SWIGLU ? p.N / 2 : p.N;
     int acc = 0;
-    uint32_t acc_phase = 0;
+    uint32_t acc_phase = 0, res_phase = 0;
     for (int w = pair; w < p.total_work; w += num_pairs) {
       int m_blk, n_blk;
       decode_work(w, m_blk, n_blk);
-      if (*s_abort || !mbar_wait(&acc_full[acc], acc_phase, p.status, ST_TIMEOUT_ACC_FULL)) {
+      // a group goes on or gives up as one: its threads meet at barriers below
+      if (!barrier_all(1 + group, 128, !*s_abort && mbar_wait(&acc_full[acc], acc_phase, p.status, ST_TIMEOUT_ACC_FULL))) {
         *s_abort = 1;
         break;
       }
       tc_fence_after();
       const uint32_t t_addr = tmem_base + (uint32_t(lane_group * 32) << 16) + uint32_t(acc * P2_BN);
       const uint32_t give_back = cluster_map_shared(smem_u32(&acc_empty[acc]), 0);
-      const int gi = m_blk * (2 * P2_BM) + int(rank) * P2_BM + row;
-      if constexpr (SWIGLU) {
-        // accumulator columns [0, 128) = gate, [128, 256) = up; out[:, n_blk * 128 + j] = silu(gate_j) * up_j
-        const int jo = n_blk * P2_BNH;
+      const int row0 = m_blk * (2 * P2_BM) + int(rank) * P2_BM;
+      const int col0 = n_blk * (SWIGLU ? P2_BNH : P2_BN);
+      constexpr int SLABS = (SWIGLU ? P2_BNH : P2_BN) / SLAB;
 #pragma unroll 1
-        for (int c = 0; c < P2_BNH / 32; ++c) {
-          uint32_t rg[32], ru[32];
-          tmem_ld_32x32(t_addr + uint32_t(c * 32), rg);
-          tmem_ld_32x32(t_addr + uint32_t(P2_BNH + c * 32), ru);
+      for (int sl = group; sl < SLABS; sl += 2) {
+        const int col = col0 + sl * SLAB;
+        const bool here = col < width && row0 < p.M;          // the same for the whole group
+        if (leader) tma_store_wait_read();                    // the slab's last store has been read out of shared memory
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
+        if (FORM == PF_RESIDUAL && leader && here) {          // what is added arrives while the accumulator is read
+          mbar_expect_tx(&res_full[group], SLAB_BYTES);
+          tma_load_2d(slab, &tma_r, &res_full[group], col, row0);
+        }
+        __syncwarp();                                         // a tensor-memory load is a warp instruction
+        uint32_t r[2][32];
+        if constexpr (!SWIGLU) {
+          tmem_ld_32x32(t_addr + uint32_t(sl * SLAB), r[0]);
+          tmem_ld_32x32(t_addr + uint32_t(sl * SLAB + 32), r[1]);
           tmem_ld_wait();
-          if (c == P2_BNH / 32 - 1) {
+          if (sl + 2 >= SLABS) {
             tc_fence_before();
             p2_arrive_cluster(give_back);
-          }
-          if (gi < p.M) {
-            __nv_bfloat16* dst = p.C + (long long)gi * p.ldc + jo + c * 32;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              uint32_t u[4];
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const int t = q * 8 + e * 2;
-                const float g0 = __uint_as_float(rg[t]), g1 = __uint_as_float(rg[t + 1]);
-                const float a = __fdividef(g0, 1.f + __expf(-g0)) * __uint_as_float(ru[t]);
-                const float b = __fdividef(g1, 1.f + __expf(-g1)) * __uint_as_float(ru[t + 1]);
-                u[e] = pack_bf16(a, b);
-              }
-              *reinterpret_cast<uint4*>(dst + q * 8) = make_uint4(u[0], u[1], u[2], u[3]);
-            }
           }
         }
-      } else {
-        const int j0 = n_blk * P2_BN;
-#pragma unroll 1
-        for (int c = 0; c < P2_BN / 32; ++c) {
-          uint32_t r[32];
-          tmem_ld_32x32(t_addr + uint32_t(c * 32), r);
-          tmem_ld_wait();
-          if (c == P2_BN / 32 - 1) {
-            tc_fence_before();
-            p2_arrive_cluster(give_back);
-          }
-          const int jb = j0 + c * 32;
-          if (gi >= p.M || jb >= p.N) continue;
-          float v[32];
+        if (FORM == PF_RESIDUAL && here) {
+          if (!mbar_wait(&res_full[group], res_phase, p.status, ST_TIMEOUT_FULL)) *s_abort = 1;    // (no barrier is skipped)
+          res_phase ^= 1;
+        }
 #pragma unroll
-          for (int t = 0; t < 32; ++t) v[t] = __uint_as_float(r[t]);
-          __nv_bfloat16* dst = p.C + (long long)gi * p.ldc + jb;
-          const bool vec_ok = (jb + 32 <= p.N) && ((reinterpret_cast<uintptr_t>(dst) & 15) == 0);
-          if (vec_ok) {
-            if (p.bias != nullptr) {
-              if ((reinterpret_cast<uintptr_t>(p.bias + jb) & 15) == 0) {
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                  const uint4 bv = *reinterpret_cast<const uint4*>(p.bias + jb + q * 8);
-                  const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
-#pragma unroll
-                  for (int e = 0; e < 4; ++e) {      // a bf16 is the upper half of the fp32 with the same value
-                    v[q * 8 + e * 2] += __uint_as_float(bw[e] << 16);
-                    v[q * 8 + e * 2 + 1] += __uint_as_float(bw[e] & 0xffff0000u);
-                  }
-                }
-              } else {
-#pragma unroll
-                for (int t = 0; t < 32; ++t) v[t] += __bfloat162float(p.bias[jb + t]);
-              }
-            }
-            if (p.act != ACT_NONE) {
-#pragma unroll
-              for (int t = 0; t < 32; ++t) v[t] = p2_act(v[t], p.act);
+        for (int half = 0; half < 2; ++half) {
+          uint32_t u[16];
+          if constexpr (SWIGLU) {
+            // accumulator columns [0, 128) = gate, [128, 256) = up
+            const int c = sl * SLAB + half * 32;
+            tmem_ld_32x32(t_addr + uint32_t(c), r[0]);
+            tmem_ld_32x32(t_addr + uint32_t(P2_BNH + c), r[1]);
+            tmem_ld_wait();
+            if (half == 1 && sl + 2 >= SLABS) {
+              tc_fence_before();
+              p2_arrive_cluster(give_back);
             }
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              uint32_t u[4];
-#pragma unroll
-              for (int e = 0; e < 4; ++e) u[e] = pack_bf16(v[q * 8 + e * 2], v[q * 8 + e * 2 + 1]);
-              *reinterpret_cast<uint4*>(dst + q * 8) = make_uint4(u[0], u[1], u[2], u[3]);
+            for (int t = 0; t < 16; ++t) {
+              const float g0 = __uint_as_float(r[0][2 * t]), g1 = __uint_as_float(r[0][2 * t + 1]);
+              u[t] = pack_bf16(g0 / (1.f + __expf(-g0)) * __uint_as_float(r[1][2 * t]),
+                               g1 / (1.f + __expf(-g1)) * __uint_as_float(r[1][2 * t + 1]));
             }
           } else {
+            float v[32];
 #pragma unroll
-            for (int t = 0; t < 32; ++t) {
-              if (jb + t < p.N) {
-                float a = v[t];
-                if (p.bias != nullptr) a += __bfloat162float(p.bias[jb + t]);
-                dst[t] = __float2bfloat16(p2_act(a, p.act));
-              }
-            }
+            for (int t = 0; t < 32; ++t) v[t] = __uint_as_float(r[half][t]);
+            if (p.bias != nullptr) add_bias_chunk(v, p.bias, col + half * 32, p.N, col + SLAB <= p.N);
+            if constexpr (FORM == PF_RESIDUAL) slab_add(slab, row, half, v);
+            else apply_act_chunk(v, p.act);
+#pragma unroll
+            for (int t = 0; t < 16; ++t) u[t] = pack_bf16(v[2 * t], v[2 * t + 1]);
           }
+          slab_put(slab, row, half, u);
+        }
+        fence_proxy_async();
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
+        if (leader && here) {
+          tma_store_2d(slab, &tma_c, col, row0);
+          tma_store_commit();
         }
       }
       acc ^= 1;
       if (acc == 0) acc_phase ^= 1;
     }
+    if (leader) tma_store_wait_all();
   }
 
   tc_fence_before();
@@ -370,9 +346,9 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
 
 int g_pairs = -1;
 
-template <bool SWIGLU>
-void p2_launch(const CUtensorMap& ta, const CUtensorMap& tb, const Pair2Params& p, int pairs, cudaStream_t stream) {
-  auto kern = gemm_bf16_2cta_kernel<SWIGLU>;
+template <int FORM>
+void p2_launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const CUtensorMap& tr, const Pair2Params& p, int pairs, cudaStream_t stream) {
+  auto kern = gemm_bf16_2cta_kernel<FORM>;
   static std::atomic<uint64_t> configured{0};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -382,7 +358,7 @@ void p2_launch(const CUtensorMap& ta, const CUtensorMap& tb, const Pair2Params& 
     if (e != cudaSuccess) throw std::runtime_error(std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
     configured.fetch_or(bit, std::memory_order_relaxed);
   }
-  kern<<<2 * pairs, P2_THREADS, P2_SMEM, stream>>>(ta, tb, p);
+  kern<<<2 * pairs, P2_THREADS, P2_SMEM, stream>>>(ta, tb, tc, tr, p);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) throw std::runtime_error(std::string("2-CTA gemm launch: ") + cudaGetErrorString(e));
 }
@@ -398,20 +374,33 @@ int gemm_pairs_mode() {
 }
 void set_gemm_pairs(int mode) { g_pairs = mode ? 1 : 0; }
 
-bool gemm_bf16_2cta(const void* x, const void* w, void* c, const void* bias, int M, int N, int K, long long ldx,
-                    long long ldw, long long ldc, int act, int sm_limit, uint32_t* status, cudaStream_t stream) {
+// Whether a pair's tiles are the faster ones: short products run at full clock, where a wave of 256 x 256 pair tiles takes
+// about 0.85 of a wave of 128 x 256 tiles (15 x 577 rows of the CLIP tower: qkv 45.4 -> 43.0 us, out 25.4 -> 22.9 us, fc2
+// 62.5 -> 53.6 us; fc1 with its activation 64.6 -> 67.2 us, where the pair's lead is the last epilogue's length; 5 x 961
+// rows of SigLIP: 37.6 -> 35.0 us, 24.1 -> 21.9 us, 63.6 -> 53.7 us, fc1 49.7 -> 47.4 us), so they are taken unless they
+// need another wave.  Products of more than PAIRS_MAX (waves x K) run at the power limit, where both take the same time, and
+// gemm_bf16 asks for pairs up to K = 2048 only (what it measured at K = 4096: gemm.cu).
+bool gemm_pairs_faster(int M, int N, int K, int sms) {
+  if (M <= 256 || N < 256 || sms < 2) return false;
+  auto up = [](long long a, long long b) { return (a + b - 1) / b; };
+  const long long n = up(N, 256), one = up(up(M, 128) * n, sms), two = up(up(M, 256) * n, sms / 2);
+  return one * K <= PAIRS_MAX && two <= one;
+}
+
+// Columns [0, N) of `residual` (pitch ldr) are added where it is given.  False where the sizes or layouts do not fit.
+bool gemm_bf16_2cta(const void* x, const void* w, void* c, const void* bias, const void* residual, int M, int N, int K,
+                    long long ldx, long long ldw, long long ldc, long long ldr, int act, int sm_limit, uint32_t* status,
+                    cudaStream_t stream) {
   const bool swiglu = act == ACT_SWIGLU;
   if (M <= 256 || N < 256 || K < P2_BK) return false;
-  if (swiglu && (N % 256 != 0 || ldc % 8 != 0 || (reinterpret_cast<uintptr_t>(c) & 15) != 0 || bias != nullptr))
-    return false;
+  if (ldc % 8 != 0 || (reinterpret_cast<uintptr_t>(c) & 15) != 0) return false;
+  if (swiglu && (N % 256 != 0 || bias != nullptr)) return false;
   const int sms = sm_limit > 0 ? sm_limit : gemm_num_sms();
   if (sms < 2) return false;
   Pair2Params p{};
   p.M = M;
   p.N = N;
   p.K = K;
-  p.C = reinterpret_cast<__nv_bfloat16*>(c);
-  p.ldc = ldc;
   p.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
   p.act = swiglu ? ACT_NONE : act;
   p.num_m = (M + 2 * P2_BM - 1) / (2 * P2_BM);
@@ -430,8 +419,10 @@ bool gemm_bf16_2cta(const void* x, const void* w, void* c, const void* bias, int
   const CUtensorMap ta = make_tmap_bf16_2d(x, M, K, ldx, P2_BM, P2_BK);
   const CUtensorMap tb = make_tmap_bf16_2d(w, N, K, ldw, P2_BNH, P2_BK);
   const int pairs = std::max(1, std::min(p.total_work, sms / 2));
-  if (swiglu) p2_launch<true>(ta, tb, p, pairs, stream);
-  else p2_launch<false>(ta, tb, p, pairs, stream);
+  const CUtensorMap tc = make_tmap_bf16_2d(c, M, swiglu ? N / 2 : N, ldc, P2_BM, SLAB);
+  if (swiglu) p2_launch<PF_SWIGLU>(ta, tb, tc, tc, p, pairs, stream);
+  else if (residual == nullptr) p2_launch<PF_PLAIN>(ta, tb, tc, tc, p, pairs, stream);
+  else p2_launch<PF_RESIDUAL>(ta, tb, tc, make_tmap_bf16_2d(residual, M, N, ldr, P2_BM, SLAB), p, pairs, stream);
   return true;
 }
 

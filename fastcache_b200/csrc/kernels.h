@@ -9,6 +9,8 @@ constexpr int DECODE_MAX_SPLITS = 32;
 
 void launch_rms_norm(const void* x, void* residual, const void* w, void* y, long long T, int H, float eps,
                      cudaStream_t s);
+void launch_add_grid_positions(const void* x, const void* table, const int* grids, void* y, int B, int N, int C, int n, int side,
+                               cudaStream_t s);
 void launch_layer_norm(const void* x, const void* w, const void* b, void* y, long long T, int H, float eps,
                        cudaStream_t s);
 void launch_silu_and_mul(const void* x, void* y, long long T, int I, cudaStream_t s);

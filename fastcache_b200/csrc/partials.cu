@@ -29,6 +29,16 @@ add_rms_norm_partials_kernel(const float* __restrict__ partial, int splits, long
   pdl_wait();
   const long long row = blockIdx.x;
   const int chunks = H >> 3;
+  // residual and weights are asked for with the first partial sums: this kernel is a chain of round trips to L2
+  uint4 res[PN_MAX_CHUNKS], gain[PN_MAX_CHUNKS];
+#pragma unroll
+  for (int c = 0; c < PN_MAX_CHUNKS; ++c) {
+    const int idx = threadIdx.x + c * PN_THREADS;
+    if (idx < chunks) {
+      res[c] = *reinterpret_cast<const uint4*>(residual + row * H + idx * 8);
+      gain[c] = *reinterpret_cast<const uint4*>(w + idx * 8);
+    }
+  }
   float v[PN_MAX_CHUNKS][8];
   float ss = 0.f;
 #pragma unroll
@@ -47,8 +57,7 @@ add_rms_norm_partials_kernel(const float* __restrict__ partial, int splits, long
         acc[4] += b.x; acc[5] += b.y; acc[6] += b.z; acc[7] += b.w;
       }
       uint4* rp = reinterpret_cast<uint4*>(residual + row * H + idx * 8);
-      const uint4 ru = *rp;
-      const __nv_bfloat162* rh = reinterpret_cast<const __nv_bfloat162*>(&ru);
+      const __nv_bfloat162* rh = reinterpret_cast<const __nv_bfloat162*>(&res[c]);
       uint4 su;
       uint32_t* sw = reinterpret_cast<uint32_t*>(&su);
 #pragma unroll
@@ -86,8 +95,7 @@ add_rms_norm_partials_kernel(const float* __restrict__ partial, int splits, long
   for (int c = 0; c < PN_MAX_CHUNKS; ++c) {
     const int idx = threadIdx.x + c * PN_THREADS;
     if (idx < chunks) {
-      const uint4 gu = *reinterpret_cast<const uint4*>(w + idx * 8);
-      const __nv_bfloat162* gh = reinterpret_cast<const __nv_bfloat162*>(&gu);
+      const __nv_bfloat162* gh = reinterpret_cast<const __nv_bfloat162*>(&gain[c]);
       uint4 ou;
       uint32_t* ow = reinterpret_cast<uint32_t*>(&ou);
 #pragma unroll

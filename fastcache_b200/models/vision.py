@@ -18,7 +18,7 @@ The towers are replicated on every tensor-parallel rank, like the reference's.
 """
 from __future__ import annotations
 
-from typing import Any, Dict, Optional, Tuple
+from typing import Any, Dict, List, Optional, Tuple
 
 import numpy as np
 import torch
@@ -238,6 +238,7 @@ class _SiglipEmbeddings(nn.Module):
         super().__init__()
         self.patch_embedding = _PatchEmbed(dim, patch, bias=True)
         self.num_patches_per_side = image_size // patch
+        self._buckets: Dict[int, np.ndarray] = {}
         self.position_embedding = nn.Embedding(self.num_patches_per_side ** 2, dim)
         self.position_embedding.weight.requires_grad_(False)
 
@@ -256,6 +257,27 @@ class _SiglipEmbeddings(nn.Module):
         return ids
 
 
+    def buckets(self, n: int) -> np.ndarray:
+        """Table row (or column) of each of n patches along one side: the statement of `position_ids`, kept per n."""
+        if n not in self._buckets:
+            side = self.num_patches_per_side
+            f = torch.arange(0, 1 - 1e-6, 1 / n)
+            self._buckets[n] = torch.bucketize(f, torch.arange(1 / side, 1.0, 1 / side), right=True).int().numpy()
+        return self._buckets[n]
+
+    def add_positions(self, x: torch.Tensor, sizes: List[List[int]]) -> Tuple[torch.Tensor, torch.Tensor]:
+        """x + its positions, and the patch counts, on the device: one small copy carries the buckets of every grid, the
+        look-up and the sum are one kernel (ids of all patches made on the host took longer than a layer)."""
+        n = max(max(s) for s in sizes)
+        grids = np.zeros((len(sizes), 2 + 2 * n), dtype=np.int32)
+        for g, (h, w) in zip(grids, sizes):
+            g[:2] = h, w
+            g[2:2 + h], g[2 + n:2 + n + w] = self.buckets(h), self.buckets(w)
+        grids_d = torch.from_numpy(grids).pin_memory().to(x.device, non_blocking=True)
+        y = ops.add_grid_positions(x, self.position_embedding.weight, grids_d, self.num_patches_per_side)
+        return y, grids_d[:, 0] * grids_d[:, 1]
+
+
 class SiglipVisionTower(nn.Module):
     def __init__(self, cfg):
         super().__init__()
@@ -271,11 +293,18 @@ class SiglipVisionTower(nn.Module):
         Returns (features [B, max_patches, dim], key mask [B, max_patches])."""
         x = self.embeddings.patch_embedding(pixels)
         B, N, _ = x.shape
-        counts = (tgt_sizes[:, 0] * tgt_sizes[:, 1]).to(x.device)
-        mask = torch.arange(N, device=x.device)[None, :] < counts[:, None]
-        pos = self.embeddings.position_ids(tgt_sizes.cpu(), N).to(x.device)
-        x = x + self.embeddings.position_embedding.weight.to(x.dtype)[pos]
-        key_mask = None if bool(mask.all()) else mask
+        sizes = tgt_sizes.tolist()
+        table = self.embeddings.position_embedding.weight
+        if x.is_cuda and x.dtype == table.dtype == torch.bfloat16 and sizes and all(h > 0 and w > 0 and h * w <= N for h, w in sizes):
+            x, counts = self.embeddings.add_positions(x, sizes)
+            mask = torch.arange(N, device=x.device)[None, :] < counts[:, None]
+            key_mask = None if all(h * w == N for h, w in sizes) else mask
+        else:
+            counts = (tgt_sizes[:, 0] * tgt_sizes[:, 1]).to(x.device)
+            mask = torch.arange(N, device=x.device)[None, :] < counts[:, None]
+            pos = self.embeddings.position_ids(tgt_sizes.cpu(), N).to(x.device)
+            x = x + table.to(x.dtype)[pos]
+            key_mask = None if bool(mask.all()) else mask
         for layer in self.encoder.layers:
             x = layer(x, key_mask)
         return self.post_layernorm(x), mask

@@ -49,6 +49,12 @@ def layer_norm(x, weight, bias, eps):
     return ref.layer_norm(x, weight, bias, eps)
 
 
+def add_grid_positions(x, table, grids, side: int):
+    """x [B, N, C] + rows of the [side * side, C] table (CUDA; `grids`: see csrc/elementwise.cu)."""
+    _n()
+    return ext().add_grid_positions(x.contiguous(), table.contiguous(), grids, int(side))
+
+
 def silu_and_mul(x):
     if x.is_cuda:
         _n()

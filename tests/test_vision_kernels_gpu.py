@@ -66,3 +66,16 @@ def test_dense_attention_at_tile_edges(D, Sq, Sk):
     nothing = torch.zeros(B, Sk, dtype=torch.bool, device=DEV)
     assert torch.equal(ops.dense_attention(q, k, v, D ** -0.5, nothing, impl=2), torch.zeros_like(q))
     _clean()
+
+
+@pytest.mark.parametrize("C", [64, 1152])
+def test_grid_positions_equal_those_made_on_the_host(C):
+    from fastcache_b200.models.vision import _SiglipEmbeddings
+    emb = _SiglipEmbeddings(C, 14, 980).to(torch.bfloat16).to(DEV)
+    emb.position_embedding.weight.data = _normal(70 * 70, C, seed=5)
+    sizes = [[1, 1], [70, 3], [31, 30], [18, 32], [2, 70], [35, 29], [13, 1]]
+    N = 1100
+    x = _normal(len(sizes), N, C, seed=6)
+    want = x + emb.position_embedding.weight[emb.position_ids(torch.tensor(sizes), N).to(DEV)]
+    got, counts = emb.add_positions(x, sizes)
+    assert torch.equal(got, want) and counts.tolist() == [h * w for h, w in sizes]
