@@ -24,6 +24,8 @@ import numpy as np
 import torch
 from torch import nn
 
+from torch.nn.modules.module import _has_any_global_hook
+
 from .. import ops
 
 CLIP_MEAN = (0.48145466, 0.4578275, 0.40821073)
@@ -34,6 +36,13 @@ SIGLIP_STD = (0.5, 0.5, 0.5)
 
 def _param(*shape) -> nn.Parameter:
     return nn.Parameter(torch.zeros(*shape), requires_grad=False)
+
+
+def _adds(module: nn.Module, kind: type) -> bool:
+    """Whether `module` may be handed the rows that its output is added to.  A block that somebody put in another's place
+    takes its own arguments only, and whoever watches a block (hooks of its own or of all modules) sees its own output."""
+    return (type(module) is kind and "forward" not in vars(module) and not _has_any_global_hook()
+            and not (module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks))
 
 
 class VLinear(nn.Module):
@@ -81,7 +90,11 @@ class VisionAttention(nn.Module):
             self.fuse()
         qkv = ops.linear(x.reshape(B * S, C), self._qkv_w, self._qkv_b).view(B, S, 3, self.heads, self.head_dim)
         o = ops.dense_attention(qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2], self.head_dim ** -0.5, key_mask)
-        return self.out_proj(o.reshape(B * S, C), residual=None if residual is None else residual.reshape(B * S, C)).view(B, S, C)
+        o = o.reshape(B * S, C)
+        if residual is not None and _adds(self.out_proj, VLinear):
+            return self.out_proj(o, residual=residual.reshape(B * S, C)).view(B, S, C)
+        y = self.out_proj(o).view(B, S, C)
+        return y if residual is None else residual + y
 
 
 class VisionMLP(nn.Module):
@@ -90,7 +103,11 @@ class VisionMLP(nn.Module):
         self.fc1, self.fc2, self.act = VLinear(dim, inter), VLinear(inter, dim), act
 
     def forward(self, x: torch.Tensor, residual: Optional[torch.Tensor] = None) -> torch.Tensor:
-        return self.fc2(self.fc1(x, self.act), residual=residual)
+        h = self.fc1(x, self.act)
+        if residual is not None and _adds(self.fc2, VLinear):
+            return self.fc2(h, residual=residual)
+        y = self.fc2(h)
+        return y if residual is None else residual + y
 
 
 class VisionLayer(nn.Module):
@@ -102,12 +119,12 @@ class VisionLayer(nn.Module):
 
     def forward(self, x: torch.Tensor, key_mask: Optional[torch.Tensor] = None) -> torch.Tensor:
         B, S, C = x.shape
-        attn, mlp = self.self_attn, self.mlp
-        if attn._forward_hooks or attn.out_proj._forward_hooks or mlp._forward_hooks or mlp.fc2._forward_hooks:
-            x = x + attn(self.layer_norm1(x), key_mask)             # whoever watches a block sees its own output
-            return x + mlp(self.layer_norm2(x).reshape(B * S, C)).view(B, S, C)
-        x = attn(self.layer_norm1(x), key_mask, residual=x)
-        return mlp(self.layer_norm2(x).reshape(B * S, C), residual=x.reshape(B * S, C)).view(B, S, C)
+        h = self.layer_norm1(x)
+        x = self.self_attn(h, key_mask, residual=x) if _adds(self.self_attn, VisionAttention) else x + self.self_attn(h, key_mask)
+        h = self.layer_norm2(x).reshape(B * S, C)
+        if _adds(self.mlp, VisionMLP):
+            return self.mlp(h, residual=x.reshape(B * S, C)).view(B, S, C)
+        return x + self.mlp(h).view(B, S, C)
 
 
 class _Encoder(nn.Module):

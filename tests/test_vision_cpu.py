@@ -1,9 +1,11 @@
 """Multimodal models on the CPU path: image rows replace the placeholder, KV accounting, slicing."""
+import pytest
 import torch
+from torch import nn
 
 from fastcache_b200 import LLM, ModelConfig, SamplingParams
 from fastcache_b200.models.minicpm import best_grid, slice_image
-from fastcache_b200.models.vision import CLIPVisionTower, sincos_2d
+from fastcache_b200.models.vision import CLIPVisionTower, VisionLayer, sincos_2d
 
 
 def _llava_cfg():
@@ -76,3 +78,66 @@ def test_minicpm_slicing_and_rows():
         out += o
     assert len(out[0][1]) == 3
     assert sincos_2d(32, 3, 5).shape == (3, 5, 32)
+
+
+class _Calls(nn.Module):
+    """A block in the place of another, with the arguments that blocks have always had."""
+
+    def __init__(self, inner, *names):
+        super().__init__()
+        self.inner, self.names = inner, names
+
+    def forward(self, x, key_mask=None):
+        return self.inner(x, key_mask) if "key_mask" in self.names else self.inner(x)
+
+
+def _vision_layer():
+    torch.manual_seed(2)
+    layer = VisionLayer(64, 4, 128, "gelu", 1e-6)
+    for p in layer.parameters():
+        nn.init.normal_(p, std=0.2)
+    return layer, torch.randn(2, 9, 64)
+
+
+def _linear(v):
+    new = nn.Linear(v.weight.shape[1], v.weight.shape[0])
+    new.weight, new.bias = v.weight, v.bias
+    return new
+
+
+@pytest.mark.parametrize("place", ["self_attn", "self_attn.out_proj", "mlp", "mlp.fc2"])
+def test_vision_blocks_can_be_replaced(place):
+    layer, x = _vision_layer()
+    want = layer(x)
+    owner = layer.get_submodule(place.rpartition(".")[0])
+    name = place.rpartition(".")[2]
+    old = getattr(owner, name)
+    setattr(owner, name, _linear(old) if "." in place else _Calls(old, "key_mask" if place == "self_attn" else ""))
+    torch.testing.assert_close(layer(x), want)
+
+
+@pytest.mark.parametrize("place", ["self_attn", "self_attn.out_proj", "mlp", "mlp.fc2"])
+@pytest.mark.parametrize("watch", ["hook", "global hook", "keyword pre-hook", "own forward"])
+def test_who_watches_a_vision_block_sees_its_own_arguments_and_output(place, watch):
+    layer, x = _vision_layer()
+    want = layer(x)
+    block = layer.get_submodule(place)
+    seen = []
+    if watch == "hook":
+        handle = block.register_forward_hook(lambda m, args, out: seen.append((args, {}, out)))
+    elif watch == "global hook":
+        handle = nn.modules.module.register_module_forward_hook(lambda m, args, out: seen.append((args, {}, out)) if m is block else None)
+    elif watch == "keyword pre-hook":
+        handle = block.register_forward_pre_hook(lambda m, args, kw: seen.append((args, kw, None)), with_kwargs=True)
+    else:
+        inner, handle = block.forward, None
+        block.forward = lambda *args, **kw: seen.append((args, kw, inner(*args, **kw))) or seen[-1][2]
+    torch.testing.assert_close(layer(x), want)
+    if handle is not None:
+        handle.remove()
+    else:
+        del block.forward
+    (args, kw, out), = seen
+    assert not kw
+    if out is not None:                                  # what the block gives for these arguments alone
+        torch.testing.assert_close(out, block(*args))
