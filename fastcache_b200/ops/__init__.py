@@ -83,10 +83,11 @@ def linear(x, weight, bias=None, act: str = "none", out: Optional[torch.Tensor] 
 
 
 def linear_add(x, weight, bias, residual):
-    """residual + x @ weight.T + bias, [T, N]; the prompt-size CUDA GEMM adds in its epilogue."""
-    if x.is_cuda:
+    """residual + x @ weight.T + bias; the prompt-size CUDA GEMM adds in its epilogue where the operands are that kernel's."""
+    if x.is_cuda and bias is not None and all(t.dtype == torch.bfloat16 for t in (x, weight, bias, residual)):
         from ..parallel.fused import get_fused_comm
-        if get_fused_comm() is None and residual.dtype == x.dtype and x.stride(-1) == 1 and residual.stride(-1) == 1:
+        if (get_fused_comm() is None and x.dim() == 2 and residual.shape == (x.shape[0], weight.shape[0])
+                and x.stride(1) == 1 and residual.stride(1) == 1 and not (torch.is_grad_enabled() and residual.requires_grad)):
             y = ext().gemm_residual(x, weight, bias, residual)
             if y is not None:
                 _n()

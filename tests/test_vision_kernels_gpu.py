@@ -50,6 +50,31 @@ def test_added_residual_of_few_rows_and_other_pitches():
         assert ((got.double() - want).abs() <= 2.0 ** -7 * (sums[:rows].abs() + want.abs()) + 1e-5).all()      # two roundings at most
 
 
+@pytest.mark.parametrize("rows", [20, 300])
+@pytest.mark.parametrize("form", ["no bias", "batches", "one row for all", "columns", "fp32 residual", "fp32", "gradient"])
+def test_added_residual_takes_what_linear_takes(rows, form):
+    """Whatever `linear` and an addition behind it take, with their result."""
+    x, w, b, r = _normal(rows, 256, seed=1), _normal(512, 256, seed=2, scale=0.06), _normal(512, seed=3), _normal(rows, 512, seed=4)
+    if form == "no bias":
+        b = None
+    elif form == "batches":
+        x, r = x.view(2, rows // 2, 256), r.view(2, rows // 2, 512)
+    elif form == "one row for all":
+        r = r[:1]
+    elif form == "columns":                                # both with another unit stride than the kernel's
+        x, r = x.t().contiguous().t(), r.t().contiguous().t()
+    elif form == "fp32 residual":
+        r = r.float()
+    elif form == "fp32":
+        x, w, b, r = x.float(), w.float(), b.float(), r.float()
+    else:
+        r.requires_grad_()
+    got, want = ops.linear_add(x, w, b, r), r + ops.linear(x, w, b)
+    assert got.dtype == want.dtype and got.shape == want.shape and got.requires_grad == want.requires_grad
+    # the sum may be rounded once instead of twice
+    assert ((got.float() - want.float()).abs() <= 2.0 ** -7 * (want.float().abs() + (want - r).float().abs()) + 1e-5).all()
+
+
 @pytest.mark.parametrize("D", [8, 40, 64, 72, 80, 96, 128])
 @pytest.mark.parametrize("Sq,Sk", [(1, 1), (127, 63), (128, 64), (129, 65), (256, 127), (257, 128), (130, 129), (64, 400)])
 def test_dense_attention_at_tile_edges(D, Sq, Sk):
