@@ -312,7 +312,8 @@ class SiglipVisionTower(nn.Module):
         B, N, _ = x.shape
         sizes = tgt_sizes.tolist()
         table = self.embeddings.position_embedding.weight
-        if x.is_cuda and x.dtype == table.dtype == torch.bfloat16 and sizes and all(h > 0 and w > 0 and h * w <= N for h, w in sizes):
+        if (x.is_cuda and x.dtype == table.dtype == torch.bfloat16 and len(sizes) == B > 0
+                and all(h > 0 and w > 0 and h * w <= N for h, w in sizes)):
             x, counts = self.embeddings.add_positions(x, sizes)
             mask = torch.arange(N, device=x.device)[None, :] < counts[:, None]
             key_mask = None if all(h * w == N for h, w in sizes) else mask

@@ -104,3 +104,17 @@ def test_grid_positions_equal_those_made_on_the_host(C):
     want = x + emb.position_embedding.weight[emb.position_ids(torch.tensor(sizes), N).to(DEV)]
     got, counts = emb.add_positions(x, sizes)
     assert torch.equal(got, want) and counts.tolist() == [h * w for h, w in sizes]
+
+
+def test_one_grid_for_several_slices():
+    """A tower takes one row of sizes for a batch of slices that all have them."""
+    from types import SimpleNamespace
+    from fastcache_b200.models.vision import SiglipVisionTower
+    tower = SiglipVisionTower(SimpleNamespace(hidden_size=64, patch_size=14, image_size=140, num_hidden_layers=2, num_attention_heads=4,
+                                              intermediate_size=128, layer_norm_eps=1e-6))
+    for i, p in enumerate(tower.parameters()):
+        p.data = _normal(*p.shape, seed=i, scale=0.1)
+    pixels = _normal(3, 3, 56, 70, seed=40)
+    one, mask = tower(pixels, torch.tensor([[4, 5]]))
+    want, _ = tower(pixels, torch.tensor([[4, 5]] * 3))
+    assert mask.shape == (1, 20) and torch.equal(one, want)
