@@ -93,6 +93,23 @@ def test_dense_attention_at_tile_edges(D, Sq, Sk):
     _clean()
 
 
+@pytest.mark.parametrize("D", [64, 72])
+@pytest.mark.parametrize("level", [-20.0, -200.0, 200.0])
+def test_first_tiles_without_a_key_before_scores_far_from_zero(D, level):
+    """The reference of a row's exponents is its first key's, not zero: no weight may vanish where all scores are low."""
+    B, Sq, Sk, H = 2, 130, 400, 2
+    q, k, v = (_normal(B, n, H, D, seed=i) for i, n in enumerate((Sq, Sk, Sk)))
+    q[..., 0], k[..., 0] = 16.0, level                      # every score is near 16 * level / 8
+    mask = torch.ones(B, Sk, dtype=torch.bool, device=DEV)
+    mask[0, :128], mask[1, :256] = False, False
+    for m in (mask, None):
+        got = ops.dense_attention(q, k, v, 0.125, m, impl=2)
+        want = ref.dense_attention(q.double(), k.double(), v.double(), 0.125, m)
+        # P and the result in bf16 as above, and scores near 2 * level whose sums carry 2^-24 for each product
+        assert (got.double() - want).abs().max() <= (2 * 2.0 ** -8 + D * 2.0 ** -24 * 2 * abs(level)) * v.float().abs().max()
+    _clean()
+
+
 @pytest.mark.parametrize("C", [64, 1152])
 def test_grid_positions_equal_those_made_on_the_host(C):
     from fastcache_b200.models.vision import _SiglipEmbeddings
