@@ -267,7 +267,7 @@ dense_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         m_ref = mx;
       } else if (__any_sync(0xffffffffu, mx > m_ref + DT_RESCALE_THRESHOLD)) {
         // some row of this warp outgrew its reference: bring O (complete up to tile j - 1) to the new one
-        if (!mbar_wait(o_done, uint32_t(j - 1) & 1u, p.status, ST_TIMEOUT_ACC_FULL)) {
+        if (!__all_sync(0xffffffffu, mbar_wait(o_done, uint32_t(j - 1) & 1u, p.status, ST_TIMEOUT_ACC_FULL))) {
           ok = false;
           break;
         }
@@ -309,13 +309,14 @@ dense_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       l += rs;
     }
     if (!ok) *s_abort = 1;
-    if (ok && mbar_wait(o_done, uint32_t(n_tiles - 1) & 1u, p.status, ST_TIMEOUT_ACC_FULL)) {
+    if (ok && __all_sync(0xffffffffu, mbar_wait(o_done, uint32_t(n_tiles - 1) & 1u, p.status, ST_TIMEOUT_ACC_FULL))) {
       tc_fence_after();
       const float inv = l > 0.f ? 1.f / l : 0.f;
       bf16* dst = p.out + (((long long)b * p.Sq + qrow) * p.H + h) * p.D;
 #pragma unroll 1
       for (int c = 0; c < DP / 32; ++c) {
         if (c * 32 >= p.D) break;                       // uniform over the warp
+        __syncwarp();                                   // a tensor-memory load is a warp instruction
         uint32_t r[32];
         tmem_ld_32x32(to + uint32_t(c * 32), r);
         tmem_ld_wait();

@@ -355,7 +355,7 @@ ccm_fused_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_constan
         //      GEMM1 (a thread has read columns 0 ... 2 c + 31 of its row when it writes columns c ... c + 15), and over
         //      the first activation tile, which GEMM2 is done with
         for (int g = 0; g < 2 && ok; ++g) {
-          if (!mbar_wait(&acc_full[g], g == 0 ? tile_phase : 0u, p.status, ST_TIMEOUT_ACC_FULL)) {
+          if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[g], g == 0 ? tile_phase : 0u, p.status, ST_TIMEOUT_ACC_FULL))) {
             ok = false;
             break;
           }
@@ -388,7 +388,7 @@ ccm_fused_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_constan
         }
         if (!ok) break;
         // ---- epilogue 3: bias, bf16, scatter the rows of this tile
-        if (!mbar_wait(&acc_full[1], 1u, p.status, ST_TIMEOUT_ACC_FULL)) {
+        if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[1], 1u, p.status, ST_TIMEOUT_ACC_FULL))) {
           ok = false;
           break;
         }
@@ -400,6 +400,7 @@ ccm_fused_kernel(const __grid_constant__ CUtensorMap tm_w1, const __grid_constan
           const uint32_t t_addr = tmem_base + (uint32_t(lane_group * 32) << 16) + 128u;
 #pragma unroll 1
           for (int c4 = 0; c4 < 4; ++c4) {
+            __syncwarp();                        // a tensor-memory load is a warp instruction
             uint32_t rr[32];
             tmem_ld_32x32(t_addr + uint32_t(c4 * 32), rr);
             tmem_ld_wait();

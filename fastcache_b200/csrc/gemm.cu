@@ -257,7 +257,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     const int group = STAGED ? (warp - 2) >> 2 : 0;  // takes the slabs group, group + 2, ...
     const bool leader = warp == 2 + 4 * group && lane == 0;
     uint8_t* const slab = smem + L::SLAB_OFF + group * SLAB_BYTES;
-    auto group_bar = [&] { asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory"); };
+    auto group_bar = [&] {                           // a warp instruction: lanes that went ways of their own meet first
+      __syncwarp();
+      asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
+    };
     constexpr int GROUPS = STAGED ? 2 : 1;
     int acc = 0;
     uint32_t acc_phase = 0, res_phase = 0;
@@ -313,14 +316,16 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         tma_store_2d(slab, &tma_c, col, row0);
         tma_store_commit();
       }
+      __syncwarp();                          // a tensor-memory load may follow, a warp instruction
     };
 
     for (int w = blockIdx.x; w < total_work; w += gridDim.x) {
       int m_blk, n_blk;
       decode_work(w, m_blk, n_blk);
       bool ok = !s_flag[0] && mbar_wait(&acc_full[acc], acc_phase, p.status, ST_TIMEOUT_ACC_FULL);
-      // a staged group goes on or gives up as one: its threads meet at barriers below
+      // a staged group goes on or gives up as one, and so does a warp: their threads meet below
       if constexpr (STAGED) ok = barrier_all(1 + group, 128, ok);
+      else ok = __all_sync(0xffffffffu, ok);
       if (!ok) {
         s_flag[0] = 1;
         break;
@@ -380,6 +385,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
               mbar_expect_tx(&res_full[group], SLAB_BYTES);
               tma_load_2d(slab, &tma_r, &res_full[group], col, row0);
             }
+            __syncwarp();
           }
           uint32_t r[2][32];
           tmem_ld_32x32(t_addr + uint32_t(sl * SLAB), r[0]);

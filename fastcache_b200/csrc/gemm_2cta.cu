@@ -251,6 +251,10 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
     const bool leader = warp == 2 + 4 * group && lane == 0;
     uint8_t* const slab = smem + P2_SLAB_OFF + group * SLAB_BYTES;
     const int width = SWIGLU ? p.N / 2 : p.N;
+    auto group_bar = [&] {                                    // a warp instruction: lanes that went ways of their own meet first
+      __syncwarp();
+      asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
+    };
     int acc = 0;
     uint32_t acc_phase = 0, res_phase = 0;
     for (int w = pair; w < p.total_work; w += num_pairs) {
@@ -272,7 +276,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
         const int col = col0 + sl * SLAB;
         const bool here = col < width && row0 < p.M;          // the same for the whole group
         if (leader) tma_store_wait_read();                    // the slab's last store has been read out of shared memory
-        asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
+        group_bar();
         if (FORM == PF_RESIDUAL && leader && here) {          // what is added arrives while the accumulator is read
           mbar_expect_tx(&res_full[group], SLAB_BYTES);
           tma_load_2d(slab, &tma_r, &res_full[group], col, row0);
@@ -324,11 +328,12 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
           slab_put(slab, row, half, u);
         }
         fence_proxy_async();
-        asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory");
+        group_bar();
         if (leader && here) {
           tma_store_2d(slab, &tma_c, col, row0);
           tma_store_commit();
         }
+        __syncwarp();
       }
       acc ^= 1;
       if (acc == 0) acc_phase ^= 1;
