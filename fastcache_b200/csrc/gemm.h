@@ -112,8 +112,11 @@ bool gemm_bf16_2cta(const void* x, const void* w, void* c, const void* bias, con
                     long long ldx, long long ldw, long long ldc, long long ldr, int act, int sm_limit, uint32_t* status,
                     cudaStream_t stream);
 bool gemm_pairs_faster(int M, int N, int K, int sms);
-int gemm_pairs_mode();            // FC_GEMM_PAIRS=1 / set_gemm_pairs(1): gemm_bf16 takes the pair form where it can
+// FC_GEMM_PAIRS / set_gemm_pairs: 0 never, 1 wherever the pair form can run, 2 (initial) where it is the faster one
+enum PairsMode : int { PAIRS_NEVER = 0, PAIRS_ALWAYS = 1, PAIRS_FASTER = 2 };
+int gemm_pairs_mode();
 void set_gemm_pairs(int mode);
+inline bool gemm_takes_pairs(bool faster) { return gemm_pairs_mode() == PAIRS_ALWAYS || (faster && gemm_pairs_mode() == PAIRS_FASTER); }
 bool streamk_enabled();
 void set_streamk(int mode);
 int streamk_mode();

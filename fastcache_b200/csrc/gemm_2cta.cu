@@ -373,11 +373,11 @@ void p2_launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& 
 int gemm_pairs_mode() {
   if (g_pairs < 0) {
     const char* e = std::getenv("FC_GEMM_PAIRS");
-    g_pairs = (e != nullptr && e[0] == '1') ? 1 : 0;
+    g_pairs = e != nullptr && (e[0] == '0' || e[0] == '1') ? e[0] - '0' : PAIRS_FASTER;
   }
   return g_pairs;
 }
-void set_gemm_pairs(int mode) { g_pairs = mode ? 1 : 0; }
+void set_gemm_pairs(int mode) { g_pairs = mode == PAIRS_NEVER || mode == PAIRS_FASTER ? mode : PAIRS_ALWAYS; }
 
 // Whether a pair's tiles are the faster ones: short products run at full clock, where a wave of 256 x 256 pair tiles takes
 // about 0.85 of a wave of 128 x 256 tiles (15 x 577 rows of the CLIP tower: qkv 45.4 -> 43.0 us, out 25.4 -> 22.9 us, fc2

@@ -59,6 +59,28 @@ def test_swiglu_on_cta_pairs(forms, M, I, K):
         assert ((y.float() - want).abs() / (want.abs() + 1.0)).max().item() < 3e-2
 
 
+def _kernels(f):
+    f()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        f()
+        torch.cuda.synchronize()
+    return [e.key for e in prof.key_averages() if "gemm_bf16" in e.key]
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2])
+# M, N, K: a short product that needs no more waves of pairs, one that does, one at the power limit, all on 148 SMs
+@pytest.mark.parametrize("M,N,K,faster", [(4805, 1152, 1152, True), (4616, 1024, 1024, False), (4096, 6144, 12288, False)])
+def test_the_switch_says_which_kernel_runs(forms, mode, M, N, K, faster):
+    forms.set_gemm_pairs(mode)
+    assert forms.gemm_pairs_mode() == mode
+    x, w, b, r = _rand(M, K), _rand(N, K), _rand(N), _rand(M, N)
+    want = mode == 1 or (mode == 2 and faster)
+    for product in (lambda: ops.linear(x, w, b), lambda: ops.linear(x, w, None, "gelu_tanh"), lambda: ops.linear(x, w, None, "swiglu"),
+                    lambda: ops.linear_add(x, w, b, r)):
+        name, = _kernels(product)
+        assert ("2cta" in name) == want, name
+
+
 def test_cta_pairs_on_a_side_stream_and_repeated(forms):
     e = forms
     e.set_gemm_pairs(1)

@@ -23,9 +23,18 @@ def _close(got, want, K):
     assert ((got.double() - want).abs() <= bound).all()
 
 
+@pytest.fixture(params=[0, 1, 2], ids=["one CTA per tile", "CTA pairs", "by size"])
+def pairs(request):
+    e = ops.ext()
+    before = e.gemm_pairs_mode()
+    e.set_gemm_pairs(request.param)
+    yield request.param
+    e.set_gemm_pairs(before)
+
+
 @pytest.mark.parametrize("M", [257, 384, 1000])
 @pytest.mark.parametrize("N,K", [(256, 64), (264, 1024), (328, 2048), (1152, 4304), (3000, 136)])
-def test_staged_epilogue_at_ragged_sizes(M, N, K):
+def test_staged_epilogue_at_ragged_sizes(pairs, M, N, K):
     x, w, b, r = _normal(M, K, seed=1), _normal(N, K, seed=2, scale=K ** -0.5), _normal(N, seed=3), _normal(M, N, seed=4)
     sums = x.double() @ w.double().T + b.double()
     _close(ops.linear(x, w, b), sums, K)
@@ -38,6 +47,27 @@ def test_staged_epilogue_at_ragged_sizes(M, N, K):
     ops.linear(x, w, b, out=odd[:, :N])
     _close(odd[:, :N], sums, K)
     assert (odd[:, N:] == 7).all()
+    _clean()
+
+
+# two tiles of a CTA and more, where a slab's last store may still be under way, and one tile of several groups of rows
+@pytest.mark.parametrize("M,N,K", [(4616, 1024, 1024), (4616, 1024, 4096), (20001, 1032, 320)])
+def test_staged_epilogue_of_many_tiles(pairs, M, N, K):
+    x, w, b, r = _normal(M, K, seed=1), _normal(N, K, seed=2, scale=K ** -0.5), _normal(N, seed=3), _normal(M, N, seed=4)
+    sums = x.double() @ w.double().T + b.double()
+    _close(ops.linear(x, w, b), sums, K)
+    _close(ops.linear_add(x, w, b, r), sums + r.double(), K)
+    _clean()
+
+
+@pytest.mark.parametrize("M,I,K", [(257, 128, 64), (1000, 384, 1024), (4616, 1024, 1024), (300, 640, 2056)])
+def test_gated_staged_epilogue(pairs, M, I, K):
+    x, w = _normal(M, K, seed=1), _normal(2 * I, K, seed=2, scale=K ** -0.5)
+    gate, up = (x.double() @ w.double().T).split(I, dim=1)
+    got, want = ops.linear(x, w, None, act="swiglu"), gate * gate.sigmoid() * up
+    # both sums carry K 2^-24 of their size; |silu'| <= 1.1; one rounding to bf16, and the fast exponential's 2^-21
+    bound = (2.0 ** -8 + 2.0 ** -20) * want.abs() + 1.1 * K * 2.0 ** -24 * (1 + gate.abs()) * (1 + up.abs()) + 1e-6
+    assert ((got.double() - want).abs() <= bound).all()
     _clean()
 
 
