@@ -1,0 +1,67 @@
+"""Decode attention with rings of two and of three tiles: which one runs follows from the number of CTAs, so both need
+batches of their own."""
+import pytest
+import torch
+
+from fastcache_b200 import ops
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _normal(*shape, seed):
+    return torch.randn(*shape, generator=torch.Generator().manual_seed(seed)).to(torch.bfloat16).to(DEV)
+
+
+def _statement(q, kc, vc, table, lens, scale):
+    B, Hq, D = q.shape
+    out = torch.zeros(B, Hq, D, dtype=torch.float64, device=DEV)
+    for i, n in enumerate(lens):
+        k, v = (c[table[i].long()].transpose(1, 2).flatten(0, 1)[:n].double() for c in (kc, vc))       # [n, Hkv, D]
+        k, v = (t.repeat_interleave(Hq // t.shape[1], dim=1) for t in (k, v))
+        out[i] = torch.einsum("hn,nhd->hd", (torch.einsum("hd,nhd->hn", q[i].double(), k) * scale).softmax(-1), v)
+    return out
+
+
+@pytest.fixture(params=[False, True], ids=["merge kernel", "merge in the kernel"])
+def merge(request):
+    e = ops.ext()
+    before = e.decode_merge_in_kernel()
+    e.set_decode_merge_in_kernel(request.param)
+    yield
+    e.set_decode_merge_in_kernel(before)
+
+
+# contexts: one tile, two, three (a ring that wraps), more; ends on and next to the edges of tiles
+LENS = [1, 63, 64, 65, 127, 128, 129, 192, 193, 256, 257, 320, 385, 700]
+
+
+@pytest.mark.parametrize("D,B,Hq,Hkv,bs,splits,stages", [
+    (128, 40, 32, 8, 256, 1, 2), (128, 75, 32, 8, 16, 1, 2), (128, 14, 56, 8, 64, 3, 2), (128, 30, 32, 8, 64, 1, 3),
+    (128, 60, 8, 8, 32, 1, 3), (64, 160, 4, 2, 16, 1, 2), (64, 56, 24, 2, 64, 3, 2), (64, 56, 24, 2, 64, 2, 3)])
+def test_both_rings(merge, D, B, Hq, Hkv, bs, splits, stages):
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the batches are made for 148 SMs")
+    lens = (LENS * 12)[:B]
+    pages = [-(-n // bs) for n in lens]
+    order = torch.randperm(sum(pages), generator=torch.Generator().manual_seed(3)).int()
+    table, at = torch.zeros(B, max(pages), dtype=torch.int32), 0
+    for i, p in enumerate(pages):
+        table[i, :p] = order[at:at + p]
+        at += p
+    kc, vc, q = _normal(at, Hkv, bs, D, seed=1), _normal(at, Hkv, bs, D, seed=2), _normal(B, Hq, D, seed=4)
+    table, ctx = table.to(DEV), torch.tensor(lens, dtype=torch.int32, device=DEV)
+
+    def call():
+        return ops.decode_attention(q, kc, vc, table, ctx, D ** -0.5, {"splits": splits})
+
+    first = call()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        got = call()
+        torch.cuda.synchronize()
+    names = [e.key.replace(" ", "") for e in prof.key_averages() if "decode_attn_kernel" in e.key]
+    assert len(names) == 1 and f"<{D},{stages}>" in names[0], names
+    assert torch.equal(got, first) and ops.ext().read_status(torch.cuda.current_device()) == 0
+    want = _statement(q, kc, vc, table, lens, D ** -0.5)
+    # weights and result are rounded to bf16 once each: 2^-9 of the largest value, and of the result
+    assert ((got.double() - want).abs() <= 2.0 ** -9 * (vc.float().abs().max() + want.abs()) * 1.01 + 1e-5).all()
