@@ -602,7 +602,7 @@ void gemm_bf16(const void* x, const void* w, void* c, const void* bias, int M, i
   p.act = act;
   p.status = ws.status;
   const bool swapped = (M <= 256);
-  if (!swapped && act != ACT_GEGLU_TANH && gemm_takes_pairs(K <= STAGED_K && sm_limit <= 0 && gemm_pairs_faster(M, N, K, sms)) &&
+  if (!swapped && act != ACT_GEGLU_TANH && gemm_takes_pairs(K <= STAGED_K && sm_limit <= 0 && gemm_pairs_faster(M, N, K, act, sms)) &&
       gemm_bf16_2cta(x, w, c, bias, nullptr, M, N, K, ldx, ldw, ldc, 0, act, sm_limit, ws.status, stream))
     return;
   if (!swapped) {
@@ -676,7 +676,7 @@ bool gemm_bf16_residual(const void* x, const void* w, void* c, const void* bias,
   constexpr int BN = 256;
   auto fits = [](const void* p, long long ld) { return ld % 8 == 0 && (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   if (M <= 256 || N < BN || K <= 0 || !fits(c, ldc) || !fits(residual, ldr)) return false;
-  if (gemm_takes_pairs(sm_limit <= 0 && gemm_pairs_faster(M, N, K, gemm_num_sms())) &&
+  if (gemm_takes_pairs(sm_limit <= 0 && gemm_pairs_faster(M, N, K, ACT_NONE, gemm_num_sms())) &&
       gemm_bf16_2cta(x, w, c, bias, residual, M, N, K, ldx, ldw, ldc, ldr, ACT_NONE, sm_limit, ws.status, stream))
     return true;
   GemmParams p = prefill_params(c, M, N, K, ldc, ws);

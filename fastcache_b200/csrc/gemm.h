@@ -111,7 +111,7 @@ bool gemm_streamk_bf16(const void* x, const void* w, void* c, const void* bias, 
 bool gemm_bf16_2cta(const void* x, const void* w, void* c, const void* bias, const void* residual, int M, int N, int K,
                     long long ldx, long long ldw, long long ldc, long long ldr, int act, int sm_limit, uint32_t* status,
                     cudaStream_t stream);
-bool gemm_pairs_faster(int M, int N, int K, int sms);
+bool gemm_pairs_faster(int M, int N, int K, int act, int sms);
 // FC_GEMM_PAIRS / set_gemm_pairs: 0 never, 1 wherever the pair form can run, 2 (initial) where it is the faster one
 enum PairsMode : int { PAIRS_NEVER = 0, PAIRS_ALWAYS = 1, PAIRS_FASTER = 2 };
 int gemm_pairs_mode();

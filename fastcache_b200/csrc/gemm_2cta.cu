@@ -48,7 +48,8 @@ constexpr int P2_BNH = 128;         // rows of B per CTA (256 per pair)
 constexpr int P2_BN = 256;
 constexpr int P2_BK = 64;
 constexpr int P2_STAGES = 6;
-constexpr long long PAIRS_MAX = 64 * 1024;
+constexpr long long PAIRS_MIN = 2 * 1024, PAIRS_MAX = 64 * 1024;      // waves x K, see gemm_pairs_faster
+constexpr int PAIRS_ACT_K = 1280;
 constexpr int P2_THREADS = 320;
 constexpr int P2_A_BYTES = P2_BM * P2_BK * 2;
 constexpr int P2_B_BYTES = P2_BNH * P2_BK * 2;
@@ -380,16 +381,23 @@ int gemm_pairs_mode() {
 void set_gemm_pairs(int mode) { g_pairs = mode == PAIRS_NEVER || mode == PAIRS_FASTER ? mode : PAIRS_ALWAYS; }
 
 // Whether a pair's tiles are the faster ones: short products run at full clock, where a wave of 256 x 256 pair tiles takes
-// about 0.85 of a wave of 128 x 256 tiles (15 x 577 rows of the CLIP tower: qkv 45.4 -> 43.0 us, out 25.4 -> 22.9 us, fc2
-// 62.5 -> 53.6 us; fc1 with its activation 64.6 -> 67.2 us, where the pair's lead is the last epilogue's length; 5 x 961
-// rows of SigLIP: 37.6 -> 35.0 us, 24.1 -> 21.9 us, 63.6 -> 53.7 us, fc1 49.7 -> 47.4 us), so they are taken unless they
-// need another wave.  Products of more than PAIRS_MAX (waves x K) run at the power limit, where both take the same time, and
-// gemm_bf16 asks for pairs up to K = 2048 only (what it measured at K = 4096: gemm.cu).
-bool gemm_pairs_faster(int M, int N, int K, int sms) {
+// about 0.85 of a wave of 128 x 256 tiles (one CTA per tile -> pairs, kernel times inside the towers: 15 x 577 rows of CLIP:
+// qkv 46.6 -> 43.3 us, out 25.2 -> 23.7 us, fc2 61.7 -> 53.8 us; 5 x 961 rows of SigLIP: 37.0 -> 34.7 us, 24.0 -> 22.3 us,
+// 63.9 -> 53.5 us, fc1 48.3 -> 47.1 us), so they are taken unless they need another wave.  What a pair adds is its longer
+// start and last epilogue, so the main loops have to be long enough to win that back:
+//  - PAIRS_MIN (waves x K): 577 x 4096 at K = 1024 12.8 -> 13.7 us, at K = 1536 15.6 -> 16.1 us; at the line 1 to 2 %
+//    either way (577 x 4096 at K = 2048 18.3 -> 18.6 us, sums with a residual a little faster); 1154 rows of CLIP: qkv 13.5 -> 14.4 us; 961 of SigLIP: qkv 14.2 -> 14.9 us, but fc2 (K = 4304) 34.5 -> 29.7 us.
+//  - an activation that takes an exponential or an error function below K = PAIRS_ACT_K, where the epilogue of every tile is
+//    longer than its main loop: CLIP's fc1 (quick GELU, K = 1024) 65.3 -> 68.5 us with 15 images, 29.5 -> 31.6 us with five;
+//    2000 x 8192 with quick GELU or SwiGLU at K = 1024: 3 and 2 % slower in pairs, at K = 1280: 4 % faster.
+// Products of more than PAIRS_MAX (waves x K) run at the power limit, where both take the same time, and gemm_bf16 asks for
+// pairs up to K = 2048 only (what it measured at K = 4096: gemm.cu).
+bool gemm_pairs_faster(int M, int N, int K, int act, int sms) {
   if (M <= 256 || N < 256 || sms < 2) return false;
   auto up = [](long long a, long long b) { return (a + b - 1) / b; };
   const long long n = up(N, 256), one = up(up(M, 128) * n, sms), two = up(up(M, 256) * n, sms / 2);
-  return one * K <= PAIRS_MAX && two <= one;
+  if (K < PAIRS_ACT_K && (act == ACT_GELU || act == ACT_QUICK_GELU || act == ACT_SILU || act == ACT_SWIGLU)) return false;
+  return one * K >= PAIRS_MIN && one * K <= PAIRS_MAX && two <= one;
 }
 
 // Columns [0, N) of `residual` (pitch ldr) are added where it is given.  False where the sizes or layouts do not fit.

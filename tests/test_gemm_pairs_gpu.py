@@ -68,17 +68,18 @@ def _kernels(f):
 
 
 @pytest.mark.parametrize("mode", [0, 1, 2])
-# M, N, K: a short product that needs no more waves of pairs, one that does, one at the power limit, all on 148 SMs
-@pytest.mark.parametrize("M,N,K,faster", [(4805, 1152, 1152, True), (4616, 1024, 1024, False), (4096, 6144, 12288, False)])
+# M, N, K: a short product that needs no more waves of pairs, one whose gated epilogue outlasts its main loop, one of a single
+# short wave, one that needs another wave, one at the power limit, all on 148 SMs
+@pytest.mark.parametrize("M,N,K,faster", [(4805, 1152, 1152, "pgar"), (8655, 4096, 1024, "par"), (577, 4096, 1024, ""), (4616, 1024, 1024, ""),
+                                          (4096, 6144, 12288, "")])
 def test_the_switch_says_which_kernel_runs(forms, mode, M, N, K, faster):
     forms.set_gemm_pairs(mode)
     assert forms.gemm_pairs_mode() == mode
     x, w, b, r = _rand(M, K), _rand(N, K), _rand(N), _rand(M, N)
-    want = mode == 1 or (mode == 2 and faster)
-    for product in (lambda: ops.linear(x, w, b), lambda: ops.linear(x, w, None, "gelu_tanh"), lambda: ops.linear(x, w, None, "swiglu"),
-                    lambda: ops.linear_add(x, w, b, r)):
+    for form, product in {"p": lambda: ops.linear(x, w, b), "a": lambda: ops.linear(x, w, None, "gelu_tanh"),
+                          "g": lambda: ops.linear(x, w, None, "swiglu"), "r": lambda: ops.linear_add(x, w, b, r)}.items():
         name, = _kernels(product)
-        assert ("2cta" in name) == want, name
+        assert ("2cta" in name) == (mode == 1 or (mode == 2 and form in faster)), name
 
 
 def test_cta_pairs_on_a_side_stream_and_repeated(forms):
