@@ -418,12 +418,18 @@ __global__ void decode_merge_kernel(const float* __restrict__ part_o, const floa
 
 // As many splits as fill the SMs once (rounded down: a few CTAs in a second wave cost as much as a full one) and at least
 // four tiles each.  24 requests x 8 heads around 1150 rows: 38.6 us with splits that overflow, 32.0 us so; 32 x 8 around
-// 100 rows, where the merge is what it costs: 18.0 us and 9.6 us.
+// 100 rows, where the merge is what it costs: 15.8 us and 8.1 us.
+// One split each where that leaves SMs with a single CTA is right while no request can be long: with contexts of more than
+// DEC_LONG rows in the batch the longest request's chain is what the step waits for, and two splits halve it.  32 x 8 heads,
+// one split and two: contexts up to 1850 rows, evenly spread 42.0 us and 44.2 us, all of 2000 rows 47.2 us and 57.1 us;
+// up to 3650 rows 76.7 us and 69.1 us, up to 7500 rows 147 us and 124 us; one of 8000 rows among 31 of 1000, 151 us and
+// 100 us.  (All of 4000 rows: 86.8 us and 95.9 us; the host knows the bound only.)
+constexpr int DEC_LONG = 2048;
 int decode_attn_pick_splits(int B, int Hkv, int max_ctx, int num_sms) {
-  const int ctas = B * Hkv;
-  const int target = dec_ctas_per_sm(2) * num_sms;
-  const int max_by_len = std::max(1, max_ctx / (4 * DEC_TILE));
-  return std::max(1, std::min({target / std::max(1, ctas), max_by_len, DECODE_MAX_SPLITS}));
+  const int ctas = std::max(1, B * Hkv);
+  int splits = dec_ctas_per_sm(2) * num_sms / ctas;
+  if (splits == 1 && ctas < 2 * num_sms && max_ctx > DEC_LONG) splits = 2;
+  return std::max(1, std::min({splits, max_ctx / (4 * DEC_TILE), DECODE_MAX_SPLITS}));
 }
 
 void launch_decode_attention(const void* q, const void* k_cache, const void* v_cache, const int* block_tables,

@@ -65,3 +65,24 @@ def test_both_rings(merge, D, B, Hq, Hkv, bs, splits, stages):
     want = _statement(q, kc, vc, table, lens, D ** -0.5)
     # weights and result are rounded to bf16 once each: 2^-9 of the largest value, and of the result
     assert ((got.double() - want).abs() <= 2.0 ** -9 * (vc.float().abs().max() + want.abs()) * 1.01 + 1e-5).all()
+
+
+@pytest.mark.parametrize("B,Hkv,bound,splits", [(32, 8, 2048, 1), (32, 8, 2304, 2), (28, 8, 4096, 2), (37, 8, 4096, 1), (27, 8, 1024, 2), (32, 8, 256, 1)])
+def test_splits_of_batches_that_leave_sms_with_one_cta(B, Hkv, bound, splits):
+    """The rule goes by the bound on the contexts: one long request among short ones is halved."""
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the batches are made for 148 SMs")
+    bs = 64
+    table = torch.arange(B * (bound // bs), dtype=torch.int32, device=DEV).view(B, -1) % 40
+    kc, vc, q = _normal(40, Hkv, bs, 128, seed=1), _normal(40, Hkv, bs, 128, seed=2), _normal(B, 4 * Hkv, 128, seed=4)
+    lens = [bound if i == 3 else 1 + 7 * i for i in range(B)]
+    ctx = torch.tensor(lens, dtype=torch.int32, device=DEV)
+    ops.decode_attention(q, kc, vc, table, ctx, 0.1)
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        got = ops.decode_attention(q, kc, vc, table, ctx, 0.1)
+        torch.cuda.synchronize()
+    names = [e.key for e in prof.key_averages()]
+    assert any("decode_attn_kernel" in n for n in names)
+    assert any("decode_merge_kernel" in n for n in names) == (splits > 1)
+    want = _statement(q, kc, vc, table, lens, 0.1)
+    assert ((got.double() - want).abs() <= 2.0 ** -9 * (vc.float().abs().max() + want.abs()) * 1.01 + 1e-5).all()
