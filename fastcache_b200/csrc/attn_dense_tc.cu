@@ -29,6 +29,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <cfloat>
 #include <mutex>
 #include <stdexcept>
 #include <string>
@@ -46,6 +47,9 @@ constexpr int DT_BN = 128;
 constexpr int DT_THREADS = 192;
 constexpr int DT_SUB_BYTES = 128 * 64 * 2;              // one [128 x 64] sub-tile
 constexpr float DT_RESCALE_THRESHOLD = 8.f;             // log2 units
+// reference of a row's exponents until its first key comes: every score that counts is above it and rescales by 2^-inf = 0
+// the zeros that are there so far
+constexpr float DT_NO_KEY = -FLT_MAX;
 
 __device__ __forceinline__ uint64_t dt_sdesc(uint32_t addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
   uint64_t d = 0;
@@ -222,7 +226,7 @@ dense_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     const uint32_t to = tmem_base + lane_addr + O_BASE;      // O
     const int qrow = q0 + row;
     const uint8_t* mrow = p.key_mask != nullptr ? p.key_mask + (long long)b * p.Sk : nullptr;
-    float m_ref = -INFINITY, l = 0.f;                        // -inf: no key attended to yet
+    float m_ref = 0.f, l = 0.f;
     bool ok = true;
     for (int j = 0; j < n_tiles && ok; ++j) {
       // keys that are not there or not attended to, looked up before the wait for S: lane t asks for key 32 c + t, all
@@ -264,7 +268,7 @@ dense_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
       mx *= p.scale_log2;
       if (j == 0) {
-        m_ref = mx;
+        m_ref = fmaxf(mx, DT_NO_KEY);
       } else if (__any_sync(0xffffffffu, mx > m_ref + DT_RESCALE_THRESHOLD)) {
         // some row of this warp outgrew its reference: bring O (complete up to tile j - 1) to the new one
         if (!__all_sync(0xffffffffu, mbar_wait(o_done, uint32_t(j - 1) & 1u, p.status, ST_TIMEOUT_ACC_FULL))) {
@@ -273,7 +277,7 @@ dense_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         }
         tc_fence_after();
         const float m_new = fmaxf(m_ref, mx);
-        const float f = m_ref == -INFINITY ? 0.f : exp2f(m_ref - m_new);
+        const float f = exp2f(m_ref - m_new);
         m_ref = m_new;
         l *= f;
 #pragma unroll 1
@@ -287,14 +291,13 @@ dense_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         }
         tmem_st_wait();
       }
-      const float base = m_ref == -INFINITY ? 0.f : m_ref;
       float rs4[4] = {0.f, 0.f, 0.f, 0.f};
       uint32_t u[64];
 #pragma unroll
       for (int t = 0; t < 64; ++t) {
         float e0, e1;
-        const float a0 = fmaf(__uint_as_float(s[2 * t]), p.scale_log2, -base);
-        const float a1 = fmaf(__uint_as_float(s[2 * t + 1]), p.scale_log2, -base);
+        const float a0 = fmaf(__uint_as_float(s[2 * t]), p.scale_log2, -m_ref);
+        const float a1 = fmaf(__uint_as_float(s[2 * t + 1]), p.scale_log2, -m_ref);
         asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e0) : "f"(a0));
         asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e1) : "f"(a1));
         rs4[t & 3] += e0 + e1;
