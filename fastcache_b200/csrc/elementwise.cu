@@ -9,6 +9,7 @@
 #include <stdexcept>
 #include <string>
 
+#include "gemm.h"
 #include "kernels.h"
 #include "launch.h"
 #include "ptx.cuh"
@@ -105,11 +106,11 @@ rms_norm_kernel(const bf16* __restrict__ x, bf16* __restrict__ residual, const b
   }
 }
 
-// One warp per row, CH 16-byte pieces per lane (rows up to 256 * CH elements, CH <= 16): both statistics are warp reductions, so
-// nothing waits at a barrier and a block has eight rows in flight.  Bound by the read and the write of a row; rows of
-// 1024 to 3584 elements (vision towers, resampler) with a block each, half of its threads idle and six barriers in
-// between, ran at a fifth of the copy rate.  8655 rows of 1024: 25.6 us
-// with a block per row, 9.7 us so.
+// One warp per row, CH 16-byte pieces per lane (rows up to 256 * CH elements, CH <= 8): both statistics are warp reductions, so
+// nothing waits at a barrier and a block has eight rows in flight.  Bound by the read and the write of a row; many rows of
+// 1024 to 2048 elements (vision towers) with a block each, half of its threads idle and six barriers in
+// between, ran at a fifth of the copy rate.  8655 rows of 1024: 24.1 us
+// with a block per row, 9.6 us so.
 template <int CH>
 __global__ void __launch_bounds__(NORM_THREADS)
 layer_norm_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const bf16* __restrict__ b,
@@ -166,9 +167,10 @@ layer_norm_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const 
   }
 }
 
-// rows of more than 4096 elements: one block each, a lane could not hold its share of a row
+// One block per row: for long rows, of which a lane's share is a long chain of its own, and where there are too few rows to
+// fill the SMs with a warp each (see launch_layer_norm).
 __global__ void __launch_bounds__(NORM_THREADS)
-layer_norm_long_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const bf16* __restrict__ b,
+layer_norm_block_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, const bf16* __restrict__ b,
                   bf16* __restrict__ y, int H, float eps) {
   __shared__ float red[32];
   const long long row = blockIdx.x;
@@ -645,12 +647,14 @@ void launch_layer_norm(const void* x, const void* w, const void* b, void* y, lon
                        cudaStream_t s) {
   if (T == 0) return;
   const int chunks = H >> 3;
-  if (chunks > 16 * 32) {
-    layer_norm_long_kernel<<<(unsigned)T, NORM_THREADS, 0, s>>>((const bf16*)x, (const bf16*)w, (const bf16*)b, (bf16*)y, H, eps);
+  // A block per row -> a warp per row: 577 rows of 1024, 2048: 3.3 -> 3.5 us, 4.0 -> 5.1 us; 800 rows: 4.7 -> 3.4 us, 5.5 ->
+  // 5.0 us, so the line is at four rows an SM; 64 rows of 512 2.7 us both, of 2048 2.9 -> 4.8 us.  Rows of 3584 never gain: 64
+  // rows 3.3 -> 6.9 us, 4805 rows 23.0 -> 23.4 us, 8655 rows 41.9 -> 50.3 us; of 2560 by 3 % from 8000 rows on.
+  if (chunks > 8 * 32 || (chunks > 2 * 32 && T <= 4ll * gemm_num_sms())) {
+    layer_norm_block_kernel<<<(unsigned)T, NORM_THREADS, 0, s>>>((const bf16*)x, (const bf16*)w, (const bf16*)b, (bf16*)y, H, eps);
     return;
   }
-  auto kern = chunks <= 4 * 32 ? layer_norm_kernel<4> : chunks <= 5 * 32 ? layer_norm_kernel<5> : chunks <= 8 * 32 ? layer_norm_kernel<8>
-              : layer_norm_kernel<16>;
+  auto kern = chunks <= 4 * 32 ? layer_norm_kernel<4> : chunks <= 5 * 32 ? layer_norm_kernel<5> : layer_norm_kernel<8>;
   constexpr int rows = NORM_THREADS / 32;
   kern<<<(unsigned)((T + rows - 1) / rows), NORM_THREADS, 0, s>>>((const bf16*)x, (const bf16*)w, (const bf16*)b, (bf16*)y, T, H, eps);
 }

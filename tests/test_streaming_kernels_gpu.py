@@ -101,6 +101,27 @@ def test_layer_norm_row_lengths(T, H):
     assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4).all()
 
 
+def _kernel(f, part):
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        f()
+        torch.cuda.synchronize()
+    name, = [e.key.replace(" ", "") for e in prof.key_averages() if part in e.key]
+    return name
+
+
+# a warp per row where there are more than four rows an SM, a block per row for fewer and for long rows
+@pytest.mark.parametrize("rows,H,kernel", [(4, 512, "<4>"), (4, 520, "block"), (4, 1280, "block"), (5, 520, "<4>"), (5, 1032, "<5>"), (5, 1288, "<8>"),
+                                           (5, 2048, "<8>"), (5, 2056, "block"), (5, 3584, "block")])
+def test_layer_norm_by_rows_per_sm(rows, H, kernel):
+    T = rows * torch.cuda.get_device_properties(0).multi_processor_count
+    x, w, b = (_normal(*s, seed=i) for i, s in enumerate([(T, H), (H,), (H,)]))
+    xd, wd, bd = (x + 3).to(DEV), w.to(DEV), b.to(DEV)
+    assert kernel in _kernel(lambda: ops.layer_norm(xd, wd, bd, 1e-5), "layer_norm")
+    want = torch.nn.functional.layer_norm(xd.double(), (H,), wd.double(), bd.double(), 1e-5)
+    # one rounding to bf16, and 32-bit sums
+    assert ((ops.layer_norm(xd, wd, bd, 1e-5).double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4).all()
+
+
 @pytest.mark.parametrize("Hq,Hkv", [(32, 8), (32, 32), (5, 3), (12, 2)])
 @pytest.mark.parametrize("norm", [False, True])
 def test_rotary_store_of_many_rows_equals_that_of_few(Hq, Hkv, norm):
