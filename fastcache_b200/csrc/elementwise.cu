@@ -377,6 +377,10 @@ rope_qknorm_store_kernel(const bf16* __restrict__ qkv, const long long* __restri
 
 // head_dim 128: eight lanes per (token, head), each lane owns 8 consecutive elements of the low
 // half and their rotation partners in the high half (two 16-byte loads, two 16-byte stores).
+// EARLY: angles (two round trips: position, then its row), slot and weights are asked for before qkv is there, which a grid of a
+// few blocks an SM waits for; where blocks follow one another the registers that this holds cost more than it hides (see
+// launch_rope_qknorm_store).
+template <bool EARLY>
 __global__ void __launch_bounds__(256)
 rope_qknorm_store_d128_kernel(const bf16* __restrict__ qkv, const long long* __restrict__ positions,
                               const float* __restrict__ cos_sin, const bf16* __restrict__ q_w,
@@ -393,15 +397,25 @@ rope_qknorm_store_d128_kernel(const bf16* __restrict__ qkv, const long long* __r
   const long long g = active ? gid : 0;
   const int t = int(g / heads);
   const int h = int(g - (long long)t * heads);
-  // position -> angles is two round trips: both are under way while the partial sums arrive, and so are slot and weights
-  const long long slot_in = h >= Hq && slots != nullptr ? (long long)slots[t] : -1;
-  const float4* cs = reinterpret_cast<const float4*>(cos_sin + positions[t] * 128);
-  const float4 c0 = cs[2 * j], c1 = cs[2 * j + 1], s0 = cs[16 + 2 * j], s1 = cs[16 + 2 * j + 1];
   const bf16* nw = h < Hq ? q_w : k_w;
+  long long slot = -1;
+  float4 c0, c1, s0, s1;
   uint4 gain_lo = make_uint4(0, 0, 0, 0), gain_hi = gain_lo;
-  if (nw != nullptr) {
+  auto load_slot = [&] {
+    if (h >= Hq && slots != nullptr) slot = slots[t];
+  };
+  auto load_angles = [&] {
+    const float4* cs = reinterpret_cast<const float4*>(cos_sin + positions[t] * 128);
+    c0 = cs[2 * j], c1 = cs[2 * j + 1], s0 = cs[16 + 2 * j], s1 = cs[16 + 2 * j + 1];
+  };
+  auto load_gains = [&] {
     gain_lo = reinterpret_cast<const uint4*>(nw)[j];
     gain_hi = reinterpret_cast<const uint4*>(nw)[8 + j];
+  };
+  if constexpr (EARLY) {
+    load_slot();
+    load_angles();
+    if (nw != nullptr) load_gains();
   }
   uint4 ulo, uhi;
   if (partial != nullptr) {
@@ -427,7 +441,7 @@ rope_qknorm_store_d128_kernel(const bf16* __restrict__ qkv, const long long* __r
     ulo = src[j];
     uhi = src[8 + j];
   }
-  long long slot = slot_in;
+  if constexpr (!EARLY) load_slot();
   if (slot >= num_slots) {
     report(status, ST_BAD_INDEX);
     slot = -1;
@@ -456,6 +470,7 @@ rope_qknorm_store_d128_kernel(const bf16* __restrict__ qkv, const long long* __r
   if (nw != nullptr) {
     const float inv = rsqrtf(ss / 128.f + eps);
     float wl[8], wh[8];
+    if constexpr (!EARLY) load_gains();
     unpack8(gain_lo, wl);
     unpack8(gain_hi, wh);
     auto rn = [](float v) { return __bfloat162float(__float2bfloat16(v)); };
@@ -465,6 +480,7 @@ rope_qknorm_store_d128_kernel(const bf16* __restrict__ qkv, const long long* __r
       hi[i] = rn(rn(hi[i] * inv) * wh[i]);
     }
   }
+  if constexpr (!EARLY) load_angles();
   const float c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
   const float s[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
   uint4 olo, ohi;
@@ -484,18 +500,16 @@ rope_qknorm_store_d128_kernel(const bf16* __restrict__ qkv, const long long* __r
   dst[8 + j] = ohi;
 }
 
-// The same for prompts, where the GEMM has finished qkv: one warp takes ROPE_HEADS * 4 heads of one token, every group
-// of eight lanes ROPE_HEADS of them, so the angles, the position and the slot are read once for them and each lane has
+// The same without norms for prompts, where the GEMM has finished qkv: one warp takes ROPE_HEADS * 4 heads of one token, every
+// group of eight lanes ROPE_HEADS of them, so the angles, the position and the slot are read once for them and each lane has
 // 2 * ROPE_HEADS 16-byte loads in flight.  Bound by reading qkv and writing it back rotated; 26120 tokens, 32 + 2 * 8 heads:
-// 147 us with one head per group of lanes, 119 us so (642 MB, 5.4 TB/s).
+// 149 us with one head per group of lanes, 114 us so (642 MB, 5.6 TB/s).
 constexpr int ROPE_HEADS = 4;
 
 __global__ void __launch_bounds__(256)
-rope_qknorm_store_rows_kernel(const bf16* __restrict__ qkv, const long long* __restrict__ positions,
-                              const float* __restrict__ cos_sin, const bf16* __restrict__ q_w,
-                              const bf16* __restrict__ k_w, bf16* __restrict__ q_out, bf16* __restrict__ k_cache,
-                              bf16* __restrict__ v_cache, const int* __restrict__ slots, int T, int Hq, int Hkv,
-                              float eps, long long num_slots, int block_size, uint32_t* status) {
+rope_store_rows_kernel(const bf16* __restrict__ qkv, const long long* __restrict__ positions, const float* __restrict__ cos_sin,
+                       bf16* __restrict__ q_out, bf16* __restrict__ k_cache, bf16* __restrict__ v_cache,
+                       const int* __restrict__ slots, int T, int Hq, int Hkv, long long num_slots, int block_size, uint32_t* status) {
   pdl_launch_dependents();
   pdl_wait();
   const int heads = Hq + 2 * Hkv, per_token = (heads + 4 * ROPE_HEADS - 1) / (4 * ROPE_HEADS);
@@ -531,28 +545,6 @@ rope_qknorm_store_rows_kernel(const bf16* __restrict__ qkv, const long long* __r
     float lo[8], hi[8];
     unpack8(ulo[i], lo);
     unpack8(uhi[i], hi);
-    const bool is_q = h < Hq;
-    const bf16* nw = is_q ? q_w : k_w;
-    if (q_w != nullptr || k_w != nullptr) {      // the same for every lane of the warp
-      float ss = 0.f;
-#pragma unroll
-      for (int e = 0; e < 8; ++e) ss += lo[e] * lo[e] + hi[e] * hi[e];
-      ss += __shfl_xor_sync(0xffffffffu, ss, 1);
-      ss += __shfl_xor_sync(0xffffffffu, ss, 2);
-      ss += __shfl_xor_sync(0xffffffffu, ss, 4);
-      if (nw != nullptr && h < Hq + Hkv) {
-        const float inv = rsqrtf(ss / 128.f + eps);
-        float wl[8], wh[8];
-        unpack8(reinterpret_cast<const uint4*>(nw)[j], wl);
-        unpack8(reinterpret_cast<const uint4*>(nw)[8 + j], wh);
-        auto rn = [](float v) { return __bfloat162float(__float2bfloat16(v)); };
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          lo[e] = rn(rn(lo[e] * inv) * wl[e]);
-          hi[e] = rn(rn(hi[e] * inv) * wh[e]);
-        }
-      }
-    }
     uint4 olo = ulo[i], ohi = uhi[i];
     bf16* dst = nullptr;
     if (h < Hq + Hkv) {
@@ -565,7 +557,7 @@ rope_qknorm_store_rows_kernel(const bf16* __restrict__ qkv, const long long* __r
         ph[e] = pack_bf16(hi[2 * e] * c[2 * e] + lo[2 * e] * s[2 * e],
                           hi[2 * e + 1] * c[2 * e + 1] + lo[2 * e + 1] * s[2 * e + 1]);
       }
-      if (is_q) dst = q_out + (t * Hq + h) * 128;
+      if (h < Hq) dst = q_out + (t * Hq + h) * 128;
       else if (row >= 0) dst = k_cache + (row + (long long)(h - Hq) * block_size) * 128;
     } else if (h < heads && row >= 0) {          // value head: plain copy into the pool
       dst = v_cache + (row + (long long)(h - Hq - Hkv) * block_size) * 128;
@@ -686,18 +678,26 @@ void launch_rope_qknorm_store(const void* qkv, const void* positions, const void
                               uint32_t* status, cudaStream_t s, const float* partial, int splits,
                               long long split_stride) {
   if (T == 0) return;
-  const long long warps = (long long)T * (Hq + 2 * Hkv);
-  // one head per eight lanes while that is what fills the chip, four of them once every SM still gets four dozen warps
-  // (1100 tokens of 48 heads: 9.0 us against 10.3 us; 26120 tokens: 147 us against 119 us)
-  if (D == 128 && slots != nullptr && partial == nullptr && warps >= 16ll * 148 * 48) {
-    const long long units = (long long)T * ((Hq + 2 * Hkv + 4 * ROPE_HEADS - 1) / (4 * ROPE_HEADS));
-    launch_pdl(PDL_ROPE, rope_qknorm_store_rows_kernel, dim3((unsigned)((units + 7) / 8)), dim3(256), 0, s, (const bf16*)qkv,
-               (const long long*)positions, (const float*)cos_sin, (const bf16*)q_w, (const bf16*)k_w, (bf16*)q_out,
-               (bf16*)k_cache, (bf16*)v_cache, (const int*)slots, T, Hq, Hkv, eps, num_slots, block_size, status);
+  const int heads = Hq + 2 * Hkv, sms = gemm_num_sms();
+  const long long warps = (long long)T * heads;
+  // One head per eight lanes while that is what fills the chip, four of them once every SM still gets four dozen warps, where a
+  // token's heads use at least three quarters of the lanes and no norm makes a lane's chain longer.  One -> four: 48 heads, 4096
+  // tokens 23.9 -> 18.9 us; 36 (of 48) heads, 8192 tokens 35.0 -> 33.6 us, but 18 (of 32) heads 14.4 -> 16.5 us; with norms
+  // 64 + 2 * 32 heads, 6000 tokens 68.0 -> 73.3 us, 36 heads, 8192 tokens 38.8 -> 50.4 us.
+  const int per_token = (heads + 4 * ROPE_HEADS - 1) / (4 * ROPE_HEADS);
+  if (D == 128 && slots != nullptr && partial == nullptr && q_w == nullptr && k_w == nullptr && warps >= 16ll * 48 * sms &&
+      4 * heads >= 3 * (4 * ROPE_HEADS) * per_token) {
+    const long long units = (long long)T * per_token;
+    launch_pdl(PDL_ROPE, rope_store_rows_kernel, dim3((unsigned)((units + 7) / 8)), dim3(256), 0, s, (const bf16*)qkv,
+               (const long long*)positions, (const float*)cos_sin, (bf16*)q_out, (bf16*)k_cache, (bf16*)v_cache, (const int*)slots, T,
+               Hq, Hkv, num_slots, block_size, status);
     return;
   }
   if (D == 128 && slots != nullptr) {
-    launch_pdl(PDL_ROPE, rope_qknorm_store_d128_kernel, dim3((unsigned)((warps + 31) / 32)), dim3(256), 0, s,
+    // EARLY for up to three blocks an SM (48 heads, 256 tokens: 3.3 -> 2.8 us; 36 heads, 512 tokens 3.4 -> 4.2 us, 1024 tokens of
+    // 48 heads 6.1 -> 7.1 us) and beside partial sums, whose loads are the longer wait
+    auto kern = partial != nullptr || warps <= 3ll * 32 * sms ? rope_qknorm_store_d128_kernel<true> : rope_qknorm_store_d128_kernel<false>;
+    launch_pdl(PDL_ROPE, kern, dim3((unsigned)((warps + 31) / 32)), dim3(256), 0, s,
                (const bf16*)qkv, (const long long*)positions, (const float*)cos_sin, (const bf16*)q_w,
                (const bf16*)k_w, (bf16*)q_out, (bf16*)k_cache, (bf16*)v_cache, (const int*)slots, T, Hq, Hkv, eps,
                num_slots, block_size, status, partial, splits, split_stride);

@@ -142,3 +142,28 @@ def test_rotary_store_of_many_rows_equals_that_of_few(Hq, Hkv, norm):
     few = [ops.rope_qknorm_store(qkv[a:a + 64], pos[a:a + 64], cs, Hq, Hkv, 128, qw, kw, 1e-6, pools[1][0], pools[1][1], slots[a:a + 64])
            for a in range(0, T, 64)]
     assert torch.equal(q, torch.cat(few)) and torch.equal(pools[0], pools[1])
+
+
+# tokens x heads per SM; several heads per group of lanes for many rows of well filled warps without norms only, loads ahead of
+# qkv for few rows only
+@pytest.mark.parametrize("Hq,Hkv,per_sm,norm,kernel", [(32, 8, 95, False, "d128_kernel<true>"), (32, 8, 97, False, "d128_kernel<false>"),
+                                                       (14, 2, 97, True, "d128_kernel<false>"), (32, 8, 770, False, "rows_kernel"),
+                                                       (32, 8, 770, True, "d128_kernel<false>"), (14, 2, 770, False, "d128_kernel<false>"),
+                                                       (16, 4, 770, False, "rows_kernel")])
+def test_rotary_store_by_rows_per_sm(Hq, Hkv, per_sm, norm, kernel):
+    heads, block = Hq + 2 * Hkv, 16
+    T = per_sm * torch.cuda.get_device_properties(0).multi_processor_count // heads
+    qkv, pos = _normal(T, heads * 128, seed=7).to(DEV), torch.randint(0, 500, (T,), generator=torch.Generator().manual_seed(8)).to(DEV)
+    cs = ref.build_cos_sin_cache(128, 512, 10000.0, DEV)
+    qw, kw = (_normal(128, seed=s).to(DEV) if norm else None for s in (10, 11))
+    slots = torch.randperm(T + 5, generator=torch.Generator().manual_seed(12))[:T].int()
+    slots[::17] = -1
+    slots = slots.to(DEV)
+    pools = [torch.zeros(2, -(-(T + 5) // block), Hkv, block, 128, dtype=torch.bfloat16, device=DEV) for _ in range(2)]
+    args = (qkv, pos, cs, Hq, Hkv, 128, qw, kw, 1e-6)
+    assert kernel in _kernel(lambda: ops.rope_qknorm_store(*args, pools[0][0], pools[0][1], slots), "rope_")
+    q, want = ops.rope_qknorm_store(*args, pools[0][0], pools[0][1], slots), ref.rope_qknorm_store(*args, pools[1][0], pools[1][1], slots)
+    # bf16 as in the statement: the norm's two roundings and the rotation's one may each fall the other way
+    for got, exp in ((q, want), (pools[0][0], pools[1][0])):
+        assert ((got.float() - exp.float()).abs() <= 3 * 2.0 ** -8 * exp.float().abs().amax(-1, keepdim=True) + 1e-6).all()
+    assert torch.equal(pools[0][1], pools[1][1])
