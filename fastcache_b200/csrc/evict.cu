@@ -20,7 +20,9 @@
 #include <stdexcept>
 #include <string>
 
+#include "gemm.h"
 #include "kernels.h"
+#include "launch.h"
 #include "ptx.cuh"
 
 namespace fc {
@@ -140,15 +142,17 @@ knorm_score_kernel(const bf16* __restrict__ pool, const int* __restrict__ block_
   }
 }
 
-// 1024 threads: the four passes are chains of shared-memory latencies, so a request of a few thousand rows wants few
-// rows per thread
-constexpr int SC_THREADS = 1024;
+// The four passes are chains of shared-memory latencies: long requests want few rows per thread (1024 threads) as long as all
+// CTAs run at once, everything else more CTAs on an SM (256 threads, see launch_select_compact).
+constexpr int SC_LONG = 2048;                    // rows
 
 // kept [n_seq, L, Hkv, s_stride]: the first n_kept entries of a row are the kept rows, ascending
+template <int SC_THREADS>
 __global__ void __launch_bounds__(SC_THREADS)
 select_rows_kernel(const float* __restrict__ scores, const int* __restrict__ kv_lens, const int* __restrict__ n_kepts,
                    int* __restrict__ kept, int L, int Hkv, int s_stride) {
   extern __shared__ uint32_t sm[];
+  pdl_launch_dependents();
   const int h = blockIdx.x, layer = blockIdx.y, seq = blockIdx.z;
   const int S = kv_lens[seq];
   int k = n_kepts[seq];
@@ -285,10 +289,11 @@ constexpr uint32_t MV_NONE = 0xffffffffu;
 
 template <int D>
 __global__ void __launch_bounds__(MV_THREADS)
-move_rows_kernel(bf16* __restrict__ pool, const int* __restrict__ kept, const int* __restrict__ block_tables,
+move_rows_kernel(bf16* __restrict__ pool, const int* kept, const int* __restrict__ block_tables,
                  const int* __restrict__ kv_lens, const int* __restrict__ n_kepts, int L, int num_blocks, int block_size,
                  int Hkv, int max_blocks, int s_stride, uint32_t* status) {
   constexpr int COLS = D / 64;
+  pdl_wait();
   const int part = blockIdx.x % (2 * COLS), h = blockIdx.x / (2 * COLS), layer = blockIdx.y, seq = blockIdx.z;
   const int S = kv_lens[seq];
   int k = n_kepts[seq];
@@ -307,16 +312,20 @@ move_rows_kernel(bf16* __restrict__ pool, const int* __restrict__ kept, const in
     }
     return (uint32_t(blk) * Hkv + h) * block_size + tok % block_size;
   };
-  for (int c0 = 0; c0 < k; c0 += MV_CHUNK) {
-    uint32_t src = MV_NONE, dst = MV_NONE;
+  auto look_up = [&](int c0, uint32_t& src, uint32_t& dst) {
+    src = dst = MV_NONE;
     const int j = c0 + grp * MV_ROWS + lane;
     if (j < k) {
-      const int r = rows[j];
+      const int r = __ldcg(rows + j);            // written by the kernel before this one: not through the read-only path
       if (r != j) {                              // a row that stays is neither read nor written
         src = number(r);
         dst = number(j);
       }
     }
+  };
+  uint32_t src, dst, next_src, next_dst;
+  look_up(0, src, dst);
+  for (int c0 = 0; c0 < k; c0 += MV_CHUNK, src = next_src, dst = next_dst) {
     uint4 v[MV_ROWS];
 #pragma unroll
     for (int u = 0; u < MV_ROWS; ++u) {
@@ -324,6 +333,7 @@ move_rows_kernel(bf16* __restrict__ pool, const int* __restrict__ kept, const in
       v[u] = make_uint4(0, 0, 0, 0);
       if (from != MV_NONE) v[u] = *reinterpret_cast<const uint4*>(base + (long long)from * D);
     }
+    look_up(c0 + MV_CHUNK, next_src, next_dst);  // two look-ups in a row, while this chunk's rows arrive
     // every row of this chunk has been read (and of the chunks before) when the first one is written; rows only move
     // towards the front, so what is written here lies before the rows of every later chunk
     __syncthreads();
@@ -350,16 +360,20 @@ void launch_select_compact(void* pool, const float* scores, const int* block_tab
                            const int* n_kepts, int* kept, int n_seq, int L, int num_blocks, int block_size, int Hkv, int D,
                            int max_blocks, int s_stride, uint32_t* status, cudaStream_t stream) {
   if (n_seq == 0) return;
-  const int smem = (s_stride + 256 + 8 + SC_THREADS / 32) * 4;
+  const int smem = (s_stride + 256 + 8 + 1024 / 32) * 4;
   if (smem > 220 * 1024) throw std::runtime_error("select_compact: request too long for one CTA's shared memory");
   if (D != 64 && D != 128) throw std::runtime_error("select_compact: head_dim must be 64 or 128");
   if ((long long)num_blocks * Hkv * block_size >= (long long)MV_NONE)
     throw std::runtime_error("select_compact: too many rows in one plane of the pool");
-  cudaFuncSetAttribute(select_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  select_rows_kernel<<<dim3(Hkv, L, n_seq), SC_THREADS, smem, stream>>>(scores, kv_lens, n_kepts, kept, L, Hkv, s_stride);
+  // 1024 -> 256 threads: 32 layers x 8 heads, 4 requests of 100 rows 38.8 -> 16.2 us (the moves included), of 800 rows 81 -> 60
+  // us; 4 layers, 8 requests of 3000 rows 55 us both; 8 layers, 2 requests of 6000 rows 65 -> 72 us
+  const bool wide = s_stride > SC_LONG && (long long)Hkv * L * n_seq <= 2ll * gemm_num_sms();
+  auto select = wide ? select_rows_kernel<1024> : select_rows_kernel<256>;
+  cudaFuncSetAttribute(select, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  select<<<dim3(Hkv, L, n_seq), wide ? 1024 : 256, smem, stream>>>(scores, kv_lens, n_kepts, kept, L, Hkv, s_stride);
   auto move = D == 128 ? move_rows_kernel<128> : move_rows_kernel<64>;
-  move<<<dim3(Hkv * 2 * (D / 64), L, n_seq), MV_THREADS, 0, stream>>>((bf16*)pool, kept, block_tables, kv_lens, n_kepts, L,
-                                                                      num_blocks, block_size, Hkv, max_blocks, s_stride, status);
+  launch_pdl(PDL_EVICT, move, dim3(Hkv * 2 * (D / 64), L, n_seq), dim3(MV_THREADS), 0, stream, (bf16*)pool, (const int*)kept,
+             block_tables, kv_lens, n_kepts, L, num_blocks, block_size, Hkv, max_blocks, s_stride, status);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) throw std::runtime_error(std::string("select_compact launch: ") + cudaGetErrorString(e));
 }

@@ -26,6 +26,7 @@ enum PdlFamily : unsigned {
   PDL_DECODE_ATTN = 1u << 7,
   PDL_DECODE_MERGE = 1u << 8,
   PDL_ALLREDUCE = 1u << 9,
+  PDL_EVICT = 1u << 10,
 };
 
 inline unsigned pdl_mask() {
