@@ -24,6 +24,7 @@
 #include <stdexcept>
 #include <string>
 
+#include "gemm.h"
 #include "kernels.h"
 #include "ptx.cuh"
 
@@ -187,7 +188,9 @@ __device__ __forceinline__ void encode_exact(uint32_t which, const uint4& raw, f
 // groups sit side by side in a warp and QU such batches are in flight per iteration.  Two pieces per lane halve what a
 // group costs besides its values (the shuffles of the reduction, the scale and its reciprocal); only groups of up to 32
 // values have one.
-constexpr int quant_batches(int ch) { return ch > 2 ? 2 : 4; }
+// FEW groups (see launch_quantize_m): one piece per lane and one batch per warp, so that as many warps as there are share the
+// work; FP8 divides there, which is a shorter chain than both ends of the interval.
+constexpr int quant_batches(int ch, bool few) { return few ? 1 : ch > 2 ? 2 : 4; }
 
 template <int W>
 __device__ __forceinline__ float sub_max(float v) {
@@ -223,7 +226,7 @@ __device__ __forceinline__ int nf4_code_fast(float t, const float* s_mid) {
 // x [groups, g] bf16 (rows of D values cut into D / g groups).  FAKE: y = decode(encode(x)) in bf16, no codes.
 // Otherwise: codes as bytes (INT8, FP8: one per value; INT4 / NF4: one per two values), `scale` [groups] (the
 // scale, or the absmax for the 4-bit modes) and, for the asymmetric mode, `zero` [groups].
-template <int MODE, bool FAKE, int W, int CH>
+template <int MODE, bool FAKE, int W, int CH, bool FEW>
 __global__ void __launch_bounds__(256)
 quantize_kernel(const bf16* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ scale,
                 float* __restrict__ zero, bf16* __restrict__ y, long long groups, int g) {
@@ -241,7 +244,7 @@ quantize_kernel(const bf16* __restrict__ x, uint8_t* __restrict__ q, float* __re
   const int lane = threadIdx.x & 31;
   const int sub = lane / W, l = lane % W;
   constexpr int GPW = 32 / W;                                    // groups per warp and batch
-  constexpr int QU = quant_batches(CH);
+  constexpr int QU = quant_batches(CH, FEW);
   const long long warp = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
   const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
   const int chunks = g >> 3;
@@ -297,8 +300,16 @@ quantize_kernel(const bf16* __restrict__ x, uint8_t* __restrict__ q, float* __re
       for (int c = 0; c < CH; ++c) {
         if (l + W * c >= chunks) continue;
         uint2 w;                                                 // eight codes, one byte each
-        const uint32_t unsure = encode8_fast<MODE>(raw[u][c], r, z, s_mid, w);
-        encode_exact<MODE>(a < 0x1p125f ? unsure : 0xFFu, raw[u][c], a, z, s_mid, w);
+        if constexpr (FEW && (MODE == QUANT_FP8_E4M3 || MODE == QUANT_FP8_E5M2)) {
+          float v[8];
+          unpack8(raw[u][c], v);
+          w = make_uint2(0, 0);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) (i < 4 ? w.x : w.y) |= uint32_t(encode<MODE>(v[i], a, z) & 0xFF) << (8 * (i & 3));
+        } else {
+          const uint32_t unsure = encode8_fast<MODE>(raw[u][c], r, z, s_mid, w);
+          encode_exact<MODE>(a < 0x1p125f ? unsure : 0xFFu, raw[u][c], a, z, s_mid, w);
+        }
         if (FAKE) {
           float out[8];
 #pragma unroll
@@ -363,22 +374,40 @@ static int quant_grid(long long work_items, int per_block) {
   return int(blocks < 1 ? 1 : (blocks > 148 * 16 ? 148 * 16 : blocks));
 }
 
-template <int MODE, int W, int CH>
+// Groups that the form for many would spread over at most QUANT_FEW_BLOCKS blocks an SM go one piece per lane instead.  INT8,
+// many -> few, groups of 64: 1000 4.5 -> 2.6 us, 60000 6.1 -> 5.1 us; of 128: 1000 4.2 -> 2.2 us, 60000 (just under the line)
+// 8.6 -> 7.8 us, 100000 11.1 -> 11.5 us; FP8 of 128: 60000 10.4 -> 8.4 us.
+constexpr int QUANT_FEW_BLOCKS = 4;
+constexpr long long quant_groups_per_block(int w, int ch, bool few) { return 8 * (32 / w) * quant_batches(ch, few); }
+
+template <int MODE, int W, int CH, bool FEW = false>
 static void launch_quantize_w(const bf16* x, uint8_t* q, float* scale, float* zero, bf16* y, long long groups, int g,
                               cudaStream_t s) {
-  const int grid = quant_grid(groups, 8 * (32 / W) * quant_batches(CH));          // groups per block and iteration
-  if (y != nullptr) quantize_kernel<MODE, true, W, CH><<<grid, 256, 0, s>>>(x, q, scale, zero, y, groups, g);
-  else quantize_kernel<MODE, false, W, CH><<<grid, 256, 0, s>>>(x, q, scale, zero, y, groups, g);
+  const int grid = quant_grid(groups, int(quant_groups_per_block(W, CH, FEW)));
+  if (y != nullptr) quantize_kernel<MODE, true, W, CH, FEW><<<grid, 256, 0, s>>>(x, q, scale, zero, y, groups, g);
+  else quantize_kernel<MODE, false, W, CH, FEW><<<grid, 256, 0, s>>>(x, q, scale, zero, y, groups, g);
 }
 template <int MODE>
 static void launch_quantize_m(const bf16* x, uint8_t* q, float* scale, float* zero, bf16* y, long long groups, int g,
                               cudaStream_t s) {
   const int chunks = g >> 3;
-  if (chunks <= 4) launch_quantize_w<MODE, 4, 1>(x, q, scale, zero, y, groups, g, s);
-  else if (chunks <= 8) launch_quantize_w<MODE, 4, 2>(x, q, scale, zero, y, groups, g, s);
-  else if (chunks <= 16) launch_quantize_w<MODE, 8, 2>(x, q, scale, zero, y, groups, g, s);
-  else if (chunks <= 32) launch_quantize_w<MODE, 16, 2>(x, q, scale, zero, y, groups, g, s);
-  else launch_quantize_w<MODE, 32, QMAX_CHUNKS>(x, q, scale, zero, y, groups, g, s);
+  const long long line = (long long)QUANT_FEW_BLOCKS * gemm_num_sms();
+  auto few = [&](int w, int ch) { return groups <= line * quant_groups_per_block(w, ch, false); };
+  if (chunks <= 4) {
+    if (few(4, 1)) launch_quantize_w<MODE, 4, 1, true>(x, q, scale, zero, y, groups, g, s);
+    else launch_quantize_w<MODE, 4, 1>(x, q, scale, zero, y, groups, g, s);
+  } else if (chunks <= 8) {
+    if (few(4, 2)) launch_quantize_w<MODE, 8, 1, true>(x, q, scale, zero, y, groups, g, s);
+    else launch_quantize_w<MODE, 4, 2>(x, q, scale, zero, y, groups, g, s);
+  } else if (chunks <= 16) {
+    if (few(8, 2)) launch_quantize_w<MODE, 16, 1, true>(x, q, scale, zero, y, groups, g, s);
+    else launch_quantize_w<MODE, 8, 2>(x, q, scale, zero, y, groups, g, s);
+  } else if (chunks <= 32) {
+    if (few(16, 2)) launch_quantize_w<MODE, 32, 1, true>(x, q, scale, zero, y, groups, g, s);
+    else launch_quantize_w<MODE, 16, 2>(x, q, scale, zero, y, groups, g, s);
+  } else {
+    launch_quantize_w<MODE, 32, QMAX_CHUNKS>(x, q, scale, zero, y, groups, g, s);
+  }
 }
 
 void launch_quantize(const void* x, void* q, float* scale, float* zero, void* y_fake, long long groups, int g,
