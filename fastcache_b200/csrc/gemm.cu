@@ -48,6 +48,7 @@ namespace fc {
 constexpr int BM = 128;
 constexpr int BK = 64;
 constexpr int STAGED_K = 2048;                    // see above
+constexpr int STAGED_DIVIDES_K = 1280;            // see launch_one
 
 struct GemmParams {
   int M, N, K;
@@ -561,11 +562,17 @@ static void launch_form(const CUtensorMap& ta, const CUtensorMap& tb, const CUte
 }
 
 // The staged epilogue for a short main loop and an output that TMA can describe; grouped rows (a tile may end inside
-// another group's rows) and the fp32 forms have the other one only.
+// another group's rows) and the fp32 forms have the other one only.  SwiGLU, its clamped form and xIELU spend their epilogue on
+// chains of divisions, which the plain form starts storing under: they gain only where a CTA has several tiles whose main loops
+// are shorter than that.  SwiGLU, plain -> staged, 300 and 961 rows of 2 x 4096 at K = 1024: 16.1 -> 21.1 us, 25.0 -> 27.1 us
+// (one tile, two); 2000 rows (four): 42.2 -> 39.5 us, at K = 1280 44.2 -> 45.0 us; 4616 rows at K = 1024 78.1 -> 64.3 us, at
+// K = 1792 100.6 -> 104.2 us.
 template <int BN, int STAGES, int GLU = GLU_NONE, int FORM = GF_PLAIN>
 static void launch_one(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int grid, cudaStream_t stream) {
   if constexpr (FORM == GF_PLAIN || FORM == GF_XIELU) {
-    if (p.K <= STAGED_K && p.ldc % 8 == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0) {
+    constexpr bool DIVIDES = GLU == GLU_SILU || GLU == GLU_CLAMPED || FORM == GF_XIELU;
+    const bool gains = DIVIDES ? p.K < STAGED_DIVIDES_K && p.total_work > 3ll * grid : p.K <= STAGED_K;
+    if (gains && p.ldc % 8 == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0) {
       const CUtensorMap tc = make_tmap_bf16_2d(p.C, p.M, p.N, p.ldc, BM, SLAB);
       launch_form<BN, STAGES, GLU, FORM, true>(ta, tb, tc, ta, p, grid, stream);
       return;

@@ -49,7 +49,7 @@ constexpr int P2_BN = 256;
 constexpr int P2_BK = 64;
 constexpr int P2_STAGES = 6;
 constexpr long long PAIRS_MIN = 2 * 1024, PAIRS_MAX = 64 * 1024;      // waves x K, see gemm_pairs_faster
-constexpr int PAIRS_ACT_K = 1280;
+constexpr int PAIRS_ACT_K = 1280, PAIRS_GATED_WAVES = 8;
 constexpr int P2_THREADS = 320;
 constexpr int P2_A_BYTES = P2_BM * P2_BK * 2;
 constexpr int P2_B_BYTES = P2_BNH * P2_BK * 2;
@@ -389,7 +389,9 @@ void set_gemm_pairs(int mode) { g_pairs = mode == PAIRS_NEVER || mode == PAIRS_F
 //    either way (577 x 4096 at K = 2048 18.3 -> 18.6 us, sums with a residual a little faster); 1154 rows of CLIP: qkv 13.5 -> 14.4 us; 961 of SigLIP: qkv 14.2 -> 14.9 us, but fc2 (K = 4304) 34.5 -> 29.7 us.
 //  - an activation that takes an exponential or an error function below K = PAIRS_ACT_K, where the epilogue of every tile is
 //    longer than its main loop: CLIP's fc1 (quick GELU, K = 1024) 65.3 -> 68.5 us with 15 images, 29.5 -> 31.6 us with five;
-//    2000 x 8192 with quick GELU or SwiGLU at K = 1024: 3 and 2 % slower in pairs, at K = 1280: 4 % faster.
+//    2000 x 8192 with quick GELU at K = 1024: 3 % slower in pairs, at K = 1280: 4 % faster.
+//  - SwiGLU in fewer than PAIRS_GATED_WAVES waves, against the plain epilogue of gemm.cu: 2000 rows of 2 x 4096 (four waves)
+//    54.5 -> 58.6 us at K = 2048, 3000 rows (six) 63.4 -> 65.5 us at K = 1536; 6000 rows (eleven) 149.0 -> 142.7 us.
 // Products of more than PAIRS_MAX (waves x K) run at the power limit, where both take the same time, and gemm_bf16 asks for
 // pairs up to K = 2048 only (what it measured at K = 4096: gemm.cu).
 bool gemm_pairs_faster(int M, int N, int K, int act, int sms) {
@@ -397,6 +399,7 @@ bool gemm_pairs_faster(int M, int N, int K, int act, int sms) {
   auto up = [](long long a, long long b) { return (a + b - 1) / b; };
   const long long n = up(N, 256), one = up(up(M, 128) * n, sms), two = up(up(M, 256) * n, sms / 2);
   if (K < PAIRS_ACT_K && (act == ACT_GELU || act == ACT_QUICK_GELU || act == ACT_SILU || act == ACT_SWIGLU)) return false;
+  if (act == ACT_SWIGLU && one < PAIRS_GATED_WAVES) return false;
   return one * K >= PAIRS_MIN && one * K <= PAIRS_MAX && two <= one;
 }
 

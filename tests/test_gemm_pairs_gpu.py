@@ -82,6 +82,18 @@ def test_the_switch_says_which_kernel_runs(forms, mode, M, N, K, faster):
         assert ("2cta" in name) == (mode == 1 or (mode == 2 and form in faster)), name
 
 
+# SwiGLU: few tiles per CTA and long main loops on the plain epilogue, several short ones on the staged one, many waves on pairs
+@pytest.mark.parametrize("M,I,K,kernel", [(961, 4096, 1024, "plain"), (2000, 4096, 1024, "staged"), (2000, 4096, 2048, "plain"),
+                                          (4616, 4096, 1024, "staged"), (6000, 4096, 2048, "pairs"), (6000, 4096, 4096, "plain")])
+def test_swiglu_by_waves_and_length(forms, M, I, K, kernel):
+    forms.set_gemm_pairs(2)
+    x, w = _rand(M, K, seed=8), _rand(2 * I, K, scale=0.05, seed=9)
+    name, = _kernels(lambda: ops.linear(x, w, None, act="swiglu"))
+    assert {"pairs": "2cta", "staged": "true>", "plain": "false>"}[kernel] in name.replace("(bool)1", "true").replace("(bool)0", "false"), name
+    want = ref.silu_and_mul(ref.linear(x.float(), w.float()).to(torch.bfloat16).float())
+    assert ((ops.linear(x, w, None, act="swiglu").float() - want).abs() / (want.abs() + 1.0)).max().item() < 3e-2
+
+
 def test_cta_pairs_on_a_side_stream_and_repeated(forms):
     e = forms
     e.set_gemm_pairs(1)

@@ -60,7 +60,7 @@ def test_staged_epilogue_of_many_tiles(pairs, M, N, K):
     _clean()
 
 
-@pytest.mark.parametrize("M,I,K", [(257, 128, 64), (1000, 384, 1024), (4616, 1024, 1024), (300, 640, 2056)])
+@pytest.mark.parametrize("M,I,K", [(257, 128, 64), (1000, 384, 1024), (4616, 1024, 1024), (8655, 1024, 1024), (9001, 1152, 64), (300, 640, 2056)])
 def test_gated_staged_epilogue(pairs, M, I, K):
     x, w = _normal(M, K, seed=1), _normal(2 * I, K, seed=2, scale=K ** -0.5)
     gate, up = (x.double() @ w.double().T).split(I, dim=1)
