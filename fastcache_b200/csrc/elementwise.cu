@@ -640,9 +640,10 @@ void launch_layer_norm(const void* x, const void* w, const void* b, void* y, lon
   if (T == 0) return;
   const int chunks = H >> 3;
   // A block per row -> a warp per row: 577 rows of 1024, 2048: 3.3 -> 3.5 us, 4.0 -> 5.1 us; 800 rows: 4.7 -> 3.4 us, 5.5 ->
-  // 5.0 us, so the line is at four rows an SM; 64 rows of 512 2.7 us both, of 2048 2.9 -> 4.8 us.  Rows of 3584 never gain: 64
-  // rows 3.3 -> 6.9 us, 4805 rows 23.0 -> 23.4 us, 8655 rows 41.9 -> 50.3 us; of 2560 by 3 % from 8000 rows on.
-  if (chunks > 8 * 32 || (chunks > 2 * 32 && T <= 4ll * gemm_num_sms())) {
+  // 5.0 us: the line is where the blocks (five an SM) need a second wave.  64 rows of 512 2.7 us both, of 2048 2.9 -> 4.8 us.
+  // Rows of 3584 never gain: 64 rows 3.3 -> 6.9 us, 4805 rows 23.0 -> 23.4 us, 8655 rows 41.9 -> 50.3 us; of 2560 by 3 % from
+  // 8000 rows on.
+  if (chunks > 8 * 32 || (chunks > 2 * 32 && T <= 5ll * gemm_num_sms())) {
     layer_norm_block_kernel<<<(unsigned)T, NORM_THREADS, 0, s>>>((const bf16*)x, (const bf16*)w, (const bf16*)b, (bf16*)y, H, eps);
     return;
   }

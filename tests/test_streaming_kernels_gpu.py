@@ -19,6 +19,14 @@ def _status():
     return ops.ext().status_tensor(torch.cuda.current_device())
 
 
+def _kernel(f, part):
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        f()
+        torch.cuda.synchronize()
+    name, = [e.key.replace(" ", "") for e in prof.key_averages() if part in e.key]
+    return name
+
+
 @pytest.mark.parametrize("mode", ["int8", "int8_asym", "int4", "nf4", "fp8_e4m3", "fp8_e5m2"])
 @pytest.mark.parametrize("g", [8, 24, 64, 128, 256, 264, 1024])
 def test_codes_equal_the_division_where_the_quotient_is_near_a_border(mode, g):
@@ -37,6 +45,21 @@ def test_codes_equal_the_division_where_the_quotient_is_near_a_border(mode, g):
     assert torch.equal(got["scale"].cpu(), want["scale"])
     assert torch.equal(got["q"].cpu().view(torch.uint8), want["q"].view(torch.uint8))
     assert torch.equal(quant.dequantize(got).cpu(), quant.dequantize(want))
+
+
+# groups per block of the form for many (which takes more than four blocks an SM), and lanes and pieces per lane of both forms
+@pytest.mark.parametrize("mode", ["int8", "int8_asym", "int4", "nf4", "fp8_e4m3", "fp8_e5m2"])
+@pytest.mark.parametrize("g,per_block,many,few", [(8, 256, "4,1", "4,1"), (40, 256, "4,2", "8,1"), (64, 256, "4,2", "8,1"), (72, 128, "8,2", "16,1"),
+                                                  (128, 128, "8,2", "16,1"), (136, 64, "16,2", "32,1"), (256, 64, "16,2", "32,1")])
+def test_many_groups_and_few_give_the_same_codes(mode, g, per_block, many, few):
+    n = 4 * torch.cuda.get_device_properties(0).multi_processor_count * per_block + 3
+    x = _normal(n, g, seed=g).to(DEV)
+    got = {}
+    assert f",{many},false>" in _kernel(lambda: got.update(quant.quantize(x, mode, g)), "quantize_kernel")
+    assert f",{few},true>" in _kernel(lambda: quant.quantize(x[3:], mode, g), "quantize_kernel")
+    parts = [quant.quantize(x[a:a + n // 2], mode, g) for a in range(0, n, n // 2)]
+    for k in ("q", "scale") + (("zero",) if mode == "int8_asym" else ()):
+        assert torch.equal(got[k].view(torch.uint8), torch.cat([p[k] for p in parts]).view(torch.uint8))
 
 
 @pytest.mark.parametrize("D,Hkv,block", [(128, 8, 256), (128, 3, 16), (64, 2, 64)])
@@ -101,17 +124,9 @@ def test_layer_norm_row_lengths(T, H):
     assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4).all()
 
 
-def _kernel(f, part):
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
-        f()
-        torch.cuda.synchronize()
-    name, = [e.key.replace(" ", "") for e in prof.key_averages() if part in e.key]
-    return name
-
-
-# a warp per row where there are more than four rows an SM, a block per row for fewer and for long rows
-@pytest.mark.parametrize("rows,H,kernel", [(4, 512, "<4>"), (4, 520, "block"), (4, 1280, "block"), (5, 520, "<4>"), (5, 1032, "<5>"), (5, 1288, "<8>"),
-                                           (5, 2048, "<8>"), (5, 2056, "block"), (5, 3584, "block")])
+# a warp per row where there are more than five rows an SM, a block per row for fewer and for long rows
+@pytest.mark.parametrize("rows,H,kernel", [(5, 512, "<4>"), (5, 520, "block"), (5, 1280, "block"), (6, 520, "<4>"), (6, 1032, "<5>"), (6, 1288, "<8>"),
+                                           (6, 2048, "<8>"), (6, 2056, "block"), (6, 3584, "block")])
 def test_layer_norm_by_rows_per_sm(rows, H, kernel):
     T = rows * torch.cuda.get_device_properties(0).multi_processor_count
     x, w, b = (_normal(*s, seed=i) for i, s in enumerate([(T, H), (H,), (H,)]))
@@ -154,7 +169,8 @@ def test_rotary_store_by_rows_per_sm(Hq, Hkv, per_sm, norm, kernel):
     heads, block = Hq + 2 * Hkv, 16
     T = per_sm * torch.cuda.get_device_properties(0).multi_processor_count // heads
     qkv, pos = _normal(T, heads * 128, seed=7).to(DEV), torch.randint(0, 500, (T,), generator=torch.Generator().manual_seed(8)).to(DEV)
-    cs = ref.build_cos_sin_cache(128, 512, 10000.0, DEV)
+    angle = torch.rand(500, 64, generator=torch.Generator().manual_seed(9)) * 6
+    cs = torch.cat([angle.cos(), angle.sin()], 1).to(DEV)
     qw, kw = (_normal(128, seed=s).to(DEV) if norm else None for s in (10, 11))
     slots = torch.randperm(T + 5, generator=torch.Generator().manual_seed(12))[:T].int()
     slots[::17] = -1
@@ -162,8 +178,6 @@ def test_rotary_store_by_rows_per_sm(Hq, Hkv, per_sm, norm, kernel):
     pools = [torch.zeros(2, -(-(T + 5) // block), Hkv, block, 128, dtype=torch.bfloat16, device=DEV) for _ in range(2)]
     args = (qkv, pos, cs, Hq, Hkv, 128, qw, kw, 1e-6)
     assert kernel in _kernel(lambda: ops.rope_qknorm_store(*args, pools[0][0], pools[0][1], slots), "rope_")
-    q, want = ops.rope_qknorm_store(*args, pools[0][0], pools[0][1], slots), ref.rope_qknorm_store(*args, pools[1][0], pools[1][1], slots)
-    # bf16 as in the statement: the norm's two roundings and the rotation's one may each fall the other way
-    for got, exp in ((q, want), (pools[0][0], pools[1][0])):
-        assert ((got.float() - exp.float()).abs() <= 3 * 2.0 ** -8 * exp.float().abs().amax(-1, keepdim=True) + 1e-6).all()
-    assert torch.equal(pools[0][1], pools[1][1])
+    q = ops.rope_qknorm_store(*args, pools[0][0], pools[0][1], slots)
+    few = [ops.rope_qknorm_store(qkv[a:a + 32], pos[a:a + 32], *args[2:], pools[1][0], pools[1][1], slots[a:a + 32]) for a in range(0, T, 32)]
+    assert torch.equal(q, torch.cat(few)) and torch.equal(pools[0], pools[1])
