@@ -1,4 +1,9 @@
 """Shared builders for the test-suite: tiny seeded models and compressors."""
+import ctypes
+import os
+import re
+import tempfile
+
 import torch
 
 from fastcache_b200.config import ModelConfig
@@ -23,3 +28,29 @@ def random_compressor(cls, n_layer, head_dim, factor, seed=0, **kw):
     for p in m.parameters():
         torch.nn.init.normal_(p, std=0.05)
     return m.eval()
+
+
+def _demangled(name):
+    lib = ctypes.CDLL("libstdc++.so.6")
+    lib.__cxa_demangle.restype = ctypes.c_char_p
+    status = ctypes.c_int()
+    plain = lib.__cxa_demangle(name.encode(), None, None, ctypes.byref(status))
+    return plain.decode() if status.value == 0 else name
+
+
+def launched(f, *parts):
+    """Names (demangled, without blanks) of the kernels that f() launches and that hold one of `parts`, read from a capture."""
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.stream(stream):
+        f()
+        stream.synchronize()
+        with torch.cuda.graph(graph, stream=stream):
+            f()
+    with tempfile.TemporaryDirectory() as folder:
+        path = os.path.join(folder, "graph.dot")
+        assert ctypes.CDLL("libcuda.so.1").cuGraphDebugDotPrint(ctypes.c_void_p(graph.raw_cuda_graph()), path.encode(), 1) == 0
+        with open(path) as dot:
+            names = {_demangled(n).replace(" ", "") for n in re.findall(r"_ZN?[A-Za-z0-9_]+", dot.read())}
+    return sorted(n for n in names if any(p in n for p in parts))

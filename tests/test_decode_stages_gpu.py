@@ -4,6 +4,7 @@ import pytest
 import torch
 
 from fastcache_b200 import ops
+from helpers import launched
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -55,16 +56,13 @@ def test_both_rings(merge, D, B, Hq, Hkv, bs, splits, stages):
     def call():
         return ops.decode_attention(q, kc, vc, table, ctx, D ** -0.5, {"splits": splits})
 
-    first = call()
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
-        got = call()
-        torch.cuda.synchronize()
-    names = [e.key.replace(" ", "") for e in prof.key_averages() if "decode_attn_kernel" in e.key]
-    assert len(names) == 1 and f"<{D},{stages}>" in names[0], names
+    first, got = call(), call()
     assert torch.equal(got, first) and ops.ext().read_status(torch.cuda.current_device()) == 0
     want = _statement(q, kc, vc, table, lens, D ** -0.5)
     # weights and result are rounded to bf16 once each: 2^-9 of the largest value, and of the result
     assert ((got.double() - want).abs() <= 2.0 ** -9 * (vc.float().abs().max() + want.abs()) * 1.01 + 1e-5).all()
+    name, = launched(call, "decode_attn_kernel")
+    assert f"<{D},{stages}>" in name, name
 
 
 @pytest.mark.parametrize("B,Hkv,bound,splits", [(32, 8, 2048, 1), (32, 8, 2304, 2), (28, 8, 4096, 2), (37, 8, 4096, 1), (27, 8, 1024, 2), (32, 8, 256, 1)])
@@ -77,12 +75,8 @@ def test_splits_of_batches_that_leave_sms_with_one_cta(B, Hkv, bound, splits):
     kc, vc, q = _normal(40, Hkv, bs, 128, seed=1), _normal(40, Hkv, bs, 128, seed=2), _normal(B, 4 * Hkv, 128, seed=4)
     lens = [bound if i == 3 else 1 + 7 * i for i in range(B)]
     ctx = torch.tensor(lens, dtype=torch.int32, device=DEV)
-    ops.decode_attention(q, kc, vc, table, ctx, 0.1)
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
-        got = ops.decode_attention(q, kc, vc, table, ctx, 0.1)
-        torch.cuda.synchronize()
-    names = [e.key for e in prof.key_averages()]
-    assert any("decode_attn_kernel" in n for n in names)
-    assert any("decode_merge_kernel" in n for n in names) == (splits > 1)
+    got = ops.decode_attention(q, kc, vc, table, ctx, 0.1)
     want = _statement(q, kc, vc, table, lens, 0.1)
     assert ((got.double() - want).abs() <= 2.0 ** -9 * (vc.float().abs().max() + want.abs()) * 1.01 + 1e-5).all()
+    names = launched(lambda: ops.decode_attention(q, kc, vc, table, ctx, 0.1), "decode_attn_kernel", "decode_merge_kernel")
+    assert any("attn" in n for n in names) and any("merge" in n for n in names) == (splits > 1), names

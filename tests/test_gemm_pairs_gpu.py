@@ -4,6 +4,7 @@ import pytest
 import torch
 
 from fastcache_b200 import ops
+from helpers import launched
 from fastcache_b200.ops import reference as ref
 
 pytestmark = pytest.mark.gpu
@@ -59,14 +60,6 @@ def test_swiglu_on_cta_pairs(forms, M, I, K):
         assert ((y.float() - want).abs() / (want.abs() + 1.0)).max().item() < 3e-2
 
 
-def _kernels(f):
-    f()
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
-        f()
-        torch.cuda.synchronize()
-    return [e.key for e in prof.key_averages() if "gemm_bf16" in e.key]
-
-
 @pytest.mark.parametrize("mode", [0, 1, 2])
 # M, N, K: a short product that needs no more waves of pairs, one whose gated epilogue outlasts its main loop, one of a single
 # short wave, one that needs another wave, one at the power limit, all on 148 SMs
@@ -78,7 +71,7 @@ def test_the_switch_says_which_kernel_runs(forms, mode, M, N, K, faster):
     x, w, b, r = _rand(M, K), _rand(N, K), _rand(N), _rand(M, N)
     for form, product in {"p": lambda: ops.linear(x, w, b), "a": lambda: ops.linear(x, w, None, "gelu_tanh"),
                           "g": lambda: ops.linear(x, w, None, "swiglu"), "r": lambda: ops.linear_add(x, w, b, r)}.items():
-        name, = _kernels(product)
+        name, = launched(product, "gemm_bf16")
         assert ("2cta" in name) == (mode == 1 or (mode == 2 and form in faster)), name
 
 
@@ -88,10 +81,10 @@ def test_the_switch_says_which_kernel_runs(forms, mode, M, N, K, faster):
 def test_swiglu_by_waves_and_length(forms, M, I, K, kernel):
     forms.set_gemm_pairs(2)
     x, w = _rand(M, K, seed=8), _rand(2 * I, K, scale=0.05, seed=9)
-    name, = _kernels(lambda: ops.linear(x, w, None, act="swiglu"))
-    assert {"pairs": "2cta", "staged": "true>", "plain": "false>"}[kernel] in name.replace("(bool)1", "true").replace("(bool)0", "false"), name
     want = ref.silu_and_mul(ref.linear(x.float(), w.float()).to(torch.bfloat16).float())
     assert ((ops.linear(x, w, None, act="swiglu").float() - want).abs() / (want.abs() + 1.0)).max().item() < 3e-2
+    name, = launched(lambda: ops.linear(x, w, None, act="swiglu"), "gemm_bf16")
+    assert {"pairs": "2cta", "staged": "true>", "plain": "false>"}[kernel] in name, name
 
 
 def test_cta_pairs_on_a_side_stream_and_repeated(forms):

@@ -6,6 +6,7 @@ import torch
 from fastcache_b200 import ops
 from fastcache_b200.compress import quant
 from fastcache_b200.ops import reference as ref
+from helpers import launched
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -17,14 +18,6 @@ def _normal(*shape, seed=0, scale=1.0):
 
 def _status():
     return ops.ext().status_tensor(torch.cuda.current_device())
-
-
-def _kernel(f, part):
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
-        f()
-        torch.cuda.synchronize()
-    name, = [e.key.replace(" ", "") for e in prof.key_averages() if part in e.key]
-    return name
 
 
 @pytest.mark.parametrize("mode", ["int8", "int8_asym", "int4", "nf4", "fp8_e4m3", "fp8_e5m2"])
@@ -54,12 +47,13 @@ def test_codes_equal_the_division_where_the_quotient_is_near_a_border(mode, g):
 def test_many_groups_and_few_give_the_same_codes(mode, g, per_block, many, few):
     n = 4 * torch.cuda.get_device_properties(0).multi_processor_count * per_block + 3
     x = _normal(n, g, seed=g).to(DEV)
-    got = {}
-    assert f",{many},false>" in _kernel(lambda: got.update(quant.quantize(x, mode, g)), "quantize_kernel")
-    assert f",{few},true>" in _kernel(lambda: quant.quantize(x[3:], mode, g), "quantize_kernel")
+    got = quant.quantize(x, mode, g)
     parts = [quant.quantize(x[a:a + n // 2], mode, g) for a in range(0, n, n // 2)]
     for k in ("q", "scale") + (("zero",) if mode == "int8_asym" else ()):
         assert torch.equal(got[k].view(torch.uint8), torch.cat([p[k] for p in parts]).view(torch.uint8))
+    for rows, form in ((x, f",{many},false>"), (x[3:], f",{few},true>")):
+        name, = launched(lambda: quant.quantize(rows, mode, g), "quantize_kernel")
+        assert form in name, name
 
 
 @pytest.mark.parametrize("D,Hkv,block", [(128, 8, 256), (128, 3, 16), (64, 2, 64)])
@@ -131,10 +125,11 @@ def test_layer_norm_by_rows_per_sm(rows, H, kernel):
     T = rows * torch.cuda.get_device_properties(0).multi_processor_count
     x, w, b = (_normal(*s, seed=i) for i, s in enumerate([(T, H), (H,), (H,)]))
     xd, wd, bd = (x + 3).to(DEV), w.to(DEV), b.to(DEV)
-    assert kernel in _kernel(lambda: ops.layer_norm(xd, wd, bd, 1e-5), "layer_norm")
     want = torch.nn.functional.layer_norm(xd.double(), (H,), wd.double(), bd.double(), 1e-5)
     # one rounding to bf16, and 32-bit sums
     assert ((ops.layer_norm(xd, wd, bd, 1e-5).double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4).all()
+    name, = launched(lambda: ops.layer_norm(xd, wd, bd, 1e-5), "layer_norm")
+    assert kernel in name, name
 
 
 @pytest.mark.parametrize("Hq,Hkv", [(32, 8), (32, 32), (5, 3), (12, 2)])
@@ -177,7 +172,8 @@ def test_rotary_store_by_rows_per_sm(Hq, Hkv, per_sm, norm, kernel):
     slots = slots.to(DEV)
     pools = [torch.zeros(2, -(-(T + 5) // block), Hkv, block, 128, dtype=torch.bfloat16, device=DEV) for _ in range(2)]
     args = (qkv, pos, cs, Hq, Hkv, 128, qw, kw, 1e-6)
-    assert kernel in _kernel(lambda: ops.rope_qknorm_store(*args, pools[0][0], pools[0][1], slots), "rope_")
     q = ops.rope_qknorm_store(*args, pools[0][0], pools[0][1], slots)
     few = [ops.rope_qknorm_store(qkv[a:a + 32], pos[a:a + 32], *args[2:], pools[1][0], pools[1][1], slots[a:a + 32]) for a in range(0, T, 32)]
     assert torch.equal(q, torch.cat(few)) and torch.equal(pools[0], pools[1])
+    name, = launched(lambda: ops.rope_qknorm_store(*args, pools[0][0], pools[0][1], slots), "rope_")
+    assert kernel in name, name
