@@ -695,9 +695,9 @@ void launch_rope_qknorm_store(const void* qkv, const void* positions, const void
     return;
   }
   if (D == 128 && slots != nullptr) {
-    // EARLY for up to three blocks an SM (48 heads, 256 tokens: 3.3 -> 2.8 us; 36 heads, 512 tokens 3.4 -> 4.2 us, 1024 tokens of
-    // 48 heads 6.1 -> 7.1 us) and beside partial sums, whose loads are the longer wait
-    auto kern = partial != nullptr || warps <= 3ll * 32 * sms ? rope_qknorm_store_d128_kernel<true> : rope_qknorm_store_d128_kernel<false>;
+    // EARLY for up to three blocks an SM: 48 heads, 256 tokens 3.3 -> 2.8 us, with partial sums and their GEMM 24.3 -> 22.6 us; 36
+    // heads, 512 tokens 3.4 -> 4.2 us, 48 heads, 1024 tokens 6.1 -> 7.1 us, 96 heads, 200 tokens with their GEMM 47.1 -> 48.3 us
+    auto kern = warps <= 3ll * 32 * sms ? rope_qknorm_store_d128_kernel<true> : rope_qknorm_store_d128_kernel<false>;
     launch_pdl(PDL_ROPE, kern, dim3((unsigned)((warps + 31) / 32)), dim3(256), 0, s,
                (const bf16*)qkv, (const long long*)positions, (const float*)cos_sin, (const bf16*)q_w,
                (const bf16*)k_w, (bf16*)q_out, (bf16*)k_cache, (bf16*)v_cache, (const int*)slots, T, Hq, Hkv, eps,
