@@ -472,7 +472,6 @@ void launch_ccm_fused(void* pool, const int* block_tables, const int* kv_lens, c
   if (factor < 1 || factor > 8) throw std::runtime_error("fused CCM kernel: factor must be in [1, 8]");
   if ((unsigned long long)(layer_end * 2ll) * num_blocks * Hkv * block_size >= 0xffffffffull)
     throw std::runtime_error("fused CCM kernel: the pool has more rows than 32 bits count");
-  if (factor > 8) throw std::runtime_error("remainder move handles fewer than 8 rows");
   CcmParams p{};
   p.pool = (bf16*)pool;
   p.block_tables = block_tables;

@@ -57,10 +57,12 @@ void gemm_bf16(const void* x, const void* w, void* c, const void* bias, int M, i
                long long ldw, long long ldc, int act, const GemmWorkspace& ws, int sm_limit, cudaStream_t stream);
 
 // Prefill-size forms of the same kernel.
-// wide: columns [wide0, wide0 + wide_n) of the product also go to `wide` [M, wide_n] in fp32.
+// residual: c = residual [M, N] (pitch ldr) + product + bias, rounded once.  Returns false without launching for M <= 256,
+// N < 256 and outputs or residuals that TMA cannot describe (base not a multiple of 16 bytes, pitch not of 8 elements).
 bool gemm_bf16_residual(const void* x, const void* w, void* c, const void* bias, const void* residual, int M, int N, int K,
                         long long ldx, long long ldw, long long ldc, long long ldr, const GemmWorkspace& ws, int sm_limit,
                         cudaStream_t stream);
+// wide: columns [wide0, wide0 + wide_n) of the product also go to `wide` [M, wide_n] in fp32.
 void gemm_bf16_wide(const void* x, const void* w, void* c, int M, int N, int K, long long ldx, long long ldw, long long ldc,
                     int wide0, int wide_n, float* wide, const GemmWorkspace& ws, int sm_limit, cudaStream_t stream);
 // acc: the fp32 product replaces y [M, N] (pitch ldy) or is added to it.

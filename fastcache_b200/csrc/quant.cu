@@ -2,9 +2,9 @@
 // (two codes per byte, even index in the low nibble) and scaled FP8 (e4m3 / e5m2), their inverses, and the
 // quantise-and-restore round trip in one pass ("fake quantisation").
 //
-// One warp owns one group of `g` consecutive values of a row (g = the whole row for the INT8 and FP8 modes): a
+// Up to 32 lanes own one group of `g` consecutive values of a row (g = the whole row for the INT8 and FP8 modes): a
 // lane holds up to QMAX_CHUNKS 16-byte pieces in registers, the group statistics (absmax, or min and max) are a
-// warp reduction, and the codes go out as packed words.  The op is a single pass over the data: bound by
+// reduction over the lanes, and the codes go out as packed words.  The op is a single pass over the data: bound by
 // bandwidth (2 bytes read, 1 / 0.5 bytes written per value), nothing to put on the tensor cores.
 //
 // The arithmetic matches the PyTorch statements of fastcache_b200/compress/quant.py operation for operation
@@ -38,26 +38,6 @@ __constant__ float c_nf4[16] = {-1.0f, -0.6961928f, -0.52507305f, -0.39491749f, 
                                 -0.09105004f, 0.0f, 0.0795803f, 0.1609302f, 0.2461123f, 0.33791524f, 0.44070983f,
                                 0.562617f, 0.72295684f, 1.0f};
 
-__device__ __forceinline__ float warp_min(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
-
-__device__ __forceinline__ int nf4_code(float t) {
-  int best = 0;
-  float bd = fabsf(t - c_nf4[0]);
-#pragma unroll
-  for (int i = 1; i < 16; ++i) {
-    const float d = fabsf(t - c_nf4[i]);
-    if (d < bd) {            // the first of equal distances wins, like argmin
-      bd = d;
-      best = i;
-    }
-  }
-  return best;
-}
-
 __device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
   const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
 #pragma unroll
@@ -79,10 +59,10 @@ __device__ __forceinline__ void store8(bf16* p, const float (&f)[8]) {
 // code of one value and the value it stands for; `a` = scale (INT8, FP8) or absmax (INT4, NF4), `z` = zero point
 template <int MODE>
 __device__ __forceinline__ int encode(float x, float a, float z) {
+  static_assert(MODE != QUANT_NF4, "by nf4_code_fast");
   if (MODE == QUANT_INT8) return int(fminf(fmaxf(rintf(__fdiv_rn(x, a)), -127.f), 127.f));
   if (MODE == QUANT_INT8_ASYM) return int(fminf(fmaxf(rintf(__fdiv_rn(x - z, a)), 0.f), 255.f));
   if (MODE == QUANT_INT4) return int(fminf(fmaxf(rintf(__fdiv_rn(x, a) * 7.0f), -8.f), 7.f)) + 8;
-  if (MODE == QUANT_NF4) return nf4_code(__fdiv_rn(x, a));
   if (MODE == QUANT_FP8_E4M3) return int(__nv_cvt_float_to_fp8(__fdiv_rn(x, a), __NV_SATFINITE, __NV_E4M3));
   return int(__nv_cvt_float_to_fp8(__fdiv_rn(x, a), __NV_SATFINITE, __NV_E5M2));
 }
@@ -176,7 +156,9 @@ __device__ __forceinline__ void encode_exact(uint32_t which, const uint4& raw, f
     which &= which - 1;
     const uint32_t pair = i < 4 ? (i < 2 ? raw.x : raw.y) : (i < 6 ? raw.z : raw.w);
     const float x = __uint_as_float((i & 1) ? pair & 0xffff0000u : pair << 16);
-    const int e = (MODE == QUANT_NF4) ? nf4_code_fast(__fdiv_rn(x, a), s_mid) : encode<MODE>(x, a, z);
+    int e;
+    if constexpr (MODE == QUANT_NF4) e = nf4_code_fast(__fdiv_rn(x, a), s_mid);
+    else e = encode<MODE>(x, a, z);
     const int at = 8 * (i & 3);
     const uint32_t old = i < 4 ? w.x : w.y, now = (old & ~(0xFFu << at)) | (uint32_t(e & 0xFF) << at);
     if (i < 4) w.x = now;

@@ -264,18 +264,12 @@ class _SiglipEmbeddings(nn.Module):
         mapped onto the side x side table by fractional coordinates."""
         side = self.num_patches_per_side
         ids = torch.zeros(tgt_sizes.shape[0], max_patches, dtype=torch.long)
-        bounds = torch.arange(1 / side, 1.0, 1 / side)
         for b, (h, w) in enumerate(tgt_sizes.tolist()):
-            fh = torch.arange(0, 1 - 1e-6, 1 / h)
-            fw = torch.arange(0, 1 - 1e-6, 1 / w)
-            bh = torch.bucketize(fh, bounds, right=True)
-            bw = torch.bucketize(fw, bounds, right=True)
-            ids[b, : h * w] = (bh[:, None] * side + bw[None, :]).flatten()
+            ids[b, : h * w] = torch.from_numpy(self.buckets(h)[:, None].astype(np.int64) * side + self.buckets(w)[None, :]).flatten()
         return ids
 
-
     def buckets(self, n: int) -> np.ndarray:
-        """Table row (or column) of each of n patches along one side: the statement of `position_ids`, kept per n."""
+        """Table row (or column) of each of n patches along one side, a constant of n and the table's side that is kept."""
         if n not in self._buckets:
             side = self.num_patches_per_side
             f = torch.arange(0, 1 - 1e-6, 1 / n)
