@@ -24,8 +24,9 @@
 // have to be in flight while it runs: gathering warps of their own do that (with the epilogue's threads gathering,
 // an SM had no read outstanding for most of a tile), and the activation tile in tensor memory is what pays for the
 // deeper ring.  LLaVA-1.5 shape, 15 requests of 576 + 64 rows, 32 layers x 32 heads,
-// factor 4 (6.3 GB): 4.11 ms with the epilogue's threads gathering into three shared stages, 2.17 ms so, 1.96 ms with
-// the first GEMM of a tile under the scatter of the one before and a full ring announced at once.
+// factor 4 (6.3 GB), the kernel alone: 4.11 ms with the epilogue's threads gathering into three shared stages, 1.97 ms so, with
+// the first GEMM of a tile under the scatter of the one before and a full ring announced at once (0.49 of the copy rate; a call
+// from the host with its tables takes 2.2 ms).
 // In-place safety: an output row index never exceeds the index of any input row of the same head it depends on, tiles
 // are processed in ascending order by one CTA, and a tile is read completely (GEMM1 is done) before it is written.
 // What the gathering warps read ahead lies behind every row that is still to be written for an earlier tile.

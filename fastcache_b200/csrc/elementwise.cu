@@ -503,7 +503,7 @@ rope_qknorm_store_d128_kernel(const bf16* __restrict__ qkv, const long long* __r
 // The same without norms for prompts, where the GEMM has finished qkv: one warp takes ROPE_HEADS * 4 heads of one token, every
 // group of eight lanes ROPE_HEADS of them, so the angles, the position and the slot are read once for them and each lane has
 // 2 * ROPE_HEADS 16-byte loads in flight.  Bound by reading qkv and writing it back rotated; 26120 tokens, 32 + 2 * 8 heads:
-// 149 us with one head per group of lanes, 114 us so (642 MB, 5.6 TB/s).
+// 149 us with one head per group of lanes, 100 us so (642 MB, 6.4 TB/s).
 constexpr int ROPE_HEADS = 4;
 
 __global__ void __launch_bounds__(256)

@@ -21,8 +21,9 @@
 // main loop of a 128 x 256 tile takes about 4500 clocks, and four warps that store 16 bytes per lane to 32 different
 // rows take longer than that for one accumulator: each store instruction touches 32 cache lines, and one warp per
 // scheduler has nothing to hide its tcgen05.ld and MUFU latencies with.  Hence STAGED: 15 images through the CLIP tower,
-// 95 products of 8655 rows: 5.69 ms with the stores from registers, 4.49 ms so; SigLIP, 5 slices of 961 rows: 5.73 ms
-// against 4.72 ms.  At K = 4096 and more the main loop hides the plain epilogue, and the second group only costs: 26120
+// 95 products of 8655 rows: 5.69 ms with the stores from registers, 4.84 ms so, the sums with the residual included; SigLIP, 5
+// slices of 961 rows: 5.73 ms against 4.96 ms.  (Most of these run on CTA pairs by now, gemm_2cta.cu: 4.54 ms, 4.54 ms.)  At K =
+// 4096 and more the main loop hides the plain epilogue, and the second group only costs: 26120
 // rows through four 8B layers took 39.8 ms with it off and 40.8 ms with it on, so the line is at K = 2048.  Three prompts
 // of 250 to 450 tokens through the same layers, at the power limit when they follow one another: 1.83 ms with the staged
 // epilogue and CTA pairs wherever they save time alone, 1.78 ms with neither beyond that line.
